@@ -142,6 +142,41 @@ __device__ __forceinline__ double sqrt_nr(double x) {
   s = fma(fma(-s, s, m), 0.5 * y, s);
   return __longlong_as_double(__double_as_longlong(s) + ((long long)k << 52));
 }
+// Seeds of 1/x and 1/sqrt(x) (relative error below 2^-21) for recurrences
+// whose steps wait on them: moved between the formats by integer operations,
+// so that no conversion sits on the FP64 pipe.  One third-order step of the
+// binomial series completes them: with r = 1 - x y0, 1/x = y0 (1 + r + r^2 +
+// O(r^3)); with r = 1 - x y0^2, 1/sqrt(x) = y0 (1 + r/2 + 3 r^2/8 + O(r^3)),
+// the remainder below 2^-63.  x must be normal, with |exponent| <= 1000, and
+// positive for the square root.
+__device__ __forceinline__ double widen_exp(float y, int e) {  // y 2^e, y normal and positive
+  const unsigned u = __float_as_uint(y);
+  const unsigned hi = (u >> 3) + ((unsigned)(1023 - 127 + e) << 20);
+  return __hiloint2double((int)hi, (int)(u << 29));
+}
+__device__ __forceinline__ double rcp_seed(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const float m = __uint_as_float(0x3F800000u | ((hi & 0xFFFFFu) << 3) | (lo >> 29));
+  const double y = widen_exp(__fdividef(1.0f, m), 1023 - (int)((hi >> 20) & 0x7FFu));
+  return __hiloint2double(__double2hiint(y) | (int)(hi & 0x80000000u), __double2loint(y));
+}
+__device__ __forceinline__ float rcp_seed(float x) { return 1.0f / x; }
+__device__ __forceinline__ double rsqrt_b3(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const int e = (int)(hi >> 20) - 1023, k = e >> 1;  // x 2^-2k in [1, 4)
+  const float m = __uint_as_float((unsigned)(127 + e - 2 * k) << 23 | ((hi & 0xFFFFFu) << 3) |
+                                  (lo >> 29));
+  const double y0 = widen_exp(rsqrtf(m), -k);
+  const double r = fma(-(x * y0), y0, 1.0);
+  return fma(y0 * r, fma(r, 0.375, 0.5), y0);
+}
+__device__ __forceinline__ float rsqrt_b3(float x) { return 1.0f / sqrtf(x); }
+// w (1 + p) for a real p
+__device__ __forceinline__ double fma_real_(double w, double p) { return fma(w, p, w); }
+__device__ __forceinline__ float fma_real_(float w, float p) { return fmaf(w, p, w); }
+template <class R> __device__ __forceinline__ cplx<R> fma_real_(cplx<R> w, R p) {
+  return {fma_(w.re, p, w.re), fma_(w.im, p, w.im)};
+}
 __device__ __forceinline__ float rcp_nr(float x) { return 1.0f / x; }
 // sqrt of a non-negative sum of squares: the Newton form inside the normal
 // range, the IEEE square root for 0, subnormals, huge values, Inf and NaN
@@ -311,6 +346,14 @@ __device__ __forceinline__ unsigned cluster_nctarank() {
   unsigned r;
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
   return r;
+}
+// the two halves of the cluster barrier, for work between them that touches
+// nothing the other CTAs read or write
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::

@@ -23,7 +23,9 @@
 //     outside a safe range, and every cross-CTA reduction is done in a fixed
 //     order, so all CTAs derive bit-identical beta/tau/w.  The panel's Gram
 //     matrix V^H V is reduced at the end and the CTAs form the T factor's
-//     columns (forward, column-wise larft recurrence).
+//     columns (forward, column-wise larft recurrence).  Panels whose columns
+//     are far from dependent take ONE round for all columns instead
+//     (panel_block_round).
 //  2. larfb on the trailing columns:  W = V^H C (split-K GEMM, V read in
 //     place through a unit-lower mask), W2 = T^H W (reduce_trmm_kernel),
 //     C -= V W2 (GEMM).
@@ -67,7 +69,419 @@ struct PanelArgs {
   int* status;
   int gstride;          // allocation stride of the per-CTA partial rows
   int pair;             // two columns per barrier round where the norms allow
+  int block;            // the whole panel in one round where its conditioning allows (the
+                        // launch's shared memory then has block_extra_bytes after the slab)
 };
+
+// ---- block round: the whole panel from one Gram matrix -----------------------
+// The pair rounds below form two reflectors per barrier from the Gram entries
+// of two columns.  When the panel's columns are far from dependent, all of
+// them follow from ONE round: with G = A^H A of the panel (rows >= j0),
+// column j's |beta_j| and the row R_jc = G_jc / beta_j are one step of the
+// Cholesky factorization of G, and the reflectors follow from the panel's top
+// jb x jb block alone (Householder reconstruction, G. Ballard et al.,
+// "Reconstructing Householder vectors from TSQR", 2014): with s_j =
+// -sign(Re alpha_j), beta_j = s_j |beta_j|,
+//   F_jc = T0_jc - R_jc (c > j),  F_jj = alpha_j - beta_j,
+//   v_ij = T0_ij / F_jj,  T0_ic -= v_ij F_jc   (i > j),
+// an LU elimination of the top block whose rows are shifted by R, since
+// A = V F + [R; 0].  The rows below the top block follow by substitution,
+// V_bot = A_bot F^-1, and the T factor from A = (I - V T V^H) [R; 0]:
+// T = -F R^-1 V_top^-H.
+//
+// The Gram entries carry an error of eps |a_j| |a_c|, so the round is taken
+// only if every column keeps at least half its squared norm after the
+// columns before it are projected out (the pair rounds' test over the whole
+// panel; then cond(R) is small and the factors are as accurate as the column
+// by column ones), and if every squared norm is finite and far from overflow
+// and underflow.  Every CTA repeats the jb x jb work on identical numbers, so
+// all of them take the same branch; nothing has been written when the test
+// fails, and the panel is factored column by column as before.
+//
+// Bound: FP64 throughput (about 1.6 DFMA per clock per SM): rows x jb^2 / 2
+// multiply-adds for G and as many for V_bot, spread over the CTAs, plus the
+// jb x jb work, a chain of dependent FP64 operations of about 0.8 us per
+// column.  1000 x 501 Float64 QR 7.40 -> 4.52 ms, 2049 x 1000 full mixed QR
+// 19.0 -> 11.0 ms, 300 uneven blocks 257 -> 188 ms against the pair rounds
+// (a 1000-row panel: 236 us before, 80 us on 8 CTAs and 60 us on 16 now).
+constexpr int BLK_TILES = 36;   // 4 x 4 tiles of the upper triangle of a 32 x 32 Gram matrix
+constexpr int BLK_ROWGRP = 7;   // row groups: 36 x 7 = 252 of the 256 threads
+constexpr int BLK_LD = NBMAX + 1;
+constexpr int BLK_MIN_COLS = 8;
+constexpr int BLK_MIN_MP_PER_COL = 3;  // fewer rows per column rarely pass the test
+template <class T>
+constexpr size_t block_extra_bytes() {
+  // partial Gram tiles, G / L / scaled F (one square), top block
+  return sizeof(T) * (size_t)(BLK_TILES * 16 + 2 * NBMAX * BLK_LD) + 16;
+}
+__device__ __forceinline__ void blk_tile(int t, int& bi, int& bj) {
+  bj = 0;
+  while ((bj + 1) * (bj + 2) / 2 <= t) bj++;
+  bi = t - bj * (bj + 1) / 2;
+}
+
+// 1: the panel is factored and stored; 0: not taken (nothing written);
+// -1: a bounded barrier gave up
+template <class T, int SYNC>
+__device__ __forceinline__ int panel_block_round(const PanelArgs<T>& a, T* Ps, int ldp, int r0, int nr,
+                                 unsigned char* extra) {
+  using R = real_t<T>;
+  constexpr bool kCl = SYNC == SYNC_CLUSTER;
+  __shared__ R dg[NBMAX];     // squared norms of the panel's columns
+  __shared__ R rsv[NBMAX];    // 1 / |beta_j|
+  __shared__ R nrm_s[NBMAX];  // |beta_j|
+  __shared__ T raw[4][2][NBMAX];  // a pair's rows of G before they are scaled, by step
+  __shared__ R sgn_s[NBMAX];  // sign of beta_j
+  __shared__ T scl[NBMAX];    // 1 / F_jj
+  __shared__ int fail_s[NBMAX + 1];  // per step, and [NBMAX]: the norms' range
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+  const int b = blockIdx.x, G = gridDim.x, jb = a.jb;
+  T* Gp = reinterpret_cast<T*>(extra);       // [36][4][4] this CTA's partial Gram
+  T* Gs = Gp + BLK_TILES * 16;               // upper: G, then D and L; lower: F_jc / F_jj, transposed
+  T* T0 = Gs + NBMAX * BLK_LD;               // lower: V_top; upper: F
+  // the top block, straight from the (still unmodified) panel
+  T top[NBMAX / 8];
+#pragma unroll
+  for (int q = 0; q < NBMAX / 8; q++) {
+    const int c = wid + q * nw;
+    top[q] = (lane < jb && c < jb) ? ld_cg(&a.A[lane + (int64_t)c * a.lda]) : zero_<T>();
+  }
+  if (tid <= NBMAX) fail_s[tid] = 0;
+
+  // ---- partial Gram over this CTA's rows: one 4 x 4 tile per thread and row
+  // group, the groups folded in order
+  {
+    const int t = tid % BLK_TILES, grp = tid / BLK_TILES;
+    int bi, bj;
+    blk_tile(t, bi, bj);
+    T acc[4][4];
+#pragma unroll
+    for (int p = 0; p < 4; p++)
+#pragma unroll
+      for (int q = 0; q < 4; q++) acc[p][q] = zero_<T>();
+    if (grp < BLK_ROWGRP) {
+      const T *pi[4], *pj[4];
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        pi[p] = Ps + min(4 * bi + p, jb - 1) * ldp;
+        pj[p] = Ps + min(4 * bj + p, jb - 1) * ldp;
+      }
+      for (int r = grp; r < nr; r += BLK_ROWGRP) {
+        T x[4], y[4];
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+          x[p] = conj_(pi[p][r]);
+          y[p] = pj[p][r];
+        }
+#pragma unroll
+        for (int p = 0; p < 4; p++)
+#pragma unroll
+          for (int q = 0; q < 4; q++) acc[p][q] = fma_(x[p], y[q], acc[p][q]);
+      }
+    }
+    // fold the row groups: 0-3 into four buffers (the later three over the
+    // squares, which are filled afterwards), 4-6 added to the first three
+    T* const buf[4] = {Gp, Gs, Gs + BLK_TILES * 16, Gs + 2 * BLK_TILES * 16};
+    T* dst = grp < 4 ? buf[grp] : buf[(grp - 4) & 3];
+    if (grp < 4) {
+#pragma unroll
+      for (int p = 0; p < 16; p++) dst[t * 16 + p] = acc[p >> 2][p & 3];
+    }
+    __syncthreads();
+    if (grp >= 4 && grp < BLK_ROWGRP) {
+#pragma unroll
+      for (int p = 0; p < 16; p++) dst[t * 16 + p] += acc[p >> 2][p & 3];
+    }
+    __syncthreads();
+    for (int e = tid; e < BLK_TILES * 16; e += blockDim.x)
+      Gp[e] = (Gp[e] + buf[1][e]) + (buf[2][e] + buf[3][e]);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NBMAX / 8; q++) T0[lane * BLK_LD + wid + q * nw] = top[q];
+  }
+  // ---- sum over the CTAs in a fixed order, the same bits in every CTA
+  if constexpr (kCl) {
+    cluster_sync_all();
+    for (int e = tid; e < BLK_TILES * 16; e += blockDim.x) {
+      T s = zero_<T>();
+      for (int q0 = 0; q0 < G; q0 += 8) {
+        T v[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+          v[q] = q0 + q < G ? dsmem_ld(&Gp[e], (unsigned)(q0 + q)) : zero_<T>();
+#pragma unroll
+        for (int q = 0; q < 8; q++) s += v[q];
+      }
+      int bi, bj;
+      blk_tile(e >> 4, bi, bj);
+      const int d = 4 * bi + ((e >> 2) & 3), c = 4 * bj + (e & 3);
+      if (d <= c) Gs[d * BLK_LD + c] = s;
+    }
+    // from here on no CTA reads another's shared memory; the barrier's second
+    // half comes before anything the other CTAs may still read is rewritten
+    cluster_arrive();
+  } else {
+    for (int e = tid; e < BLK_TILES * 16; e += blockDim.x)
+      a.part_g[(int64_t)b * NBMAX * NBMAX + e] = Gp[e];
+    if (!panel_sync<SYNC>(a.bar, G, a.status)) return -1;
+    // one warp per entry
+    for (int e = b * nw + wid; e < BLK_TILES * 16; e += G * nw) {
+      T s = zero_<T>();
+      for (int q = lane; q < G; q += 32) s += ld_cg(&a.part_g[(int64_t)q * NBMAX * NBMAX + e]);
+      s = warp_sum(s);
+      if (lane == 0) a.gram[e] = s;
+    }
+    if (!panel_sync<SYNC>(a.bar, G, a.status)) return -1;
+    for (int e = tid; e < BLK_TILES * 16; e += blockDim.x) {
+      int bi, bj;
+      blk_tile(e >> 4, bi, bj);
+      const int d = 4 * bi + ((e >> 2) & 3), c = 4 * bj + (e & 3);
+      if (d <= c) Gs[d * BLK_LD + c] = ld_cg(&a.gram[e]);
+    }
+  }
+  __syncthreads();
+  if (wid == 0) {
+    const R g = lane < jb ? re_(Gs[lane * BLK_LD + lane]) : R(1);
+    const int lim = sizeof(R) == 8 ? 900 : 90;
+    const int e = exp2_of(g);
+    if (!(g > R(0) && finite_(g) && e > -lim && e < lim)) fail_s[NBMAX] = 1;
+    dg[lane] = g;
+  }
+  __syncthreads();
+  int failed = fail_s[NBMAX];
+
+  // ---- warps 0-3: G = L^H D L (L unit upper), then |beta_j| = sqrt(D_j), one
+  // step behind; warps 4-7: the elimination of the top block, two steps
+  // behind.  A step takes the column pair 2P, 2P + 1, whose two rows one warp
+  // owns (pair P: warp P mod 4 of each group; lane = column): the owner forms
+  // both in registers and publishes them, a barrier follows, then the other
+  // rows.  On GB300 a dependent FP64 operation takes about 100 cycles and a
+  // warp-wide one holds its sub-partition's FP64 pipe for 64, so the chains
+  // are kept short (four operations from D_j to D_{j+1} with no square root
+  // between them, five from alpha_j to alpha_{j+1}), and the next owner
+  // updates only the pair it needs before it goes on, the rest of its rows a
+  // step later.
+  if (!failed) {
+    const int w4 = wid & 3;
+    const bool chol = wid < 4;
+    const int np = (jb + 1) >> 1;
+    // one step of G = L^H D L on row g (lanes >= j): D_j returned, L_j in l
+    auto chol_row = [&](T g, int j, T& l) -> bool {
+      const R d = shfl_idx_(re_(g), j);
+      if (!(d >= R(0.5) * dg[j])) return false;
+      const R y = rcp_seed(d);
+      const R r = fma_(-d, y, R(1));
+      l = fma_real_(g * y, fma_(r, r, r));
+      return true;
+    };
+    // one step of the elimination on the top block's row t (current, lanes =
+    // columns): F_j (lanes >= j) over t, F_jc / F_jj in fn (lanes > j).  The
+    // sign of beta_j is opposite to alpha_j's real part.
+    auto lu_row = [&](T& t, int j, T& fn) {
+      const T alpha = shfl_idx_(t, j);
+      const R nrm = nrm_s[j];
+      const R sg = re_(alpha) >= R(0) ? R(-1) : R(1);
+      const R bj = sg * nrm;
+      const T fjj = alpha - make_scalar<T>(bj, R(0));
+      const T f = lane > j ? t - Gs[j * BLK_LD + lane] * bj : zero_<T>();
+      T y;
+      R p;
+      if constexpr (traits<T>::cpx) {
+        const R z2 = fma_(fjj.re, fjj.re, fjj.im * fjj.im);
+        const R y0 = rcp_seed(z2);
+        const R r = fma_(-z2, y0, R(1));
+        p = fma_(r, r, r);
+        y = conj_(fjj) * y0;
+      } else {
+        y = rcp_seed(fjj);
+        const R r = fma_(-fjj, y, R(1));
+        p = fma_(r, r, r);
+      }
+      fn = fma_real_(f * y, p);
+      if (lane > j) t = f;
+      if (lane == j) {
+        t = fjj;
+        sgn_s[j] = sg;
+        scl[j] = fma_real_(y, p);
+      }
+    };
+#pragma unroll 1
+    for (int it = 0; it < np + 2; it++) {
+      const int P = chol ? it : it - 2;
+      const bool live = P >= 0 && P < np;
+      const int j0 = 2 * P, j1 = j0 + 1;
+      const bool two = j1 < jb;
+      if (live && w4 == (P & 3)) {
+        if (chol) {
+          T* const G0 = Gs + j0 * BLK_LD;
+          T* const G1 = G0 + BLK_LD;
+          const T g0 = lane >= j0 ? G0[lane] : zero_<T>();
+          T l0 = zero_<T>(), l1 = zero_<T>(), g1 = zero_<T>();
+          bool ok = chol_row(g0, j0, l0);
+          if (two && ok) {
+            const T f = conj_(shfl_idx_(g0, j1));
+            g1 = lane >= j1 ? fma_(-f, l0, G1[lane]) : zero_<T>();
+            ok = chol_row(g1, j1, l1);
+          }
+          if (!ok) {
+            if (lane == 0) fail_s[P] = 1;
+          } else {
+            raw[P & 3][0][lane] = g0;
+            raw[P & 3][1][lane] = g1;
+            if (lane > j0) G0[lane] = l0;
+            if (two && lane >= j1) G1[lane] = lane == j1 ? g1 : l1;
+          }
+        } else {
+          T* const t0p = T0 + j0 * BLK_LD;
+          T t0 = t0p[lane], t1 = two ? t0p[BLK_LD + lane] : zero_<T>(), fn;
+          lu_row(t0, j0, fn);
+          t0p[lane] = t0;
+          if (lane > j0) Gs[lane * BLK_LD + j0] = fn;
+          if (two) {
+            const T e = shfl_idx_(t1, j0);
+            if (lane > j0) t1 = fma_(-e, fn, t1);
+            lu_row(t1, j1, fn);
+            t0p[BLK_LD + lane] = t1;
+            if (lane > j1) Gs[lane * BLK_LD + j1] = fn;
+          }
+        }
+      }
+      if (chol && it >= 1 && it <= np && w4 == ((it + 2) & 3)) {
+        const int j = 2 * (it - 1) + (lane & 1);
+        if (j < jb) {
+          const R d = re_(Gs[j * BLK_LD + j]);
+          const R rs = rsqrt_b3(d), s = d * rs;
+          if (lane < 2) {
+            nrm_s[j] = fma_(fma_(-s, s, d), R(0.5) * rs, s);  // sqrt(d), corrected
+            rsv[j] = rs;
+          }
+        }
+      }
+      __syncthreads();
+      // this step's flag (written by its owner before the barrier; one word
+      // per step, so that a later step's owner cannot race a slow reader)
+      if (it < np && fail_s[it]) {
+        failed = 1;
+        break;
+      }
+      if (!live) continue;
+      // the rows below: the next owner its next pair only; this step's owner
+      // its remaining pairs with the previous step's columns and this step's
+      const bool next = w4 == ((P + 1) & 3), prev = w4 == (P & 3) && P > 0;
+      const int pend = next ? min(P + 2, np) : np;
+      for (int p = P + 1 + ((w4 - P - 1) & 3); p < pend; p += 4) {
+        const int d0 = 2 * p, d1 = d0 + 1;
+        if (chol) {
+          T* const X = Gs + d0 * BLK_LD;
+          T a0 = X[lane], a1 = d1 < jb ? X[BLK_LD + lane] : zero_<T>();
+          for (int q = prev ? P - 1 : P; q <= P; q++) {
+            const T l0 = Gs[2 * q * BLK_LD + lane], l1 = Gs[(2 * q + 1) * BLK_LD + lane];
+            const T* r0p = raw[q & 3][0];
+            const T* r1p = raw[q & 3][1];
+            a0 = fma_(-conj_(r0p[d0]), l0, a0);
+            a1 = fma_(-conj_(r0p[d1]), l0, a1);
+            a0 = fma_(-conj_(r1p[d0]), l1, a0);
+            a1 = fma_(-conj_(r1p[d1]), l1, a1);
+          }
+          if (lane >= d0) X[lane] = a0;
+          if (lane >= d1 && d1 < jb) X[BLK_LD + lane] = a1;
+        } else {
+          T* const X = T0 + d0 * BLK_LD;
+          T a0 = X[lane], a1 = d1 < jb ? X[BLK_LD + lane] : zero_<T>();
+          for (int q = prev ? 2 * (P - 1) : 2 * P; q <= 2 * P + 1; q++) {
+            const T fn = lane > q ? Gs[lane * BLK_LD + q] : zero_<T>();
+            const T e0 = shfl_idx_(a0, q), e1 = shfl_idx_(a1, q);
+            a0 = fma_(-e0, fn, a0);
+            a1 = fma_(-e1, fn, a1);
+          }
+          X[lane] = a0;
+          if (d1 < jb) X[BLK_LD + lane] = a1;
+        }
+      }
+    }
+  }
+  if constexpr (kCl) cluster_wait();
+  if (failed) return 0;
+  __syncthreads();
+  // V_top's entries, scaled
+  for (int c = wid; c < jb; c += nw)
+    if (lane > c && lane < jb) T0[lane * BLK_LD + c] = T0[lane * BLK_LD + c] * scl[c];
+  __syncthreads();
+
+  // ---- T = -F R^-1 V_top^-H, a warp per row, spread over the CTAs
+  for (int i = b * nw + wid; i < NBMAX; i += G * nw) {
+    T t = zero_<T>();
+    if (i < jb) {
+      const bool in = lane >= i && lane < jb;
+      if (in) t = -T0[i * BLK_LD + lane];
+      for (int k = i; k < jb; k++) {
+        const T u = shfl_idx_(t, k);
+        if (lane > k && lane < jb) t = fma_(-u, Gs[k * BLK_LD + lane], t);
+      }
+      if (in) t = t * (sgn_s[lane] * rsv[lane]);
+      for (int k = i; k < jb; k++) {
+        const T u = shfl_idx_(t, k);
+        if (lane > k && lane < jb) t = fma_(-u, conj_(T0[lane * BLK_LD + k]), t);
+      }
+      if (!in) t = zero_<T>();
+    }
+    a.Tm[i + lane * NBMAX] = t;
+  }
+  // ---- rows below the top block: V_bot F = A_bot by substitution.  Eight
+  // threads per row hold four columns each (cyclic); u_j = x_j unscaled is
+  // passed on by a shuffle and F is read scaled by 1 / F_jj, so a step is one
+  // multiply-add per column.
+  {
+    const int q = lane & 7, rl = lane >> 3;
+    for (int rb = wid * 4; rb < nr; rb += nw * 4) {
+      const int r = rb + rl;
+      const bool in = r < nr && r0 + r >= jb;
+      T x[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        x[k] = (in && q + 8 * k < jb) ? Ps[r + (q + 8 * k) * ldp] : zero_<T>();
+#pragma unroll
+      for (int j = 0; j < NBMAX; j++) {
+        if (j < jb) {
+          T u = x[j >> 3];
+          if constexpr (traits<T>::cpx) {
+            u.re = __shfl_sync(0xffffffffu, u.re, j & 7, 8);
+            u.im = __shfl_sync(0xffffffffu, u.im, j & 7, 8);
+          } else {
+            u = __shfl_sync(0xffffffffu, u, j & 7, 8);
+          }
+#pragma unroll
+          for (int k = 0; k < 4; k++)
+            if (8 * k + 7 > j) {
+              const int c = q + 8 * k;
+              if (c > j && c < jb) x[k] = fma_(-u, Gs[c * BLK_LD + j], x[k]);
+            }
+        }
+      }
+      if (in) {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (q + 8 * k < jb) Ps[r + (q + 8 * k) * ldp] = x[k] * scl[q + 8 * k];
+      }
+    }
+  }
+  __syncthreads();
+  for (int c = wid; c < jb; c += nw)
+    for (int r = max(0, jb - r0) + lane; r < nr; r += 32)
+      a.A[(r0 + r) + (int64_t)c * a.lda] = Ps[r + c * ldp];
+  if (b == 0) {
+    // R above V_top, and tau_j = (beta_j - alpha_j) / beta_j
+    for (int c = wid; c < jb; c += nw)
+      if (lane < jb)
+        a.A[lane + (int64_t)c * a.lda] =
+            lane < c ? Gs[lane * BLK_LD + c] * (sgn_s[lane] * nrm_s[lane])
+                     : (lane == c ? make_scalar<T>(sgn_s[c] * nrm_s[c], R(0))
+                                  : T0[lane * BLK_LD + c]);
+    if (wid == 0 && lane < jb)
+      a.tau[lane] = -(T0[lane * BLK_LD + lane] * (sgn_s[lane] * rsv[lane]));
+  }
+  return 1;
+}
 
 template <class T, int SYNC>
 __global__ void __launch_bounds__(PANEL_THREADS, SYNC == SYNC_CLUSTER ? 2 : 1)
@@ -109,9 +523,26 @@ qr_panel_kernel(PanelArgs<T> a) {
   const int r0 = b * rpc;
   const int nr = max(0, min(a.mp, r0 + rpc) - r0);
 
-  for (int c = 0; c < jb; c++)
-    for (int r = tid; r < nr; r += blockDim.x) Ps[r + c * ldp] = a.A[(r0 + r) + (int64_t)c * a.lda];
+  // a warp takes four columns at a time: four independent loads per thread
+  for (int r = lane; r < nr; r += 32) {
+    T v[NBMAX / 8];
+#pragma unroll
+    for (int q = 0; q < NBMAX / 8; q++) {
+      const int c = wid + q * nw;
+      v[q] = c < jb ? a.A[(r0 + r) + (int64_t)c * a.lda] : zero_<T>();
+    }
+#pragma unroll
+    for (int q = 0; q < NBMAX / 8; q++)
+      if (wid + q * nw < jb) Ps[r + (wid + q * nw) * ldp] = v[q];
+  }
   __syncthreads();
+  if constexpr (!kH) {
+    if (a.block) {
+      const size_t slab = ((size_t)ldp * jb * sizeof(T) + 15) / 16 * 16;
+      const int done = panel_block_round<T, SYNC>(a, Ps, ldp, r0, nr, smem_raw + slab);
+      if (done != 0) return;
+    }
+  }
 
   // Per column one grid-wide reduction: the partial sums of squares of x =
   // column j below the diagonal, its largest magnitude, the partial dot
@@ -884,35 +1315,55 @@ static size_t panel_slab_cap() {
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap);
     cudaFuncSetAttribute(qr_panel_kernel<T, SYNC_HIER>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap);
+    cudaFuncSetAttribute(qr_panel_kernel<T, SYNC_CLUSTER>,
+                         cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return cap;
   });
 }
 
+constexpr int kPanelClusterWide = 16;
 // Panels of at most this many rows per CTA (times the cluster limit) run as
 // one thread-block cluster: below it a column's FP64 work per CTA stays
 // smaller than what a global barrier costs.
 constexpr int PANEL_CLUSTER_ROWS = 256;
 
 // Launch shape of the panel kernel.  Cluster (sync = SYNC_CLUSTER): panels
-// of up to kPanelClusterMax x PANEL_CLUSTER_ROWS rows, at least 64 rows per
+// of up to kPanelClusterMax x PANEL_CLUSTER_ROWS rows, at least 32 rows per
 // CTA.  Cooperative grid (SYNC_GRID) beyond that: rows per CTA bounded below
 // by 64 (a grid barrier is only paid when there is real parallel work) and
 // above by the shared-memory slab size; at most one CTA per SM.
 struct PanelShape {
   int G, rpc, sync;
+  int block = 0;  // the block round may be tried (its shared memory follows the slab)
   int cl = 1;  // CTAs per cluster (SYNC_CLUSTER: G; SYNC_HIER: the cluster size)
   size_t smem;
 };
+// shared memory of a launch: the slab, and the block round's scratch where
+// the panel is tall enough to take it and the scratch fits beside the slab
 template <class T>
-static int panel_shape(int64_t mp, int jb, PanelShape& ps, int want_ctas) {
+static void panel_smem(PanelShape& ps, int64_t mp, int jb, size_t cap) {
+  const size_t slab = (size_t)(ps.rpc | 1) * jb * sizeof(T);
+  const size_t both = align_up(slab, 16) + block_extra_bytes<T>();
+  ps.block = tuning(TUNE_PANEL_PAIR) != 0 && jb >= BLK_MIN_COLS &&
+             mp >= (int64_t)BLK_MIN_MP_PER_COL * jb && both <= cap;
+  ps.smem = ps.block ? both : slab;
+}
+template <class T>
+static int panel_shape(int64_t mp, int jb, PanelShape& ps, int want_ctas, bool main_stream) {
   const int max_ctas = num_sms();
   const size_t cap = panel_slab_cap<T>();
   int64_t rpc_max = (int64_t)(cap / ((size_t)jb * sizeof(T))) - 1;  // ld = rpc | 1
   const int64_t cl_rows = rpc_max < PANEL_CLUSTER_ROWS ? rpc_max : PANEL_CLUSTER_ROWS;
-  if (mp <= (int64_t)kPanelClusterMax * cl_rows) {
-    int64_t G = ceil_div(mp, 64);
-    if (G > kPanelClusterMax) G = kPanelClusterMax;
-    if (G < 1) G = 1;
+  // Clusters of up to 16 CTAs (a non-portable size) of at least 32 rows: the
+  // block round's FP64 work is shared by the CTAs (1000 x 501 Float64 QR 4.72
+  // -> 4.50 ms against 8 CTAs of at least 64 rows, 2049 x 1000 mixed 11.65 ->
+  // 10.76 ms, the 300 uneven blocks 189.7 -> 186.6 ms).  8 CTAs on the
+  // look-ahead side stream, where the main stream's grid leaves 16 free SMs of
+  // one cluster group only by chance, and where 16 do not fit.
+  for (int cmax = main_stream ? kPanelClusterWide : kPanelClusterMax;
+       mp <= (int64_t)kPanelClusterMax * cl_rows; cmax = kPanelClusterMax) {
+    int64_t G = ceil_div(mp, 32);
+    if (G > cmax) G = cmax;
     int64_t rpc = ceil_div(mp, G);
     if (rpc < 1) rpc = 1;
     G = ceil_div(mp, rpc);
@@ -921,7 +1372,7 @@ static int panel_shape(int64_t mp, int jb, PanelShape& ps, int want_ctas) {
     ps.rpc = (int)rpc;
     ps.sync = SYNC_CLUSTER;
     ps.cl = (int)G;
-    ps.smem = (size_t)(ps.rpc | 1) * jb * sizeof(T);
+    panel_smem<T>(ps, mp, jb, cap);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     cfg.gridDim = dim3((unsigned)G);
@@ -938,7 +1389,8 @@ static int panel_shape(int64_t mp, int jb, PanelShape& ps, int want_ctas) {
             cudaSuccess &&
         nclusters >= 1)
       return 0;
-    (void)cudaGetLastError();  // fall through to the cooperative grid
+    (void)cudaGetLastError();  // the smaller cluster, then the cooperative grid
+    if (cmax == kPanelClusterMax) break;
   }
   // taller panels: a cooperative grid of clusters of C CTAs when the tuning
   // table asks for it (MAK_PANEL_HIER_C), else a plain cooperative grid
@@ -992,7 +1444,7 @@ static int panel_shape(int64_t mp, int jb, PanelShape& ps, int want_ctas) {
   ps.rpc = (int)rpc;
   ps.sync = SYNC_GRID;
   ps.cl = 1;
-  ps.smem = (size_t)(ps.rpc | 1) * jb * sizeof(T);
+  panel_smem<T>(ps, mp, jb, cap);
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, qr_panel_kernel<T, SYNC_GRID>,
                                                     PANEL_THREADS, ps.smem) != cudaSuccess)
@@ -1163,10 +1615,11 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
   auto panel = [&](int64_t j0, int jb, cudaStream_t s) -> int {
     const int64_t mp = m - j0;
     PanelShape ps;
-    MAK_TRY(panel_shape<T>(mp, jb, ps, s == st ? sms : tl_side_ctas));
+    MAK_TRY(panel_shape<T>(mp, jb, ps, s == st ? sms : tl_side_ctas, s == st));
     PanelArgs<T> pa{A + j0 + j0 * lda, lda, (int)mp, jb, ps.rpc, tau + j0,
                     Ts + (j0 / nb) * NBMAX * NBMAX, part_nrm, part_w, part_g, alpha_buf,
-                    gram_buf, bar, cflag, status, gmax, ps.sync != SYNC_HIER && tuning(TUNE_PANEL_PAIR) != 0};
+                    gram_buf, bar, cflag, status, gmax, ps.sync != SYNC_HIER && tuning(TUNE_PANEL_PAIR) != 0,
+                    ps.block};
     ProfScope prof(s, PROF_QR_PANEL, 2.0 * (double)mp * jb * sizeof(T));
     note_launch();
     if (ps.sync == SYNC_CLUSTER || ps.sync == SYNC_HIER) {
