@@ -30,12 +30,12 @@ __global__ void splitk_fold_kernel(int64_t M, int64_t N, int splits, const T* pa
 template <class T>
 static int gemm_native(cudaStream_t st, int64_t M, int64_t N, int64_t K, T alpha, Operand<T> A,
                        Operand<T> B, T beta, T* C, int64_t ldc, Arena& ar) {
-  const int splits = (M > 0 && N > 0 && K > 0) ? pick_splits(M, N, K, num_sms()) : 1;
+  const int splits = (M > 0 && N > 0 && K > 0) ? pick_splits<T>(M, N, K, num_sms()) : 1;
   if (ar.base == nullptr) {
     // measuring: a bound valid for every smaller output too (pick_splits
     // keeps splits * tiles <= 4 * SMs), since the split count grows as the
     // output shrinks while call sites measure at their largest shape
-    if (K > 64) {  // pick_splits keeps >= 64 of K per split
+    if (K > 32) {  // pick_splits keeps >= 32 of K per split
       const size_t bound = (size_t)4 * num_sms() * 64 * 64;
       const size_t cap = (size_t)64 * (size_t)(M > 0 ? M : 1) * (size_t)(N > 0 ? N : 1);
       ar.take<T>(bound < cap ? bound : cap);

@@ -10,9 +10,9 @@
 // packed QR storage without materialising copies.
 //
 // On GB300 FP64 runs at ~1 TFLOP/s for the whole chip (measured: DFMA and
-// DMMA alike), i.e. ~3.3 flop/clk/SM, so a plain 64x64x16 smem tile is already
-// issue-bound on the FP64 pipe; the tensor-core path is the split-precision
-// GEMM in ozaki.cuh.
+// DMMA alike), i.e. ~2 multiply-adds per clock per SM, so even a 16 x 16 tile
+// is bound by the FP64 pipe and the only question is whether every SM has
+// work; the tensor-core path is the split-precision GEMM in ozaki.cu.
 #pragma once
 #include "mak_common.cuh"
 
@@ -56,9 +56,15 @@ __device__ __forceinline__ T load_op(const Operand<T>& X, int64_t i, int64_t k) 
   return X.op == OP_C ? conj_(v) : v;
 }
 
+int num_sms();
+constexpr int GEMM_BK = 32;  // K per step (and the granule of a K split)
+
 template <class T>
 __device__ __forceinline__ bool is_zero_(T v) { return v == zero_<T>(); }
 
+// One BM x BN tile of C per CTA of 256 threads (TM x TN outputs each).  The
+// next K step's elements are fetched into registers while the current one is
+// multiplied.
 template <class T, int BM, int BN, int BK, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_kernel(int M, int N, int K, T alpha, Operand<T> A, Operand<T> B, T beta, T* C,
@@ -67,6 +73,8 @@ gemm_kernel(int M, int N, int K, T alpha, Operand<T> A, Operand<T> B, T beta, T*
   constexpr int RX = BM / TM;  // threads along rows
   constexpr int RY = BN / TN;  // threads along columns
   constexpr int NT = RX * RY;
+  constexpr int LA = BM * BK / NT, LB = BN * BK / NT;  // elements fetched per thread
+  static_assert(LA * NT == BM * BK && LB * NT == BN * BK, "whole tiles");
   __shared__ T As[BK][BM + 1];
   __shared__ T Bs[BK][BN + 1];
   const int64_t m0 = (int64_t)blockIdx.x * BM;
@@ -82,22 +90,43 @@ gemm_kernel(int M, int N, int K, T alpha, Operand<T> A, Operand<T> B, T beta, T*
 #pragma unroll
     for (int c = 0; c < TN; c++) acc[r][c] = zero_<T>();
 
-  for (int k0 = kbeg; k0 < kend; k0 += BK) {
-    for (int e = tid; e < BM * BK; e += NT) {
+  T ra[LA], rb[LB];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < LA; q++) {
+      const int e = tid + q * NT;
       int ii, kk;
       if (A.op == OP_N) { ii = e % BM; kk = e / BM; } else { kk = e % BK; ii = e / BK; }
-      int64_t gi = m0 + ii;
-      int gk = k0 + kk;
-      As[kk][ii] = (gi < M && gk < kend) ? load_op(A, gi, gk) : zero_<T>();
+      const int64_t gi = m0 + ii;
+      const int gk = k0 + kk;
+      ra[q] = (gi < M && gk < kend) ? load_op(A, gi, gk) : zero_<T>();
     }
-    for (int e = tid; e < BK * BN; e += NT) {
+#pragma unroll
+    for (int q = 0; q < LB; q++) {
+      const int e = tid + q * NT;
       int kk, jj;
       if (B.op == OP_N) { kk = e % BK; jj = e / BK; } else { jj = e % BN; kk = e / BN; }
-      int64_t gj = n0 + jj;
-      int gk = k0 + kk;
-      Bs[kk][jj] = (gj < N && gk < kend) ? load_op(B, gk, gj) : zero_<T>();
+      const int64_t gj = n0 + jj;
+      const int gk = k0 + kk;
+      rb[q] = (gj < N && gk < kend) ? load_op(B, gk, gj) : zero_<T>();
+    }
+  };
+  if (kbeg < kend) fetch(kbeg);
+  for (int k0 = kbeg; k0 < kend; k0 += BK) {
+#pragma unroll
+    for (int q = 0; q < LA; q++) {
+      const int e = tid + q * NT;
+      if (A.op == OP_N) As[e / BM][e % BM] = ra[q];
+      else As[e % BK][e / BK] = ra[q];
+    }
+#pragma unroll
+    for (int q = 0; q < LB; q++) {
+      const int e = tid + q * NT;
+      if (B.op == OP_N) Bs[e % BK][e / BK] = rb[q];
+      else Bs[e / BN][e % BN] = rb[q];
     }
     __syncthreads();
+    if (k0 + BK < kend) fetch(k0 + BK);
 #pragma unroll 4
     for (int kk = 0; kk < BK; kk++) {
       T a[TM], b[TN];
@@ -150,35 +179,51 @@ int gemm(cudaStream_t st, int64_t M, int64_t N, int64_t K, T alpha, Operand<T> A
     return cudaGetLastError() == cudaSuccess ? 0 : MAK_ERR_CUDA;
   }
   if (splits < 1) splits = 1;
-  constexpr int BK = 16;
-  int kchunk = (int)ceil_div(ceil_div(K, splits), BK) * BK;
+  int kchunk = (int)ceil_div(ceil_div(K, splits), GEMM_BK) * GEMM_BK;
   splits = (int)ceil_div(K, kchunk);
   if (used_splits) *used_splits = splits;
   if (splits > 1) beta = zero_<T>();
   ProfScope prof(st, PROF_GEMM_NATIVE, (traits<T>::cpx ? 8.0 : 2.0) * M * N * K);
-  if (M <= 32) {
-    dim3 g((unsigned)ceil_div(M, 32), (unsigned)ceil_div(N, 64), (unsigned)splits);
-    note_launch();
-    gemm_kernel<T, 32, 64, BK, 2, 4><<<g, 256, 0, st>>>((int)M, (int)N, (int)K, alpha, A, B,
-                                                         beta, C, ldc, kchunk, split_stride,
-                                                         skip_flag());
+  note_launch();
+#define MAK_GEMM_TILE(BM, BN, BK, TM, TN)                                                        \
+  gemm_kernel<T, BM, BN, BK, TM, TN>                                                             \
+      <<<dim3((unsigned)ceil_div(M, BM), (unsigned)ceil_div(N, BN), (unsigned)splits), 256, 0,   \
+         st>>>((int)M, (int)N, (int)K, alpha, A, B, beta, C, ldc, kchunk, split_stride,          \
+               skip_flag())
+  const int64_t t32 = ceil_div(M, 32) * ceil_div(N, 32) * splits;
+  if constexpr (sizeof(real_t<T>) == 8) {
+    // The FP64 pipe is so slow that the operand traffic of a small tile costs
+    // nothing, while every SM left without a tile costs its share of the
+    // chip's FP64 rate: 32 x 32 tiles from three per SM, else 16 x 16.
+    // Against 64 x 64 (and 32 x 64) tiles: a 512 x 64 x 32 complex update 140
+    // -> 14.5 us, 1000 x 501 Float64 QR 4.5 -> 2.6 ms, 300 uneven blocks 188
+    // -> 139 ms; 3000^3 45.3 -> 44.4 ms (1.22 TFLOP/s), 700^3 0.85 -> 0.83 ms.
+    if (t32 >= 3 * (int64_t)num_sms()) MAK_GEMM_TILE(32, 32, GEMM_BK, 2, 2);
+    else MAK_GEMM_TILE(16, 16, GEMM_BK, 1, 1);
   } else {
-    dim3 g((unsigned)ceil_div(M, 64), (unsigned)ceil_div(N, 64), (unsigned)splits);
-    note_launch();
-    gemm_kernel<T, 64, 64, BK, 4, 4><<<g, 256, 0, st>>>((int)M, (int)N, (int)K, alpha, A, B,
-                                                         beta, C, ldc, kchunk, split_stride,
-                                                         skip_flag());
+    // FP32 is bound by shared memory bandwidth in a small tile (two loads per
+    // FMA), so it is taken only where the wide ones would leave SMs idle
+    // (1537 x 4093 Float32 LQ 8.6 -> 6.0 ms)
+    if (t32 < 2 * (int64_t)num_sms()) MAK_GEMM_TILE(32, 32, GEMM_BK, 2, 2);
+    else if (M <= 32) MAK_GEMM_TILE(32, 64, 16, 2, 4);
+    else MAK_GEMM_TILE(64, 64, 16, 4, 4);
   }
+#undef MAK_GEMM_TILE
   return cudaGetLastError() == cudaSuccess ? 0 : MAK_ERR_CUDA;
 }
 
-// number of K-splits that fills the GPU for an output of M x N
+// number of K-splits that fills the GPU for an output of M x N: two 32 x 32
+// tiles per SM for the FP64 types (at least 32 of K per split), two 64-wide
+// tiles for the FP32 types (at least 64)
+template <class T>
 inline int pick_splits(int64_t M, int64_t N, int64_t K, int sms) {
-  int64_t tiles = ceil_div(M, M <= 32 ? 32 : 64) * ceil_div(N, 64);
+  constexpr bool f64 = sizeof(real_t<T>) == 8;
+  const int64_t tiles = f64 ? ceil_div(M, 32) * ceil_div(N, 32)
+                            : ceil_div(M, M <= 32 ? 32 : 64) * ceil_div(N, 64);
   int64_t want = 2LL * sms;
   if (tiles >= want) return 1;
   int64_t s = ceil_div(want, tiles);
-  int64_t maxs = ceil_div(K, 64);  // keep >= 64 of K per split
+  int64_t maxs = ceil_div(K, f64 ? 32 : 64);
   if (s > maxs) s = maxs;
   if (s < 1) s = 1;
   if (s > 64) s = 64;

@@ -1102,7 +1102,11 @@ qr_panel_kernel(PanelArgs<T> a) {
 }
 
 // W2[:, c] = op(Tm) * sum_s Wpart[s][:, c]   (op = ^H for the factorization,
-// identity for Q formation).  Fixed summation order -> deterministic.
+// identity for Q formation).  Fixed summation order -> deterministic.  Eight
+// columns per CTA, one output per thread: the FP64 work of the product is
+// spread over as many SMs as there are column groups (32 columns per CTA left
+// most of them idle: 500 columns 17.5 us).
+constexpr int TRMM_COLS = 8;
 template <class T>
 __global__ void __launch_bounds__(256) reduce_trmm_kernel(int jb, int nt, int splits,
                                                           const T* __restrict__ Wpart,
@@ -1110,27 +1114,35 @@ __global__ void __launch_bounds__(256) reduce_trmm_kernel(int jb, int nt, int sp
                                                           const T* __restrict__ Tm, int conjtrans,
                                                           T* __restrict__ W2) {
   __shared__ T Ts[NBMAX][NBMAX + 1];
-  __shared__ T Ws[NBMAX][33];
-  const int c0 = blockIdx.x * 32;
+  __shared__ T Ws[TRMM_COLS][NBMAX];
+  const int i = threadIdx.x & 31, cc = threadIdx.x >> 5;
+  const int c = blockIdx.x * TRMM_COLS + cc;
   for (int e = threadIdx.x; e < jb * jb; e += blockDim.x) {
-    const int i = e % jb, l = e / jb;
-    Ts[i][l] = conjtrans ? conj_(Tm[l + i * NBMAX]) : Tm[i + l * NBMAX];
+    const int r = e % jb, l = e / jb;
+    if (conjtrans) Ts[l][r] = conj_(Tm[r + l * NBMAX]);
+    else Ts[r][l] = Tm[r + l * NBMAX];
   }
-  for (int e = threadIdx.x; e < jb * 32; e += blockDim.x) {
-    const int i = e % jb, cc = e / jb;
-    T s = zero_<T>();
-    if (c0 + cc < nt)
-      for (int q = 0; q < splits; q++) s += Wpart[q * sstride + i + (int64_t)(c0 + cc) * jb];
-    Ws[i][cc] = s;
+  T w = zero_<T>();
+  if (i < jb && c < nt) {
+    const T* src = Wpart + i + (int64_t)c * jb;
+    int q = 0;
+    for (; q + 3 < splits; q += 4) {
+      const T a = src[q * sstride], b = src[(q + 1) * sstride];
+      const T d = src[(q + 2) * sstride], f = src[(q + 3) * sstride];
+      w += (a + b) + (d + f);
+    }
+    for (; q < splits; q++) w += src[q * sstride];
   }
+  Ws[cc][i] = w;
   __syncthreads();
-  for (int e = threadIdx.x; e < jb * 32; e += blockDim.x) {
-    const int i = e % jb, cc = e / jb;
-    if (c0 + cc >= nt) continue;
-    T s = zero_<T>();
-    for (int l = 0; l < jb; l++) s = fma_(Ts[i][l], Ws[l][cc], s);
-    W2[i + (int64_t)(c0 + cc) * jb] = s;
-  }
+  if (i >= jb || c >= nt) return;
+  T s[4] = {zero_<T>(), zero_<T>(), zero_<T>(), zero_<T>()};
+  int l = 0;
+  for (; l + 3 < jb; l += 4)
+#pragma unroll
+    for (int q = 0; q < 4; q++) s[q] = fma_(Ts[i][l + q], Ws[cc][l + q], s[q]);
+  for (; l < jb; l++) s[0] = fma_(Ts[i][l], Ws[cc][l], s[0]);
+  W2[i + (int64_t)c * jb] = (s[0] + s[1]) + (s[2] + s[3]);
 }
 
 constexpr int QR_OUTER_NB = 128;  // outer block of the mixed-precision path
@@ -1570,13 +1582,13 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
     const int64_t mp = m - j0;
     const T* Ap = A + j0 + j0 * lda;
     T* C = A + j0 + c0 * lda;
-    int splits = pick_splits(jb, nt, mp, sms);
+    int splits = pick_splits<T>(jb, nt, mp, sms);
     if (splits > max_splits) splits = max_splits;
     int used = 1;
     MAK_TRY(gemm<T>(s, jb, nt, mp, one_<T>(), opnd<T>(Ap, lda, OP_C, MASK_UNIT_LOWER),
                     opnd<T>(C, lda), zero_<T>(), Wpart, jb, splits, (int64_t)jb * nt, &used));
     note_launch();
-    reduce_trmm_kernel<T><<<(unsigned)ceil_div(nt, 32), 256, 0, s>>>(jb, (int)nt, used, Wpart,
+    reduce_trmm_kernel<T><<<(unsigned)ceil_div(nt, TRMM_COLS), 256, 0, s>>>(jb, (int)nt, used, Wpart,
                                                                       (int64_t)jb * nt, Tb, 1, W2);
     MAK_CUDA_TRY(cudaGetLastError());
     return gemm<T>(s, mp, nt, jb, -one_<T>(), opnd<T>(Ap, lda, OP_N, MASK_UNIT_LOWER),
@@ -1601,7 +1613,7 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
                            Wp, jb, ga, status, mc));
     }
     note_launch();
-    reduce_trmm_kernel<T><<<(unsigned)ceil_div(nt, 32), 256, 0, s>>>(jb, (int)nt, 1, Wp,
+    reduce_trmm_kernel<T><<<(unsigned)ceil_div(nt, TRMM_COLS), 256, 0, s>>>(jb, (int)nt, 1, Wp,
                                                                       (int64_t)jb * nt, Tb, 1, W2p);
     MAK_CUDA_TRY(cudaGetLastError());
     Arena ga(grams, gram_bytes);
@@ -1760,13 +1772,13 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
     const T* Ap = A + j0 + j0 * lda;
     const T* Tb = Ts + bi * NBMAX * NBMAX;
     T* Qs = Q + j0 + j0 * ldq;
-    int splits = pick_splits(jb, qt, mp, sms);
+    int splits = pick_splits<T>(jb, qt, mp, sms);
     if (splits > max_splits) splits = max_splits;
     int used = 1;
     MAK_TRY(gemm<T>(st, jb, qt, mp, one_<T>(), opnd<T>(Ap, lda, OP_C, MASK_UNIT_LOWER),
                     opnd<T>(Qs, ldq), zero_<T>(), Wpart, jb, splits, (int64_t)jb * qt, &used));
     note_launch();
-    reduce_trmm_kernel<T><<<(unsigned)ceil_div(qt, 32), 256, 0, st>>>(
+    reduce_trmm_kernel<T><<<(unsigned)ceil_div(qt, TRMM_COLS), 256, 0, st>>>(
         jb, (int)qt, used, Wpart, (int64_t)jb * qt, Tb, 0, W2);
     MAK_CUDA_TRY(cudaGetLastError());
     MAK_TRY(gemm<T>(st, mp, qt, jb, -one_<T>(), opnd<T>(Ap, lda, OP_N, MASK_UNIT_LOWER),

@@ -1,0 +1,46 @@
+"""The native product at the edges of its tiles (16 x 16 and 32 x 32), of its
+K step (32) and of its K splits, every op, against a 64-bit product.
+
+Bound: an inner product of K terms summed in any order is within
+(K + 2) eps sum |a||b| of the exact one (complex: four times that).
+"""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from conftest import to_dev, to_host
+
+pytestmark = pytest.mark.gpu
+# (1, 1, 1) .. one tile; 31/32/33 around a K step; tall K: split; many tiles: 32 x 32
+SHAPES = [(1, 1, 1), (16, 16, 32), (17, 15, 33), (32, 33, 31), (31, 250, 1000), (5, 7, 4097),
+          (700, 705, 40), (1500, 64, 96)]
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.complex128], ids=lambda d: np.dtype(d).name)
+@pytest.mark.parametrize("ops", ["NN", "CN", "NC", "TT"])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
+def test_native_gemm_tiles(mak, cuda, dt, ops, shape):
+    from mak_gb300 import blas
+
+    m, n, k = shape
+    rng = np.random.default_rng(m + 7 * n + 13 * k)
+
+    def rand(r, c):
+        x = rng.standard_normal((r, c))
+        return (x + 1j * rng.standard_normal((r, c)) if dt is np.complex128 else x).astype(dt)
+
+    A = rand(m, k) if ops[0] == "N" else rand(k, m)
+    B = rand(k, n) if ops[1] == "N" else rand(n, k)
+    C0 = rand(m, n)
+    f = {"N": lambda x: x, "T": lambda x: x.T, "C": lambda x: x.conj().T}
+    a, b = f[ops[0]](A), f[ops[1]](B)
+    C = to_dev(C0, cuda)
+    blas.gemm(to_dev(A, cuda), to_dev(B, cuda), ops[0], ops[1], alpha=-1.0, beta=0.5, C=C)
+    torch.cuda.synchronize()
+    ref = -(a @ b) + 0.5 * C0
+    eps = np.finfo(np.float64).eps
+    bound = 4 * (k + 4) * eps * (np.abs(a) @ np.abs(b) + np.abs(C0))
+    assert np.all(np.abs(to_host(C) - ref) <= 2 * bound)
