@@ -244,53 +244,100 @@ __global__ void __launch_bounds__(GJ_THREADS) gje_panel_kernel(GjArgs<T> a) {
     for (int r = tid; r < nr; r += blockDim.x) Xp[(r0 + r) + (int64_t)c * a.ldx] = Ps[r + c * rpc];
 }
 
-// For every column outside the panel: apply the panel's row exchanges in
-// order, save rows k0..k0+b-1 into buf (b x n) and zero them in X.
+// For every column outside the panel [k0, k0 + b): apply the panel's row
+// exchanges, save rows k0 .. k0+b-1 into buf (b x n) and zero them in X.
 // Only columns c in [c_lo, c_hi) are touched.
+//
+// The exchanges are composed first: only rows k0 .. k0+b-1 and the pivots
+// take part, and the source of each is found by walking the exchanges
+// backwards (every CTA repeats this small integer work).  Then a column is
+// one batch of independent loads and one of stores, instead of b dependent
+// exchanges through memory (4096 rows: 140 us per call before).
+// perm, when given, is the composed row permutation of the whole
+// elimination so far, exchanged along by one extra CTA.
+constexpr int LASWP_MAX_B = 128;
 template <class T>
-__global__ void gje_laswp_save_kernel(int n, T* X, int64_t ldx, int k0, int b, const int* piv,
-                                      T* buf, int c_lo, int c_hi, const int* skip) {
+__global__ void __launch_bounds__(256) gje_laswp_save_kernel(int n, T* X, int64_t ldx, int k0,
+                                                             int b, const int* piv, T* buf,
+                                                             int c_lo, int c_hi, int* perm,
+                                                             const int* skip) {
   if (skipped(skip)) return;
-  const int c = c_lo + blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ int pv[LASWP_MAX_B];
+  __shared__ int pos[2 * LASWP_MAX_B], src[2 * LASWP_MAX_B];
+  const int tid = threadIdx.x;
+  for (int t = tid; t < b; t += blockDim.x) {
+    const int p = piv[k0 + t];
+    pv[t] = (p >= k0 + t && p < n) ? p : k0 + t;
+  }
+  __syncthreads();
+  // entry t < b: row k0 + t; entry b + t: row pv[t] if it lies below the
+  // panel's rows (a row that is the pivot twice is listed twice with the same
+  // source, so both entries store the same value)
+  for (int e = tid; e < 2 * b; e += blockDim.x) {
+    const int x = e < b ? k0 + e : pv[e - b];
+    int s = -1;
+    if (e < b || x >= k0 + b) {
+      s = x;
+      for (int t = b - 1; t >= 0; t--) {
+        if (s == k0 + t) s = pv[t];
+        else if (s == pv[t]) s = k0 + t;
+      }
+    }
+    pos[e] = x;
+    src[e] = s;
+  }
+  __syncthreads();
+  if (perm != nullptr && blockIdx.x == gridDim.x - 1) {
+    // at most 2 x 128 entries: one per thread
+    const int s = tid < 2 * b ? src[tid] : -1;
+    const int v = s >= 0 ? perm[s] : 0;
+    __syncthreads();
+    if (s >= 0) perm[pos[tid]] = v;
+    return;
+  }
+  // a warp per column
+  const int lane = tid & 31;
+  const int c = c_lo + blockIdx.x * (int)(blockDim.x >> 5) + (tid >> 5);
   if (c >= c_hi || (c >= k0 && c < k0 + b)) return;
   T* col = X + (int64_t)c * ldx;
-  for (int t = 0; t < b; t++) {
-    const int jj = k0 + t, p = piv[jj];
-    if (p != jj && p >= 0 && p < n) {
-      T x = col[jj];
-      col[jj] = col[p];
-      col[p] = x;
-    }
+  constexpr int U = 2 * LASWP_MAX_B / 32;
+  T v[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const int e = lane + 32 * u;
+    if (32 * u < 2 * b && e < 2 * b && src[e] >= 0) v[u] = col[src[e]];
   }
-  for (int t = 0; t < b; t++) {
-    buf[t + (int64_t)c * b] = col[k0 + t];
-    col[k0 + t] = zero_<T>();
-  }
-}
-
-__global__ void iota_kernel(int n, int* v) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) v[i] = i;
-}
-
-// iperm = inverse of the composed row permutation
-__global__ void gje_perm_kernel(int n, const int* piv, int* iperm, const int* skip) {
-  if (skipped(skip)) return;
-  extern __shared__ int perm[];
-  for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = i;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int jj = 0; jj < n; jj++) {
-      const int p = piv[jj];
-      if (p != jj && p >= 0 && p < n) {
-        int t = perm[jj];
-        perm[jj] = perm[p];
-        perm[p] = t;
+  __syncwarp();  // every load of the column before any store to it
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const int e = lane + 32 * u;
+    if (32 * u < 2 * b && e < 2 * b && src[e] >= 0) {
+      if (e < b) {
+        buf[e + (int64_t)c * b] = v[u];
+        col[pos[e]] = zero_<T>();
+      } else {
+        col[pos[e]] = v[u];
       }
     }
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) iperm[perm[i]] = i;
+}
+
+__global__ void iota_kernel(int n, int* v, int* w) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) {
+    v[i] = i;
+    w[i] = i;
+  }
+}
+
+// iperm = inverse of the composed row permutation
+__global__ void gje_perm_kernel(int n, const int* perm, int* iperm, const int* skip) {
+  if (skipped(skip)) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) {
+    const int p = perm[i];
+    if (p >= 0 && p < n) iperm[p] = i;
+  }
 }
 
 // slab capacity of the panel kernel; the kernels' dynamic shared-memory
@@ -311,8 +358,6 @@ static size_t gj_slab_cap() {
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap);
     cudaFuncSetAttribute(gje_panel_kernel<T, SYNC_CLUSTER>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap);
-    cudaFuncSetAttribute(gje_perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         max_smem_optin() - 1024);
     return cap;
   });
 }
@@ -337,6 +382,7 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
                      (traits<T>::cpx ? 4.0 : 1.0) * (double)n * (double)n * GJ_OUTER_NB >= gate;
   const int NBO = mixed ? GJ_OUTER_NB : GJ_NB;
   int* piv = ar.take<int>(n > 0 ? n : 1);
+  int* perm = ar.take<int>(n > 0 ? n : 1);
   // per-CTA pivot partials and candidate rows, double-buffered by column parity
   real_t<T>* part_val = ar.take<real_t<T>>(2 * sms);
   int* part_idx = ar.take<int>(2 * sms);
@@ -357,12 +403,13 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
   if (ar.base == nullptr) return 0;
   if (!ar.ok()) return MAK_ERR_WORKSPACE;
   if (n <= 0) return 0;
+  // (the largest n whose inverse is provided)
   if ((size_t)n * sizeof(int) > (size_t)max_smem_optin() - 1024) return MAK_ERR_UNSUPPORTED;
   MAK_CUDA_TRY(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), st));
   // pivots start as the identity so that an aborted panel (bounded barrier
-  // timeout) still leaves every index in range
+  // timeout) still leaves every index in range; so does the permutation
   note_launch();
-  iota_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>((int)n, piv);
+  iota_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>((int)n, piv, perm);
   const size_t cap = gj_slab_cap<T>();
   // one 32-wide panel (cooperative launch, at most max_ctas CTAs: on the
   // look-ahead side stream it leaves the other SMs to the main stream)
@@ -434,8 +481,8 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
       const int b = (int)((K0 + KB - k0) < GJ_NB ? (K0 + KB - k0) : GJ_NB);
       MAK_TRY(panel(k0, b, s, max_ctas));
       note_launch();
-      gje_laswp_save_kernel<T><<<(unsigned)ceil_div(c_hi - c_lo, 128), 128, 0, s>>>(
-          (int)n, X, ldx, (int)k0, b, piv, buf, (int)c_lo, (int)c_hi, skip_flag());
+      gje_laswp_save_kernel<T><<<(unsigned)ceil_div(c_hi - c_lo, 8) + 1, 256, 0, s>>>(
+          (int)n, X, ldx, (int)k0, b, piv, buf, (int)c_lo, (int)c_hi, perm, skip_flag());
       MAK_CUDA_TRY(cudaGetLastError());
       const T* F = X + k0 * ldx;
       if (k0 > c_lo)
@@ -453,8 +500,8 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
                          int max_ctas) -> int {
     if (c_hi <= c_lo) return 0;
     note_launch();
-    gje_laswp_save_kernel<T><<<(unsigned)ceil_div(c_hi - c_lo, 128), 128, 0, s>>>(
-        (int)n, X, ldx, (int)K0, (int)KB, piv, bufo, (int)c_lo, (int)c_hi, skip_flag());
+    gje_laswp_save_kernel<T><<<(unsigned)ceil_div(c_hi - c_lo, 8), 256, 0, s>>>(
+        (int)n, X, ldx, (int)K0, (int)KB, piv, bufo, (int)c_lo, (int)c_hi, nullptr, skip_flag());
     MAK_CUDA_TRY(cudaGetLastError());
     const T* Fb = X + K0 * ldx;
     const int64_t l1 = c_hi < K0 ? c_hi : K0;  // left part [c_lo, l1)
@@ -507,7 +554,7 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
     }
   }
   note_launch();
-  gje_perm_kernel<<<1, 1024, (size_t)n * sizeof(int), st>>>((int)n, piv, iperm, skip_flag());
+  gje_perm_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>((int)n, perm, iperm, skip_flag());
   MAK_CUDA_TRY(cudaGetLastError());
   return 0;
 }
