@@ -421,6 +421,26 @@ __device__ __forceinline__ cplx<R> dsmem_ld(const cplx<R>* p, unsigned rank) {
   return {dsmem_ld(&p->re, rank), dsmem_ld(&p->im, rank)};
 }
 
+// Stores to the same variable in CTA `rank` of the cluster.
+__device__ __forceinline__ void dsmem_st(double* p, unsigned rank, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(dsmem_addr(p, rank)), "d"(v) : "memory");
+}
+__device__ __forceinline__ void dsmem_st(float* p, unsigned rank, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dsmem_addr(p, rank)), "f"(v) : "memory");
+}
+__device__ __forceinline__ void dsmem_st(int* p, unsigned rank, int v) {
+  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(dsmem_addr(p, rank)), "r"(v) : "memory");
+}
+__device__ __forceinline__ void dsmem_st(unsigned long long* p, unsigned rank,
+                                         unsigned long long v) {
+  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(dsmem_addr(p, rank)), "l"(v) : "memory");
+}
+template <class R>
+__device__ __forceinline__ void dsmem_st(cplx<R>* p, unsigned rank, cplx<R> v) {
+  dsmem_st(&p->re, rank, v.re);
+  dsmem_st(&p->im, rank, v.im);
+}
+
 // --------------------------------------------------------------- host side --
 #define MAK_CUDA_TRY(expr)                         \
   do {                                             \

@@ -14,10 +14,9 @@
 // The inverse is an in-place blocked Gauss-Jordan elimination with partial
 // pivoting (gje_inverse): per block column of 32 a panel kernel (pivot
 // search + row exchange + elimination, one barrier per column, panel rows
-// resident in shared memory; a thread-block cluster of up to 8 CTAs for
-// n <= 2048, a cooperative grid with a bounded global barrier beyond), a
-// row-exchange/save kernel
-// for the other columns and one rank-32 GEMM update -- 2n^3 flops in total,
+// resident in shared memory; a thread-block cluster of up to 16 CTAs for
+// n <= 4096, a cooperative grid with a bounded global barrier beyond), a
+// row-exchange/save kernel for the other columns and one rank-32 GEMM update -- 2n^3 flops in total,
 // the same count as the reference's LU + inverse.  The Newton update reads
 // X^{-H} straight out of the eliminated matrix through the inverse column
 // permutation (no separate transpose or permutation pass) and fuses the
@@ -36,7 +35,6 @@ namespace mak {
 constexpr int GJ_NB = 32;
 constexpr int GJ_OUTER_NB = 128;  // block column of the mixed-precision path
 constexpr int GJ_THREADS = 256;
-constexpr int GJ_CLUSTER_ROWS = 256;  // rows per CTA up to which a panel runs as one cluster
 
 template <class T>
 struct GjArgs {
@@ -45,6 +43,7 @@ struct GjArgs {
   int n, k0, b, rpc;
   int* piv;
   real_t<T>* part_val;
+  unsigned long long* part_key;  // [2][gstride] the same by key (register panel)
   int* part_idx;
   T* swapbuf;  // [2][GJ_NB]: row jj by column parity
   T* cand;     // [2][gstride][GJ_NB]: each CTA's pivot candidate row, by column parity
@@ -65,7 +64,10 @@ __device__ __forceinline__ void amax_merge(R& v, int& i, R v2, int i2) {
   if (v2 > v || (v2 == v && i2 < i)) { v = v2; i = i2; }
 }
 
-template <class T, int SYNC>
+// The panel of an inverse whose rows do not fit shared memory twice (from
+// about 200 rows per CTA, n beyond 10^4): one grid round per column, the slab
+// once in shared memory.  All smaller ones take gje_panel_ahead_kernel.
+template <class T>
 __global__ void __launch_bounds__(GJ_THREADS) gje_panel_kernel(GjArgs<T> a) {
   using R = real_t<T>;
   if (skipped(a.skip)) return;  // the same in every CTA: no barrier is reached
@@ -78,14 +80,6 @@ __global__ void __launch_bounds__(GJ_THREADS) gje_panel_kernel(GjArgs<T> a) {
   __shared__ T srow[GJ_NB];
   __shared__ T dinv_s;
   __shared__ int pivs, pivq;
-  // cluster variant: this CTA's published pivot candidate, candidate row and
-  // (its holder) row jj, by column parity, read by the other CTAs through
-  // distributed shared memory after the cluster barrier
-  __shared__ R x_val[2];
-  __shared__ int x_idx[2];
-  __shared__ T x_cand[2][GJ_NB];
-  __shared__ T x_rowjj[2][GJ_NB];
-  constexpr bool kCl = SYNC == SYNC_CLUSTER;
   const int G = gridDim.x, cb = blockIdx.x, tid = threadIdx.x;
   const int lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
   const int rpc = a.rpc, b = a.b, k0 = a.k0;
@@ -127,8 +121,7 @@ __global__ void __launch_bounds__(GJ_THREADS) gje_panel_kernel(GjArgs<T> a) {
     if (lane == 0) { sv[wid] = best; si[wid] = bidx; }
     if (jj >= r0 && jj < r0 + nr)
       for (int c = tid; c < b; c += blockDim.x) {
-        if constexpr (kCl) x_rowjj[par][c] = Ps[(jj - r0) + c * rpc];
-        else rowjj[c] = Ps[(jj - r0) + c * rpc];
+        rowjj[c] = Ps[(jj - r0) + c * rpc];
       }
     __syncthreads();
     if (wid == 0) {
@@ -141,13 +134,8 @@ __global__ void __launch_bounds__(GJ_THREADS) gje_panel_kernel(GjArgs<T> a) {
         amax_merge(v, ix, v2, i2);
       }
       if (lane == 0) {
-        if constexpr (kCl) {
-          x_val[par] = v;
-          x_idx[par] = ix;
-        } else {
-          pval[cb] = v;
-          pidx[cb] = ix;
-        }
+        pval[cb] = v;
+        pidx[cb] = ix;
         pivs = ix;
       }
     }
@@ -156,26 +144,18 @@ __global__ void __launch_bounds__(GJ_THREADS) gje_panel_kernel(GjArgs<T> a) {
       const int li = pivs;  // this CTA's candidate row (global index)
       if (li != INT_MAX)
         for (int c = tid; c < b; c += blockDim.x) {
-          if constexpr (kCl) x_cand[par][c] = Ps[(li - r0) + c * rpc];
-          else cand[(int64_t)cb * GJ_NB + c] = Ps[(li - r0) + c * rpc];
+          cand[(int64_t)cb * GJ_NB + c] = Ps[(li - r0) + c * rpc];
         }
     }
-    if (!panel_sync<SYNC>(a.bar, G, a.status)) return;
+    if (!panel_sync<SYNC_GRID>(a.bar, G, a.status)) return;
 
     // ---- global pivot (identical in every CTA), then the exchange
     if (wid == 0) {
       R v = R(-1);
       int ix = INT_MAX, iq = -1;
       for (int q = lane; q < G; q += 32) {
-        R v2;
-        int i2;
-        if constexpr (kCl) {
-          v2 = dsmem_ld(&x_val[par], (unsigned)q);
-          i2 = dsmem_ld(&x_idx[par], (unsigned)q);
-        } else {
-          v2 = ld_cg(&pval[q]);
-          i2 = ld_cg(&pidx[q]);
-        }
+        const R v2 = ld_cg(&pval[q]);
+        const int i2 = ld_cg(&pidx[q]);
         if (v2 > v || (v2 == v && i2 < ix)) { v = v2; ix = i2; iq = q; }
       }
 #pragma unroll
@@ -193,20 +173,10 @@ __global__ void __launch_bounds__(GJ_THREADS) gje_panel_kernel(GjArgs<T> a) {
     __syncthreads();
     const int p = pivs, q = pivq;
     // pivot row: the winning CTA's candidate (row jj itself when p == jj)
-    if constexpr (kCl) {
-      const unsigned own = (unsigned)(jj / rpc);  // the CTA holding row jj
-      for (int c = tid; c < b; c += blockDim.x)
-        prow[c] = q < 0 ? dsmem_ld(&x_rowjj[par][c], own)
-                        : dsmem_ld(&x_cand[par][c], (unsigned)q);
-      if (p != jj && p >= r0 && p < r0 + nr)
-        for (int c = tid; c < b; c += blockDim.x)
-          Ps[(p - r0) + c * rpc] = dsmem_ld(&x_rowjj[par][c], own);
-    } else {
-      for (int c = tid; c < b; c += blockDim.x)
-        prow[c] = q < 0 ? ld_cg(&rowjj[c]) : ld_cg(&cand[(int64_t)q * GJ_NB + c]);
-      if (p != jj && p >= r0 && p < r0 + nr)
-        for (int c = tid; c < b; c += blockDim.x) Ps[(p - r0) + c * rpc] = ld_cg(&rowjj[c]);
-    }
+    for (int c = tid; c < b; c += blockDim.x)
+      prow[c] = q < 0 ? ld_cg(&rowjj[c]) : ld_cg(&cand[(int64_t)q * GJ_NB + c]);
+    if (p != jj && p >= r0 && p < r0 + nr)
+      for (int c = tid; c < b; c += blockDim.x) Ps[(p - r0) + c * rpc] = ld_cg(&rowjj[c]);
     if (cb == 0 && tid == 0) a.piv[jj] = p;
     __syncthreads();
     if (tid == 0) {
@@ -237,11 +207,317 @@ __global__ void __launch_bounds__(GJ_THREADS) gje_panel_kernel(GjArgs<T> a) {
     }
     __syncthreads();
   }
-  // cluster variant: no CTA leaves (releasing its shared memory) while
-  // another may still read its last column's partials
-  if constexpr (kCl) panel_sync<SYNC>(a.bar, G, a.status);
   for (int c = 0; c < b; c++)
     for (int r = tid; r < nr; r += blockDim.x) Xp[(r0 + r) + (int64_t)c * a.ldx] = Ps[r + c * rpc];
+}
+
+// ---- the panel one column ahead ------------------------------------------------
+// The panel's rows sit row-major in shared memory, in two buffers by column
+// parity.  Warp 0 of a CTA runs one column ahead of the others: after the
+// pivot of column j is known it updates column j + 1 alone (lane = row),
+// picks the CTA's next candidate (the largest magnitude at or below row
+// jj + 1, the first row on ties; complex: the larger component), forms that
+// row, scales it by its pivot's reciprocal and publishes it, while the other
+// warps eliminate column j from all rows.  So a column's chain is one search,
+// one reciprocal and one round between the CTAs, and the elimination's FP64
+// work (rows x 32 per column at 1.66 per clock per SM) runs beside it.  In a
+// cluster (SYNC_CLUSTER) the candidates are pushed into every CTA's shared
+// memory before the cluster barrier, so that nothing is fetched after it; in
+// a grid they go through L2.  Elementwise arithmetic only: the result does
+// not depend on the number of CTAs.
+__device__ __forceinline__ unsigned long long pivot_key(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+  return b > 0x7FF0000000000000ull ? 0ull : b;  // NaN is never preferred
+}
+__device__ __forceinline__ unsigned long long pivot_key(float x) {
+  const unsigned b = __float_as_uint(x) & 0x7FFFFFFFu;
+  return b > 0x7F800000u ? 0ull : (unsigned long long)b << 32;
+}
+template <class R> __device__ __forceinline__ unsigned long long pivot_key(cplx<R> x) {
+  const unsigned long long a = pivot_key(x.re), b = pivot_key(x.im);
+  return a > b ? a : b;
+}
+// by integer comparison (a comparison of doubles would take the FP64 pipe)
+__device__ __forceinline__ bool is_nan_(double x) {
+  return ((unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull) >
+         0x7FF0000000000000ull;
+}
+__device__ __forceinline__ bool is_nan_(float x) {
+  return (__float_as_uint(x) & 0x7FFFFFFFu) > 0x7F800000u;
+}
+template <class R> __device__ __forceinline__ bool is_nan_(cplx<R> x) {
+  return is_nan_(x.re) || is_nan_(x.im);
+}
+// the lanes' largest key, the smallest index among equals; the lane it is in
+__device__ __forceinline__ int warp_pivot(unsigned long long& key, int& idx) {
+  const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(key >> 32));
+  bool in = (unsigned)(key >> 32) == hi;
+  const unsigned lo = __reduce_max_sync(0xffffffffu, in ? (unsigned)key : 0u);
+  in = in && (unsigned)key == lo;
+  const int i = __reduce_min_sync(0xffffffffu, in ? idx : INT_MAX);
+  const unsigned at = __ballot_sync(0xffffffffu, in && idx == i);
+  key = (unsigned long long)hi << 32 | lo;
+  idx = i;
+  return __ffs((int)at) - 1;
+}
+// 1 / d into y (1 + p): y close to 1/d with r = 1 - d y, p = r + r^2; beyond
+// the normal range y is the IEEE quotient and p = 0
+__device__ __forceinline__ void inv_split(double d, double& y, double& p) {
+  const int e = exp2_of(d);
+  if (e > -1000 && e < 1000) {
+    y = rcp_seed(d);
+    const double r = fma(-d, y, 1.0);
+    p = fma(r, r, r);
+  } else {
+    y = 1.0 / d;
+    p = 0.0;
+  }
+}
+__device__ __forceinline__ void inv_split(float d, float& y, float& p) {
+  y = 1.0f / d;
+  p = 0.0f;
+}
+template <class R> __device__ __forceinline__ void inv_split(cplx<R> d, cplx<R>& y, R& p) {
+  const R w = fmax(fabs(d.re), fabs(d.im));
+  const int e = exp2_of(w);
+  const int lim = sizeof(R) == 8 ? 480 : 50;
+  if (w > R(0) && e > -lim && e < lim) {
+    R q;
+    inv_split(fma_(d.re, d.re, d.im * d.im), q, p);
+    y = conj_(d) * q;
+  } else {
+    y = inv_fast(d);
+    p = R(0);
+  }
+}
+
+constexpr int kGjClusterWide = 16;
+constexpr int GJA_LD = GJ_NB + 1;
+// Warps 1-3 and 5-7 eliminate; warp 4 shares warp 0's SM sub-partition, whose
+// FP64 pipe is left to it, and only passes row jj + 1 on.
+constexpr int GJA_MAIN = 6;
+// NL: rows per lane of warp 0 (32 NL rows per CTA at most)
+template <class T, int SYNC, int NL>
+__global__ void __launch_bounds__(GJ_THREADS, 1) gje_panel_ahead_kernel(GjArgs<T> a) {
+  using R = real_t<T>;
+  if (skipped(a.skip)) return;  // the same in every CTA: no barrier is reached
+  constexpr bool kCl = SYNC == SYNC_CLUSTER;
+  constexpr int GC = kCl ? kGjClusterWide : 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* const Xs = reinterpret_cast<T*>(smem_raw);  // [2][rpc][GJA_LD]
+  // by column parity: the CTAs' candidates (scaled rows) and row jj
+  // (cluster: written by the other CTAs)
+  __shared__ unsigned long long x_key[2][GC];
+  __shared__ int x_idx[2][GC];
+  __shared__ T x_row[2][GC][GJ_NB];
+  __shared__ T x_rowjj[2][GJ_NB];
+  const int G = gridDim.x, cb = blockIdx.x, tid = threadIdx.x;
+  const int lane = tid & 31, wid = tid >> 5, nw = GJ_THREADS / 32;
+  const int b = a.b, k0 = a.k0, rpc = a.rpc;
+  const int r0 = cb * rpc;
+  const int nr = max(0, min(a.n, r0 + rpc) - r0);
+  const size_t slab = (size_t)rpc * GJA_LD;
+  T* Xp = a.X + (int64_t)k0 * a.ldx + r0;
+  {
+    T* const X0 = Xs + slab;  // "column -1"
+    for (int r = lane; r < nr; r += 32) {
+      T v[GJ_NB / 8];
+#pragma unroll
+      for (int q = 0; q < GJ_NB / 8; q++) {
+        const int c = wid + q * nw;
+        v[q] = c < b ? Xp[r + (int64_t)c * a.ldx] : zero_<T>();
+      }
+#pragma unroll
+      for (int q = 0; q < GJ_NB / 8; q++) X0[r * GJA_LD + wid + q * nw] = v[q];
+    }
+  }
+  __syncthreads();
+  // a CTA may be written to only once it runs
+  if constexpr (kCl) cluster_sync_all();
+
+  // publish row v (lane = column) of column j's round as this CTA's candidate
+  auto put_cand = [&](int par, unsigned long long key, int idx, T v) {
+    if constexpr (kCl) {
+      for (int q = 0; q < G; q++) dsmem_st(&x_row[par][cb][lane], (unsigned)q, v);
+      if (lane < G) {
+        dsmem_st(&x_key[par][cb], (unsigned)lane, key);
+        dsmem_st(&x_idx[par][cb], (unsigned)lane, idx);
+      }
+    } else {
+      if (lane < b) a.cand[((int64_t)par * a.gstride + cb) * GJ_NB + lane] = v;
+      if (lane == 0) {
+        a.part_key[par * a.gstride + cb] = key;
+        a.part_idx[par * a.gstride + cb] = idx;
+      }
+    }
+  };
+  auto put_rowjj = [&](int par, T v) {
+    if constexpr (kCl) {
+      for (int q = 0; q < G; q++) dsmem_st(&x_rowjj[par][lane], (unsigned)q, v);
+    } else {
+      if (lane < b) a.swapbuf[par * GJ_NB + lane] = v;
+    }
+  };
+  // the candidate among warp 0's column values cv (rows r0 + lane + 32 l, at
+  // or below row jj): key, row index (INT_MAX: none) and value
+  T cv[NL];
+  auto pick = [&](int jj, unsigned long long& key, int& idx, T& d) {
+    key = 0;
+    idx = INT_MAX;
+    d = zero_<T>();
+#pragma unroll
+    for (int l = 0; l < NL; l++) {
+      const int r = lane + 32 * l;
+      const unsigned long long k2 = pivot_key(cv[l]);
+      // a NaN is no candidate, as in a comparison by magnitude
+      if (r < nr && r0 + r >= jj && !is_nan_(cv[l]) && (idx == INT_MAX || k2 > key)) {
+        key = k2;
+        idx = r0 + r;
+        d = cv[l];
+      }
+    }
+    const int at = warp_pivot(key, idx);
+    d = shfl_idx_(d, at);
+  };
+
+  if (wid == 0) {
+    const T* X0 = Xs + slab;
+#pragma unroll
+    for (int l = 0; l < NL; l++)
+      cv[l] = lane + 32 * l < nr ? X0[(lane + 32 * l) * GJA_LD] : zero_<T>();
+    unsigned long long key;
+    int idx;
+    T d, y;
+    R pr;
+    pick(k0, key, idx, d);
+    inv_split(d, y, pr);
+    const T v = idx == INT_MAX ? zero_<T>() : X0[(idx - r0) * GJA_LD + lane];
+    put_cand(0, key, idx, fma_real_(lane == 0 ? y : v * y, pr));
+  } else if (wid == 4 && k0 >= r0 && k0 < r0 + nr) {
+    put_rowjj(0, Xs[slab + (k0 - r0) * GJA_LD + lane]);
+  }
+
+  for (int j = 0; j < b; j++) {
+    const int jj = k0 + j, par = j & 1;
+    const T* const Xo = Xs + (par ^ 1) * slab;  // through column j - 1
+    T* const Xn = Xs + par * slab;
+    if (!panel_sync<SYNC>(a.bar, G, a.status)) return;
+
+    // ---- the pivot, the same in every warp of every CTA
+    int p, q = 0;
+    unsigned long long key = 0;
+    {
+      int idx = INT_MAX;
+      if constexpr (kCl) {
+        if (lane < G) {
+          key = x_key[par][lane];
+          idx = x_idx[par][lane];
+          q = lane;
+        }
+      } else {
+        for (int g = lane; g < G; g += 32) {
+          const unsigned long long k2 = __ldcg(&a.part_key[par * a.gstride + g]);
+          const int i2 = ld_cg(&a.part_idx[par * a.gstride + g]);
+          if (k2 > key || (k2 == key && i2 < idx)) {
+            key = k2;
+            idx = i2;
+            q = g;
+          }
+        }
+      }
+      q = __shfl_sync(0xffffffffu, q, warp_pivot(key, idx));
+      p = idx == INT_MAX ? jj : idx;
+      if (idx == INT_MAX) q = -1;
+    }
+    T srow, rjj = zero_<T>();
+    if (p != jj || q < 0) {
+      if constexpr (kCl) rjj = x_rowjj[par][lane];
+      else rjj = lane < b ? ld_cg(&a.swapbuf[par * GJ_NB + lane]) : zero_<T>();
+    }
+    if (q >= 0) {
+      if constexpr (kCl) srow = x_row[par][q][lane];
+      else srow = lane < b ? ld_cg(&a.cand[((int64_t)par * a.gstride + q) * GJ_NB + lane])
+                           : zero_<T>();
+    } else {  // no candidate (NaN only): row jj itself
+      T y;
+      R pr;
+      inv_split(shfl_idx_(rjj, j), y, pr);
+      srow = fma_real_(lane == j ? y : rjj * y, pr);
+    }
+    if (cb == 0 && tid == 0) {
+      a.piv[jj] = p;
+      if (q >= 0 && key == 0) atomicExch(a.singular, 1);
+    }
+    const int lp = p != jj ? p - r0 : -1;  // the pivot's old row here: row jj moves into it
+    const T rjj_j = shfl_idx_(rjj, j);
+    // row r through column j (lane = column)
+    auto through = [&](int r, T x, T f) -> T {
+      return r0 + r == jj ? srow : fma_(-f, srow, lane == j ? zero_<T>() : x);
+    };
+
+    if (wid == 0) {
+      if (j + 1 < b) {
+        const T sj1 = shfl_idx_(srow, j + 1), rj1 = shfl_idx_(rjj, j + 1);
+        T fv[NL];
+#pragma unroll
+        for (int l = 0; l < NL; l++) {
+          const int r = lane + 32 * l;
+          const bool at = r == lp;
+          fv[l] = at ? rjj_j : cv[l];
+          const T x = at ? rj1 : (r < nr ? Xo[r * GJA_LD + j + 1] : zero_<T>());
+          cv[l] = fma_(-fv[l], sj1, x);
+        }
+        unsigned long long k2;
+        int idx;
+        T d, y;
+        R pr;
+        pick(jj + 1, k2, idx, d);
+        inv_split(d, y, pr);
+        T v = zero_<T>();
+        if (idx != INT_MAX) {
+          const int r = idx - r0;
+          T f = fv[0];
+#pragma unroll
+          for (int l = 1; l < NL; l++)
+            if (r >> 5 == l) f = fv[l];
+          f = shfl_idx_(f, r & 31);
+          v = through(r, r == lp ? rjj : Xo[r * GJA_LD + lane], f);
+        }
+        put_cand(par ^ 1, k2, idx, fma_real_(lane == j + 1 ? y : v * y, pr));
+      }
+    } else if (wid == 4) {
+      const int r = jj + 1 - r0;
+      if (j + 1 < b && r >= 0 && r < nr) {
+        const bool at = r == lp;
+        put_rowjj(par ^ 1, through(r, at ? rjj : Xo[r * GJA_LD + lane],
+                                   at ? rjj_j : Xo[r * GJA_LD + j]));
+      }
+    } else {
+      const int mi = wid < 4 ? wid - 1 : wid - 2;
+      for (int rb = mi; rb < nr; rb += 4 * GJA_MAIN) {
+        T x[4], f[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const int r = rb + k * GJA_MAIN;
+          if (r < nr) {
+            x[k] = r == lp ? rjj : Xo[r * GJA_LD + lane];
+            f[k] = r == lp ? rjj_j : Xo[r * GJA_LD + j];
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const int r = rb + k * GJA_MAIN;
+          if (r < nr) Xn[r * GJA_LD + lane] = through(r, x[k], f[k]);
+        }
+      }
+    }
+  }
+  // the last pushes into a CTA's shared memory came before the last column's
+  // barrier, so none is on its way when a CTA leaves
+  __syncthreads();
+  const T* const Xl = Xs + ((b - 1) & 1) * slab;
+  for (int c = wid; c < b; c += nw)
+    for (int r = lane; r < nr; r += 32) Xp[r + (int64_t)c * a.ldx] = Xl[r * GJA_LD + c];
 }
 
 // For every column outside the panel [k0, k0 + b): apply the panel's row
@@ -340,26 +616,100 @@ __global__ void gje_perm_kernel(int n, const int* perm, int* iperm, const int* s
   }
 }
 
-// slab capacity of the panel kernel; the kernels' dynamic shared-memory
-// limits are raised once per type and device
+// slab capacity of the panel kernel, whose dynamic shared-memory limit is
+// raised once per type and device
 template <class T>
 static size_t gj_slab_cap() {
   static PerDevice<size_t> pd;
   return pd.get([] {
     cudaFuncAttributes fa;
     size_t stat = 16 * 1024;
-    if (cudaFuncGetAttributes(&fa, gje_panel_kernel<T, SYNC_GRID>) == cudaSuccess)
-      stat = fa.sharedSizeBytes;
-    if (cudaFuncGetAttributes(&fa, gje_panel_kernel<T, SYNC_CLUSTER>) == cudaSuccess &&
-        fa.sharedSizeBytes > stat)
-      stat = fa.sharedSizeBytes;
+    if (cudaFuncGetAttributes(&fa, gje_panel_kernel<T>) == cudaSuccess) stat = fa.sharedSizeBytes;
     const size_t cap = (size_t)max_smem_optin() - stat - 1024;
-    cudaFuncSetAttribute(gje_panel_kernel<T, SYNC_GRID>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap);
-    cudaFuncSetAttribute(gje_panel_kernel<T, SYNC_CLUSTER>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap);
+    cudaFuncSetAttribute(gje_panel_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)cap);
     return cap;
   });
+}
+
+// Launches the panel that runs one column ahead on G CTAs of ga.rpc rows; 1 if
+// it does not fit (shared memory, or the cluster or grid cannot be resident).
+template <class T, int SYNC, int NL>
+static int gje_ahead_launch_nl(cudaStream_t s, GjArgs<T>& ga, int G) {
+  auto kern = gje_panel_ahead_kernel<T, SYNC, NL>;
+  const size_t smem = 2 * (size_t)ga.rpc * GJA_LD * sizeof(T);
+  static PerDevice<int> pd;  // the dynamic shared memory the kernel may take (0: cannot run)
+  const int cap = pd.get([&] {
+    cudaFuncAttributes fa;
+    int v = 0;
+    if (cudaFuncGetAttributes(&fa, kern) == cudaSuccess) v = max_smem_optin() - (int)fa.sharedSizeBytes;
+    if (v <= 0 || cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, v) !=
+                      cudaSuccess)
+      v = 0;
+    if (SYNC == SYNC_CLUSTER && v > 0) {
+      // 16 CTAs at the largest slab this instance takes
+      cudaLaunchConfig_t c16 = {};
+      cudaLaunchAttribute at[1];
+      c16.gridDim = dim3(kGjClusterWide);
+      c16.blockDim = dim3(GJ_THREADS);
+      const size_t most = 2 * (size_t)32 * NL * GJA_LD * sizeof(T);
+      c16.dynamicSmemBytes = most < (size_t)v ? most : (size_t)v;
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = kGjClusterWide;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      c16.attrs = at;
+      c16.numAttrs = 1;
+      int nc = 0;
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+              cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&nc, kern, &c16) != cudaSuccess || nc < 1)
+        v = 0;
+    }
+    (void)cudaGetLastError();
+    return v;
+  });
+  if (smem > (size_t)cap) return 1;
+  if (SYNC == SYNC_GRID) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, GJ_THREADS, smem) !=
+            cudaSuccess ||
+        (int64_t)per_sm * num_sms() < G) {
+      (void)cudaGetLastError();
+      return 1;
+    }
+    ProfScope prof(s, PROF_GJ_PANEL, 2.0 * (double)ga.n * ga.b * sizeof(T));
+    note_launch();
+    void* args[] = {&ga};
+    MAK_CUDA_TRY(cudaLaunchCooperativeKernel((void*)kern, dim3((unsigned)G), dim3(GJ_THREADS),
+                                             args, smem, s));
+    return 0;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3((unsigned)G);
+  cfg.blockDim = dim3(GJ_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)G;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  ProfScope prof(s, PROF_GJ_PANEL, 2.0 * (double)ga.n * ga.b * sizeof(T));
+  note_launch();
+  MAK_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ga));
+  return 0;
+}
+template <class T, int SYNC>
+static int gje_ahead_launch(cudaStream_t s, GjArgs<T>& ga, int G) {
+  const int nl = (int)ceil_div(ga.rpc, 32);
+  if (nl <= 1) return gje_ahead_launch_nl<T, SYNC, 1>(s, ga, G);
+  if (nl <= 2) return gje_ahead_launch_nl<T, SYNC, 2>(s, ga, G);
+  if (nl <= 4) return gje_ahead_launch_nl<T, SYNC, 4>(s, ga, G);
+  if (nl <= 8) return gje_ahead_launch_nl<T, SYNC, 8>(s, ga, G);
+  return 1;
 }
 
 template <class T>
@@ -385,6 +735,7 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
   int* perm = ar.take<int>(n > 0 ? n : 1);
   // per-CTA pivot partials and candidate rows, double-buffered by column parity
   real_t<T>* part_val = ar.take<real_t<T>>(2 * sms);
+  unsigned long long* part_key = ar.take<unsigned long long>(2 * sms);
   int* part_idx = ar.take<int>(2 * sms);
   T* swapbuf = ar.take<T>(2 * GJ_NB);
   T* cand = ar.take<T>((size_t)2 * sms * GJ_NB);
@@ -414,39 +765,33 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
   // one 32-wide panel (cooperative launch, at most max_ctas CTAs: on the
   // look-ahead side stream it leaves the other SMs to the main stream)
   auto panel = [&](int64_t k0, int b, cudaStream_t s, int max_ctas) -> int {
-    GjArgs<T> ga{X, ldx, (int)n, (int)k0, b, 0, piv, part_val, part_idx, swapbuf,
+    GjArgs<T> ga{X, ldx, (int)n, (int)k0, b, 0, piv, part_val, part_key, part_idx, swapbuf,
                  cand, sms, bar, &info->status, &info->singular, skip_flag()};
-    // n <= 8 x 256: one thread-block cluster of at most 8 CTAs (>= 64 rows
-    // each); clusters of different streams run side by side
-    if (n <= (int64_t)kPanelClusterMax * GJ_CLUSTER_ROWS &&
-        (size_t)GJ_CLUSTER_ROWS * (b + 1) * sizeof(T) <= cap) {
-      int64_t G = ceil_div(n, 64);
-      if (G > kPanelClusterMax) G = kPanelClusterMax;
+    // The panel that runs one column ahead: one cluster of up to 16 CTAs (at
+    // least 32 rows each) up to the size where a column's elimination on 16 SMs
+    // (rows per CTA x 32, complex four times that) takes longer than a grid's
+    // round between its CTAs, about 4.5 us per column; beyond, a cooperative
+    // grid while a CTA's rows fit shared memory twice.  Per panel, cluster /
+    // grid: Float64 n = 3000 105 / 146 us, 4096 137 / 163 us (both beside the
+    // look-ahead's product); ComplexF64 n = 2048 204 / 184 us.
+    const int64_t cluster_max = traits<T>::cpx && sizeof(real_t<T>) == 8 ? 1536 : 4096;
+    if (n <= cluster_max) {
+      int64_t G = ceil_div(n, 32);
+      if (G > kGjClusterWide) G = kGjClusterWide;
       const int64_t rpc = ceil_div(n, G);
       G = ceil_div(n, rpc);
       ga.rpc = (int)rpc;
-      cudaLaunchConfig_t cfg = {};
-      cudaLaunchAttribute attr[1];
-      cfg.gridDim = dim3((unsigned)G);
-      cfg.blockDim = dim3(GJ_THREADS);
-      cfg.dynamicSmemBytes = (size_t)rpc * (b + 1) * sizeof(T);
-      cfg.stream = s;
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = (unsigned)G;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      int nclusters = 0;
-      if (cudaOccupancyMaxActiveClusters(&nclusters, gje_panel_kernel<T, SYNC_CLUSTER>, &cfg) ==
-              cudaSuccess &&
-          nclusters >= 1) {
-        ProfScope prof(s, PROF_GJ_PANEL, 2.0 * (double)n * b * sizeof(T));
-        note_launch();
-        MAK_CUDA_TRY(cudaLaunchKernelEx(&cfg, gje_panel_kernel<T, SYNC_CLUSTER>, ga));
-        return 0;
-      }
-      (void)cudaGetLastError();  // fall through to the cooperative grid
+      const int rc = gje_ahead_launch<T, SYNC_CLUSTER>(s, ga, (int)G);
+      if (rc != 1) return rc;
+    }
+    {
+      int64_t G = ceil_div(n, 32);
+      if (G > max_ctas) G = max_ctas;
+      const int64_t rpc = ceil_div(n, G);
+      G = ceil_div(n, rpc);
+      ga.rpc = (int)rpc;
+      const int rc = gje_ahead_launch<T, SYNC_GRID>(s, ga, (int)G);
+      if (rc != 1) return rc;
     }
     // grid: rows per CTA >= 64, at most one CTA per SM, slab within shared memory
     int64_t G = ceil_div(n, 64);
@@ -461,7 +806,7 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
     G = ceil_div(n, rpc);
     size_t smem = (size_t)rpc * (b + 1) * sizeof(T);
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gje_panel_kernel<T, SYNC_GRID>,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gje_panel_kernel<T>,
                                                       GJ_THREADS, smem) != cudaSuccess ||
         (int64_t)per_sm * sms < G)
       return MAK_ERR_UNSUPPORTED;
@@ -469,7 +814,7 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
     void* args[] = {&ga};
     ProfScope prof(s, PROF_GJ_PANEL, 2.0 * (double)n * b * sizeof(T));
     note_launch();
-    MAK_CUDA_TRY(cudaLaunchCooperativeKernel((void*)gje_panel_kernel<T, SYNC_GRID>,
+    MAK_CUDA_TRY(cudaLaunchCooperativeKernel((void*)gje_panel_kernel<T>,
                                              dim3((unsigned)G), dim3(GJ_THREADS), args, smem, s));
     return 0;
   };
