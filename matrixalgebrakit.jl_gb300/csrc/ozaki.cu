@@ -692,88 +692,103 @@ __device__ __forceinline__ bool oz_plain(const OzSrc<T>& s) {
 }
 
 
+// Largest component magnitude of an element, as IEEE bits
+__device__ __forceinline__ unsigned long long mag_bits(double x) { return absbits(x); }
+__device__ __forceinline__ unsigned long long mag_bits(zcomplex x) {
+  const unsigned long long a = absbits(x.re), b = absbits(x.im);
+  return a > b ? a : b;
+}
+// element (r, k) of the operand as stored (rows of op(A) / columns of op(B));
+// a conjugation changes no magnitude
+template <class T>
+__device__ __forceinline__ T oz_elem(const OzSrc<T>& s, int r, int k) {
+  return s.side == 0 ? load_op(s.op, r, k) : load_op(s.op, k, r);
+}
+
 // Row maxima of |X| as IEEE bit patterns (non-negative doubles order like
 // their bits), accumulated with atomicMax over a 2-D grid of (rows, K
-// chunks) so that tall K ranges are read by many CTAs in parallel.
-constexpr int OZ_EXP_KCHUNK = 1024;
+// chunks).  Complex operands are read once, as elements: a row's real and
+// imaginary parts share its exponent, and so do the two logical columns that
+// a column of op(B) becomes.  Eight loads in flight per thread; the K chunk
+// shrinks until the grid has two CTAs per SM (512 x 512 ComplexF64: 102 us
+// with 1024 of K walked by each thread).
 template <class T>
 __global__ void __launch_bounds__(256) oz_absmax_kernel(OzSrc<T> sa, int Ra,
                                                         unsigned long long* bits_a, OzSrc<T> sb,
                                                         int Rb, unsigned long long* bits_b, int K,
-                                                        const int* skip) {
+                                                        int kchunk, const int* skip) {
   if (skipped(skip)) return;
   // blockIdx.z: 0 the rows of op(A), 1 the columns of op(B)
   const OzSrc<T>& s = blockIdx.z == 0 ? sa : sb;
   const int R = blockIdx.z == 0 ? Ra : Rb;
   unsigned long long* mx_bits = blockIdx.z == 0 ? bits_a : bits_b;
-  const int k0 = blockIdx.y * OZ_EXP_KCHUNK;
-  const int k1 = min(K, k0 + OZ_EXP_KCHUNK);
-  if (oz_contig_r(s)) {
-    // 256 consecutive rows per CTA, each thread walks the chunk of K
-    const int r = blockIdx.x * 256 + threadIdx.x;
-    if (r >= R) return;
-    unsigned long long mx = 0;
-    int k = k0;
-    if (oz_plain(s)) {
-      // eight independent loads in flight per thread
-      const double* q = reinterpret_cast<const double*>(s.op.p) + r;
-      const int64_t ld = s.op.ld;
-      for (; k + 7 < k1; k += 8) {
-        unsigned long long b[8];
+  const int k0 = blockIdx.y * kchunk;
+  const int k1 = min(K, k0 + kchunk);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const bool cr = oz_contig_r(s);
+  // contiguous along r: 32 rows per CTA (lane = row), the warps share K; else
+  // 8 rows per CTA, a warp per row, lanes along K
+  const int r = cr ? blockIdx.x * 32 + lane : blockIdx.x * 8 + wid;
+  const int kf = k0 + (cr ? wid : lane), ks = cr ? 8 : 32;
+  unsigned long long mx = 0;
+  if (r < R) {
+    int k = kf;
+    if (s.op.mask == MASK_FULL) {
+      const T* q = s.op.p + (cr ? (int64_t)r : (int64_t)r * s.op.ld);
+      const int64_t st = cr ? s.op.ld : 1;
+      for (; k + 7 * ks < k1; k += 8 * ks) {
+        T v[8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) b[i] = absbits(q[(int64_t)(k + i) * ld]);
+        for (int i = 0; i < 8; i++) v[i] = q[(int64_t)(k + i * ks) * st];
 #pragma unroll
-        for (int i = 0; i < 8; i++) mx = b[i] > mx ? b[i] : mx;
+        for (int i = 0; i < 8; i++) {
+          const unsigned long long b = mag_bits(v[i]);
+          mx = b > mx ? b : mx;
+        }
       }
     }
-    for (; k < k1; k++) {
-      const unsigned long long b = absbits(oz_fetch(s, r, k));
+#pragma unroll 4
+    for (; k < k1; k += ks) {
+      const unsigned long long b = mag_bits(oz_elem(s, r, k));
       mx = b > mx ? b : mx;
     }
-    if (mx) atomicMax(&mx_bits[r], mx);
+  }
+  if (cr) {
+    __shared__ unsigned long long part[8][32];
+    part[wid][lane] = mx;
+    __syncthreads();
+    if (wid != 0) return;
+#pragma unroll
+    for (int w = 1; w < 8; w++) mx = part[w][lane] > mx ? part[w][lane] : mx;
   } else {
-    // 8 rows per CTA, one warp per row, lanes along K
-    const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (r >= R) return;
-    unsigned long long mx = 0;
-    int k = k0 + lane;
-    if (oz_plain(s)) {
-      const double* q = reinterpret_cast<const double*>(s.op.p) + (int64_t)r * s.op.ld;
-      for (; k + 7 * 32 < k1; k += 8 * 32) {
-        unsigned long long b[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) b[i] = absbits(q[k + 32 * i]);
-#pragma unroll
-        for (int i = 0; i < 8; i++) mx = b[i] > mx ? b[i] : mx;
-      }
-    }
-    for (; k < k1; k += 32) {
-      const unsigned long long b = absbits(oz_fetch(s, r, k));
-      mx = b > mx ? b : mx;
-    }
 #pragma unroll
     for (int m = 16; m > 0; m >>= 1) {
-      unsigned long long o = __shfl_xor_sync(0xffffffffu, mx, m);
+      const unsigned long long o = __shfl_xor_sync(0xffffffffu, mx, m);
       mx = o > mx ? o : mx;
     }
-    if (lane == 0 && mx) atomicMax(&mx_bits[r], mx);
+    if (lane != 0) return;
+  }
+  if (r < R && mx) {
+    atomicMax(&mx_bits[r], mx);
+    if (traits<T>::cpx && s.side == 1) atomicMax(&mx_bits[r + R], mx);
   }
 }
-// Row maxima of both operands in one launch into bits_a[0, Ra) and
-// bits_b[0, Rb); the nbits words from bits_a on (which hold both) are
-// zeroed first
+// Row maxima of both operands in one launch into bits_a (rows of op(A)) and
+// bits_b (logical columns of op(B)); the nbits words from bits_a on (which
+// hold both) are zeroed first.  Ra, Rb and K count elements as stored.
 template <class T>
 static int oz_exponents(cudaStream_t st, const OzSrc<T>& sa, int Ra, unsigned long long* bits_a,
                         const OzSrc<T>& sb, int Rb, unsigned long long* bits_b, int K,
                         int64_t nbits) {
   MAK_CUDA_TRY(cudaMemsetAsync(bits_a, 0, (size_t)nbits * sizeof(unsigned long long), st));
-  const unsigned gy = (unsigned)ceil_div(K > 0 ? K : 1, OZ_EXP_KCHUNK);
-  const int64_t gxa = oz_contig_r(sa) ? ceil_div(Ra, 256) : ceil_div(Ra, 8);
-  const int64_t gxb = oz_contig_r(sb) ? ceil_div(Rb, 256) : ceil_div(Rb, 8);
+  const int64_t gxa = oz_contig_r(sa) ? ceil_div(Ra, 32) : ceil_div(Ra, 8);
+  const int64_t gxb = oz_contig_r(sb) ? ceil_div(Rb, 32) : ceil_div(Rb, 8);
   const unsigned gx = (unsigned)(gxa > gxb ? gxa : gxb);
+  int kchunk = 1024;
+  while (kchunk > 64 && (gxa + gxb) * ceil_div(K, kchunk) < 2 * (int64_t)num_sms()) kchunk /= 2;
+  const unsigned gy = (unsigned)ceil_div(K > 0 ? K : 1, kchunk);
   note_launch();
-  oz_absmax_kernel<T><<<dim3(gx, gy, 2), 256, 0, st>>>(sa, Ra, bits_a, sb, Rb, bits_b, K,
+  oz_absmax_kernel<T><<<dim3(gx, gy, 2), 256, 0, st>>>(sa, Ra, bits_a, sb, Rb, bits_b, K, kchunk,
                                                         skip_flag());
   return cudaGetLastError() == cudaSuccess ? 0 : MAK_ERR_CUDA;
 }
@@ -1035,7 +1050,7 @@ int oz_gemm(cudaStream_t st, int64_t M, int64_t N, int64_t K, T alpha, Operand<T
 
   OzSrc<T> sa{A, 0, (int)M, (int)K};
   OzSrc<T> sb{B, 1, (int)N, (int)K};
-  MAK_TRY(oz_exponents<T>(st, sa, (int)M, bitsA, sb, (int)Nl, bitsB, (int)Kl, Mpad + Npad));
+  MAK_TRY(oz_exponents<T>(st, sa, (int)M, bitsA, sb, (int)N, bitsB, (int)K, Mpad + Npad));
   {
     const OzPlaneOut oa{(int)M, (int)Mpad, bitsA, PA}, ob{(int)Nl, (int)Npad, bitsB, PB};
     const int64_t rows = Mpad > Npad ? Mpad : Npad;
