@@ -171,6 +171,22 @@ __device__ __forceinline__ double rsqrt_b3(double x) {
   return fma(y0 * r, fma(r, 0.375, 0.5), y0);
 }
 __device__ __forceinline__ float rsqrt_b3(float x) { return 1.0f / sqrtf(x); }
+// 1 / z by the same series (complex: conj(z) / |z|^2, |z|^2 within range)
+__device__ __forceinline__ double inv_b3(double z) {
+  const double y = rcp_seed(z), r = fma(-z, y, 1.0);
+  return fma(y, fma(r, r, r), y);
+}
+__device__ __forceinline__ float inv_b3(float z) { return 1.0f / z; }
+template <class R> __device__ __forceinline__ cplx<R> inv_b3(cplx<R> z) {
+  const R d = inv_b3(fma_(z.re, z.re, z.im * z.im));
+  return {z.re * d, -z.im * d};
+}
+// the larger component's magnitude
+__device__ __forceinline__ double abs_max_(double z) { return fabs(z); }
+__device__ __forceinline__ float abs_max_(float z) { return fabsf(z); }
+template <class R> __device__ __forceinline__ R abs_max_(cplx<R> z) {
+  return fmax(fabs(z.re), fabs(z.im));
+}
 // w (1 + p) for a real p
 __device__ __forceinline__ double fma_real_(double w, double p) { return fma(w, p, w); }
 __device__ __forceinline__ float fma_real_(float w, float p) { return fmaf(w, p, w); }

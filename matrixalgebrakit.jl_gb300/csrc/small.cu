@@ -51,15 +51,108 @@ __host__ __device__ size_t small_qr_bytes(int dtype, int64_t m, int64_t n) {
   return (size_t)(m * n + 2 * k) * es;  // the block, tau and the gauge signs
 }
 
+// Measured (Float64, one block): 128 x 64 in about 630 us, of which 255 us is
+// the FP64 pipe's floor on one SM; 400 blocks of up to 128 x 64 1818 -> 775 us
+// against eight warps with a warp and its butterfly sums per column.
+// The QR's CTA: four warps, one per SM sub-partition.  One warp already holds
+// its sub-partition's FP64 pipe (a warp-wide operation every 64 cycles,
+// dependent or not), so more warps would only repeat the scalar work.
+constexpr int SMALL_QR_THREADS = 128;
+constexpr int SMALL_QR_WARPS = SMALL_QR_THREADS / 32;
+constexpr int SMALL_CHUNK_MAX = 256;
+
+// Scratch of the dot products: `chunk` columns are combined together, as many
+// as fit the shared memory the block leaves free, at least the static 32.
+template <class T>
+struct SmallQrScratch {
+  T* part;   // [SMALL_QR_WARPS][chunk] the warps' partial dot products
+  T* fs;     // [chunk] the updates of the rows below row j
+  unsigned long long* key;  // [SMALL_QR_WARPS]
+  int chunk;
+};
+constexpr int SMALL_STATIC_CHUNK = 32;
+constexpr int SMALL_QR_THIRD = 72 * 1024;  // three CTAs per SM
+
+// magnitudes for which neither a product x a (|a| up to the type's range over
+// this window) nor a sum of squares leaves the range
+__device__ __forceinline__ bool small_in_window(double v) { return v > 0x1p-100 && v < 0x1p100; }
+__device__ __forceinline__ bool small_in_window(float v) { return v > 0x1p-20f && v < 0x1p20f; }
+
+// this warp's partial dot products d_c = sum_r conj(x_r) S[r, c] over its
+// slice of the rows j+1 .. m-1, for the columns c0 .. c0 + nc - 1: lane =
+// column, so that no cross-lane sums are needed (five FP64 additions per
+// column against one multiply-add per 32 rows)
+template <class T>
+__device__ __forceinline__ void small_dots(const T* S, int ld, int m, int j, const T* x, int c0,
+                                           int nc, SmallQrScratch<T>& q) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int rows = m - (j + 1);
+  const int per = (rows + SMALL_QR_WARPS - 1) / SMALL_QR_WARPS;
+  const int ra = j + 1 + wid * per, rb = min(m, ra + per);
+  for (int g = 0; g < nc; g += 32) {
+    const int c = c0 + min(g + lane, nc - 1);
+    const T* pc = S + c * ld;
+    T s0 = zero_<T>(), s1 = zero_<T>(), s2 = zero_<T>(), s3 = zero_<T>();
+    int r = ra;
+    for (; r + 3 < rb; r += 4) {
+      const T x0 = x[r], x1 = x[r + 1], x2 = x[r + 2], x3 = x[r + 3];
+      const T a0 = pc[r], a1 = pc[r + 1], a2 = pc[r + 2], a3 = pc[r + 3];
+      s0 = fma_(conj_(x0), a0, s0);
+      s1 = fma_(conj_(x1), a1, s1);
+      s2 = fma_(conj_(x2), a2, s2);
+      s3 = fma_(conj_(x3), a3, s3);
+    }
+    for (; r < rb; r++) s0 = fma_(conj_(x[r]), pc[r], s0);
+    q.part[wid * q.chunk + g + lane] = (s0 + s1) + (s2 + s3);
+  }
+}
+template <class T>
+__device__ __forceinline__ T small_sum(const SmallQrScratch<T>& q, int c) {
+  const int n = q.chunk;
+  return (q.part[c] + q.part[n + c]) + (q.part[2 * n + c] + q.part[3 * n + c]);
+}
+// S[r, c] -= x_r fs_c (r > j) for the columns c0 + first .. c0 + nc - 1: a
+// warp per column, lanes along the rows
+template <class T>
+__device__ __forceinline__ void small_update(T* S, int ld, int m, int j, const T* x, int c0,
+                                             int first, int nc, const SmallQrScratch<T>& q) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // 32 rows at a time, the reflector's values in registers, four columns per
+  // step: all loads before the stores, which the compiler cannot reorder
+  for (int r = j + 1 + lane; r - lane < m; r += 32) {
+    const bool in = r < m;
+    const T xr = in ? x[r] : zero_<T>();
+    int e = first + wid;
+    for (; e + 3 * SMALL_QR_WARPS < nc; e += 4 * SMALL_QR_WARPS) {
+      T* pc = S + (c0 + e) * ld + r;
+      T a[4], f[4];
+#pragma unroll
+      for (int q4 = 0; q4 < 4; q4++) {
+        f[q4] = q.fs[e + q4 * SMALL_QR_WARPS];
+        a[q4] = in ? pc[q4 * SMALL_QR_WARPS * ld] : zero_<T>();
+      }
+#pragma unroll
+      for (int q4 = 0; q4 < 4; q4++) {
+        const T y = fma_(-xr, f[q4], a[q4]);
+        if (in) pc[q4 * SMALL_QR_WARPS * ld] = y;
+      }
+    }
+    for (; e < nc; e += SMALL_QR_WARPS)
+      if (in) {
+        T* pc = S + (c0 + e) * ld + r;
+        *pc = fma_(-xr, q.fs[e], *pc);
+      }
+  }
+}
+
 template <class T>
 __device__ void small_qr_item(const mak_batch_item& it, int positive, mak_info* info,
-                              unsigned char* dyn, int cap_bytes, SmallScratch& sh) {
+                              unsigned char* dyn, int cap_bytes, unsigned char* stat) {
   using R = real_t<T>;
   using NK = NormKey<R>;
-  using Key = typename NK::K;
   const int64_t m64 = it.m, n64 = it.n;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
-  const int bd = blockDim.x;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  constexpr int nw = SMALL_QR_WARPS, bd = SMALL_QR_THREADS;
   if (tid == 0) {
     info->status = 0;
     info->iterations = 0;
@@ -77,133 +170,174 @@ __device__ void small_qr_item(const mak_batch_item& it, int positive, mak_info* 
   }
   const int m = (int)m64, n = (int)n64, k = m < n ? m : n;
   if (k == 0) return;
+  // an odd leading dimension (lanes along the columns then fall on distinct
+  // banks) where the padded block fits
+  const int ld = ((size_t)(m | 1) * n + 2 * k) * sizeof(T) <= (size_t)cap_bytes ? (m | 1) : m;
   const T* A = (const T*)it.A;
-  T* S = reinterpret_cast<T*>(dyn);  // m x n, ld m
-  T* taus = S + (int64_t)m * n;      // k
+  T* S = reinterpret_cast<T*>(dyn);  // m x n, leading dimension ld
+  T* taus = S + (int64_t)ld * n;     // k
   T* sgn = taus + k;                 // k
-  for (int c = 0; c < n; c++)
-    for (int r = tid; r < m; r += bd) S[r + c * m] = A[r + (int64_t)c * it.lda];
+  SmallQrScratch<T> sh;
+  sh.key = reinterpret_cast<unsigned long long*>(stat);
+  sh.part = reinterpret_cast<T*>(stat + 8 * SMALL_QR_WARPS);
+  sh.chunk = SMALL_STATIC_CHUNK;
+  {
+    const size_t used = ((size_t)(sgn + k - S) * sizeof(T) + 15) / 16 * 16;
+    for (int ch = SMALL_CHUNK_MAX; ch > SMALL_STATIC_CHUNK; ch /= 2)
+      if (used + (size_t)(SMALL_QR_WARPS + 1) * ch * sizeof(T) <= (size_t)cap_bytes) {
+        sh.part = reinterpret_cast<T*>(dyn + used);
+        sh.chunk = ch;
+        break;
+      }
+  }
+  sh.fs = sh.part + SMALL_QR_WARPS * sh.chunk;
+  for (int c = wid; c < n; c += 4 * nw)
+    for (int r = lane; r < m; r += 32) {
+      T v[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (c + q * nw < n) v[q] = A[r + (int64_t)(c + q * nw) * it.lda];
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (c + q * nw < n) S[r + (c + q * nw) * ld] = v[q];
+    }
   __syncthreads();
 
-  // ---- factorization: one reflector per column
-  R* red_r = reinterpret_cast<R*>(sh.red_r);
-  Key* red_k = reinterpret_cast<Key*>(sh.red_k);
-  T* sc = reinterpret_cast<T*>(sh.sc);
+  // ---- factorization: one reflector per column.  The dot products of the
+  // unscaled column x with itself and the columns to its right come first;
+  // with beta, tau = 1 - alpha / beta and tau scal = -1 / beta (scal = 1 /
+  // (alpha - beta)), row j's update is f_c = conj(tau) A[j, c] - d_c / beta
+  // and the rows below take x_r (scal f_c): the column itself is scaled
+  // beside the next column's work.
   for (int j = 0; j < k; j++) {
-    T* col = S + j * m;
-    // sum of squares and largest magnitude of x = column j below the diagonal
-    R ss = R(0);
-    Key mk = 0;
-    for (int r = j + 1 + tid; r < m; r += bd) {
-      const T x = col[r];
-      ss = sq_add(ss, x);
-      const Key q = mag_key(x);
-      mk = q > mk ? q : mk;
-    }
-    ss = warp_sum(ss);
-    mk = warp_max_key(mk);
-    if (lane == 0) {
-      red_r[wid] = ss;
-      red_k[wid] = mk;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      R s2 = R(0);
-      Key m2 = 0;
-      for (int w = 0; w < nw; w++) {
-        s2 += red_r[w];
-        m2 = red_k[w] > m2 ? red_k[w] : m2;
+    T* x = S + j * ld;
+    bool scaled = false;  // x already holds v (rescaled path)
+    T beta = zero_<T>(), tau = zero_<T>(), scal = one_<T>();
+    R rb = R(0);          // 1 / beta (fast path)
+    bool fast = false;
+    for (int c0 = j; c0 < n; c0 += sh.chunk) {
+      const int nc = min(sh.chunk, n - c0);
+      if (c0 == j) {
+        // largest magnitude of x (the slice's, lanes along the rows)
+        typename NK::K mk = 0;
+        for (int r = j + 1 + tid; r < m; r += bd) {
+          const typename NK::K q = mag_key(x[r]);
+          mk = q > mk ? q : mk;
+        }
+        mk = warp_max_key(mk);
+        if (lane == 0) sh.key[wid] = (unsigned long long)mk;
       }
-      sh.sc_r[0] = (double)s2;
-      sh.sc_r[1] = (double)NK::val(m2);
-      sh.sc_flag = norm_needs_rescale<R>(m2);
+      small_dots(S, ld, m, j, x, c0, nc, sh);
+      __syncthreads();
+      if (c0 == j) {
+        // every warp repeats the scalars (each on its own FP64 pipe)
+        unsigned long long mk = sh.key[0];
+#pragma unroll
+        for (int w = 1; w < nw; w++) mk = sh.key[w] > mk ? sh.key[w] : mk;
+        const R amax = NK::val((typename NK::K)mk);
+        const T alpha = x[j];
+        if (small_in_window(amax) && (!(abs2_(alpha) > R(0)) || small_in_window(abs_max_(alpha)))) {
+          const R ssq = re_(small_sum(sh, 0));
+          const R n2 = sq_add(ssq, alpha);
+          const R rs = rsqrt_b3(n2);
+          R nrm = n2 * rs;
+          nrm = fma_(fma_(-nrm, nrm, n2), R(0.5) * rs, nrm);
+          const bool up = re_(alpha) >= R(0);
+          const R bt = up ? -nrm : nrm;
+          rb = up ? -rs : rs;
+          beta = make_scalar<T>(bt, R(0));
+          tau = one_<T>() - alpha * rb;
+          scal = inv_b3(alpha - beta);
+          fast = true;
+        } else if (amax < R(INFINITY) && amax > R(0)) {
+          // rare: outside the window, the norm of x scaled by 2^-e, e the
+          // exponent of the largest magnitude (clamped); v first, then its
+          // dot products
+          int e = 0;
+          frexp(amax, &e);
+          e = e > 1000 ? 1000 : (e < -1000 ? -1000 : e);
+          const R scale = ldexp(R(1), -e);
+          R s3 = R(0);
+          for (int r = j + 1 + lane; r < m; r += 32) ssq_scaled_add(s3, x[r], scale);
+          s3 = warp_sum(s3);
+          larfg_scalars(alpha, sqrt(s3) * ldexp(R(1), e), beta, tau, scal);
+          scaled = true;
+        } else {
+          larfg_scalars_ssq(alpha, re_(small_sum(sh, 0)), amax, beta, tau, scal);
+        }
+        if (scaled) {
+          __syncthreads();
+          for (int r = j + 1 + tid; r < m; r += bd) x[r] = x[r] * scal;
+          __syncthreads();
+          small_dots(S, ld, m, j, x, c0, nc, sh);
+          __syncthreads();
+        }
+      }
+      for (int e = wid * 32 + lane; e < nc; e += bd) {
+        if (c0 + e <= j) continue;
+        const T d = small_sum(sh, e), a = S[j + (c0 + e) * ld];
+        T f;
+        if (fast) f = conj_(tau) * a - d * rb;
+        else f = conj_(tau) * (scaled ? a + d : fma_(conj_(scal), d, a));
+        sh.fs[e] = scaled ? f : f * scal;
+        S[j + (c0 + e) * ld] = a - f;
+      }
+      __syncthreads();
+      small_update(S, ld, m, j, x, c0, c0 == j ? 1 : 0, nc, sh);
+      __syncthreads();
     }
-    __syncthreads();
-    R xnorm = R(0);
-    const bool rescale = sh.sc_flag != 0;
-    if (rescale) {
-      // rare: the squares would overflow or underflow; sum them scaled by
-      // 2^-e, e the exponent of the largest magnitude (clamped)
-      int e = 0;
-      frexp((R)sh.sc_r[1], &e);
-      e = e > 1000 ? 1000 : (e < -1000 ? -1000 : e);
-      const R scale = ldexp(R(1), -e);
-      R s3 = R(0);
-      for (int r = j + 1 + tid; r < m; r += bd) ssq_scaled_add(s3, col[r], scale);
-      s3 = block_sum(s3, red_r);
-      xnorm = sqrt(s3) * ldexp(R(1), e);
-    }
+    if (!scaled)
+      for (int r = j + 1 + tid; r < m; r += bd) x[r] = x[r] * scal;
     if (tid == 0) {
-      T beta, tau, scal;
-      if (rescale) larfg_scalars(col[j], xnorm, beta, tau, scal);
-      else larfg_scalars_ssq(col[j], (R)sh.sc_r[0], (R)sh.sc_r[1], beta, tau, scal);
-      sc[0] = beta;
-      sc[1] = tau;
-      sc[2] = scal;
+      x[j] = beta;
       taus[j] = tau;
     }
-    __syncthreads();
-    const T beta = sc[0], tau = sc[1], scal = sc[2];
-    for (int r = j + 1 + tid; r < m; r += bd) col[r] = col[r] * scal;
-    __syncthreads();
-    // H_j^H on the columns to the right: w_c = A[j,c] + sum_{r>j} conj(v_r)
-    // A[r,c], A[:,c] -= v conj(tau) w_c (v_j = 1); a warp per column
-    for (int c = j + 1 + wid; c < n; c += nw) {
-      T* pc = S + c * m;
-      const T ajc = pc[j];
-      T acc = zero_<T>();
-      for (int r = j + 1 + lane; r < m; r += 32) acc = fma_(conj_(col[r]), pc[r], acc);
-      acc = warp_sum(acc);
-      const T f = conj_(tau) * (ajc + acc);
-      __syncwarp();
-      if (lane == 0) pc[j] = ajc - f;
-      for (int r = j + 1 + lane; r < m; r += 32) pc[r] = fma_(-col[r], f, pc[r]);
-    }
-    if (tid == 0) col[j] = beta;
-    __syncthreads();
   }
+  __syncthreads();
 
   // ---- R with the gauge: R[i, c] = conj(s_i) A[i, c] (i <= c), 0 below
-  for (int i = tid; i < k; i += bd) sgn[i] = positive ? sign_safe_(S[i + i * m]) : one_<T>();
+  for (int i = tid; i < k; i += bd) sgn[i] = positive ? sign_safe_(S[i + i * ld]) : one_<T>();
   __syncthreads();
   if (it.R != nullptr) {
     T* Rout = (T*)it.R;
-    for (int c = 0; c < n; c++)
-      for (int i = tid; i < k; i += bd)
-        Rout[i + (int64_t)c * it.ldr] = (i <= c) ? conj_(sgn[i]) * S[i + c * m] : zero_<T>();
+    for (int c = wid; c < n; c += nw)
+      for (int i = lane; i < k; i += 32)
+        Rout[i + (int64_t)c * it.ldr] = (i <= c) ? conj_(sgn[i]) * S[i + c * ld] : zero_<T>();
   }
   __syncthreads();
 
   // ---- Q = H_0 ... H_{k-1} [I_k; 0], formed in place over the reflectors
   for (int j = k - 1; j >= 0; j--) {
-    T* col = S + j * m;
+    T* v = S + j * ld;
     const T tau = taus[j];
     // H_j on the columns c in (j, k): rows >= j (rows < j are zero there)
-    for (int c = j + 1 + wid; c < k; c += nw) {
-      T* pc = S + c * m;
-      const T qj = pc[j];
-      T acc = zero_<T>();
-      for (int r = j + 1 + lane; r < m; r += 32) acc = fma_(conj_(col[r]), pc[r], acc);
-      acc = warp_sum(acc);
-      const T f = tau * (qj + acc);
-      __syncwarp();
-      if (lane == 0) pc[j] = qj - f;
-      for (int r = j + 1 + lane; r < m; r += 32) pc[r] = fma_(-col[r], f, pc[r]);
+    for (int c0 = j + 1; c0 < k; c0 += sh.chunk) {
+      const int nc = min(sh.chunk, k - c0);
+      small_dots(S, ld, m, j, v, c0, nc, sh);
+      __syncthreads();
+      for (int e = tid; e < nc; e += bd) {
+        const T a = S[j + (c0 + e) * ld];
+        const T f = tau * (a + small_sum(sh, e));
+        sh.fs[e] = f;
+        S[j + (c0 + e) * ld] = a - f;
+      }
+      __syncthreads();
+      small_update(S, ld, m, j, v, c0, 0, nc, sh);
+      __syncthreads();
     }
-    __syncthreads();
     // column j of Q: e_j - tau v
     for (int r = tid; r < m; r += bd) {
       T q;
       if (r < j) q = zero_<T>();
       else if (r == j) q = one_<T>() - tau;
-      else q = -(tau * col[r]);
-      col[r] = q;
+      else q = -(tau * v[r]);
+      v[r] = q;
     }
     __syncthreads();
   }
   T* Qout = (T*)it.Q;
-  for (int c = 0; c < k; c++)
-    for (int r = tid; r < m; r += bd) Qout[r + (int64_t)c * it.ldq] = S[r + c * m] * sgn[c];
+  for (int c = wid; c < k; c += nw)
+    for (int r = lane; r < m; r += 32) Qout[r + (int64_t)c * it.ldq] = S[r + c * ld] * sgn[c];
 }
 
 // ---------------------------------------------------------------- polar --
@@ -556,35 +690,44 @@ small_polar_device_kernel(const mak_batch_item* items, int count, int maxiter, d
 }
 
 __device__ void small_qr_dispatch(const mak_batch_item& it, int positive, mak_info* info,
-                                  unsigned char* dyn, int cap_bytes, SmallScratch& sh) {
+                                  unsigned char* dyn, int cap_bytes) {
+  // keys and the smallest dot-product scratch, sized for the widest type
+  __shared__ __align__(16) unsigned char
+      stat[8 * SMALL_QR_WARPS + sizeof(zcomplex) * (SMALL_QR_WARPS + 1) * SMALL_STATIC_CHUNK];
   switch (it.dtype) {
-    case MAK_F64: small_qr_item<double>(it, positive, info, dyn, cap_bytes, sh); break;
-    case MAK_C64: small_qr_item<zcomplex>(it, positive, info, dyn, cap_bytes, sh); break;
-    case MAK_F32: small_qr_item<float>(it, positive, info, dyn, cap_bytes, sh); break;
-    case MAK_C32: small_qr_item<ccomplex>(it, positive, info, dyn, cap_bytes, sh); break;
+    case MAK_F64: small_qr_item<double>(it, positive, info, dyn, cap_bytes, stat); break;
+    case MAK_C64: small_qr_item<zcomplex>(it, positive, info, dyn, cap_bytes, stat); break;
+    case MAK_F32: small_qr_item<float>(it, positive, info, dyn, cap_bytes, stat); break;
+    case MAK_C32: small_qr_item<ccomplex>(it, positive, info, dyn, cap_bytes, stat); break;
     default:
       if (threadIdx.x == 0) info->status = MAK_ERR_UNSUPPORTED;
   }
   __syncthreads();  // the shared block is reused by the next item
 }
 
-__global__ void __launch_bounds__(SMALL_THREADS)
+// Items of more than lo_bytes up to the launch's cap_bytes (and, with all set,
+// those beyond it, which report MAK_ERR_UNSUPPORTED)
+__device__ __forceinline__ bool small_qr_mine(const mak_batch_item& it, int lo_bytes,
+                                              int cap_bytes, int all) {
+  if (it.m < 0 || it.n < 0) return all != 0;
+  const int64_t need = (int64_t)small_qr_bytes(it.dtype, it.m, it.n);
+  return need > lo_bytes && (all || need <= cap_bytes);
+}
+__global__ void __launch_bounds__(SMALL_QR_THREADS)
 small_qr_list_kernel(const __grid_constant__ SmallList L, int positive, mak_info* infos,
                      int cap_bytes) {
   extern __shared__ __align__(16) unsigned char small_dyn[];
-  __shared__ SmallScratch sh;
   for (int q = blockIdx.x; q < L.count; q += gridDim.x)
-    small_qr_dispatch(L.items[q], positive, infos + L.idx[q], small_dyn, cap_bytes, sh);
+    small_qr_dispatch(L.items[q], positive, infos + L.idx[q], small_dyn, cap_bytes);
 }
 
-__global__ void __launch_bounds__(SMALL_THREADS)
+__global__ void __launch_bounds__(SMALL_QR_THREADS)
 small_qr_device_kernel(const mak_batch_item* items, int count, int positive, mak_info* infos,
-                       int cap_bytes) {
+                       int lo_bytes, int cap_bytes, int all) {
   extern __shared__ __align__(16) unsigned char small_dyn[];
-  __shared__ SmallScratch sh;
-  for (int q = blockIdx.x; q < count; q += gridDim.x) {
-    small_qr_dispatch(items[q], positive, infos + q, small_dyn, cap_bytes, sh);
-  }
+  for (int q = blockIdx.x; q < count; q += gridDim.x)
+    if (small_qr_mine(items[q], lo_bytes, cap_bytes, all))
+      small_qr_dispatch(items[q], positive, infos + q, small_dyn, cap_bytes);
 }
 
 // the largest dynamic shared memory of the small-block kernels on this
@@ -595,7 +738,7 @@ static int small_smem_limit() {
     cudaFuncAttributes fa;
     size_t stat = 4096;
     if (cudaFuncGetAttributes(&fa, small_qr_list_kernel) == cudaSuccess) stat = fa.sharedSizeBytes;
-    const int cap = max_smem_optin() - (int)stat - 1024;
+    const int cap = max_smem_optin() - (int)stat;
     cudaFuncSetAttribute(small_qr_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
     cudaFuncSetAttribute(small_qr_device_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          cap);
@@ -649,21 +792,32 @@ int small_polar_launch(cudaStream_t st, const mak_batch_item* items, const int* 
   return 0;
 }
 
-// one persistent launch (per SMALL_LIST_MAX items) over the listed items
+// one persistent launch (per SMALL_LIST_MAX items and shared-memory class)
+// over the listed items: the blocks that fit a third of an SM's shared memory
+// run three CTAs per SM
 int small_qr_launch(cudaStream_t st, const mak_batch_item* items, const int* which, int count,
                     int positive, mak_info* infos, int cap) {
   static thread_local SmallList L;
-  for (int q0 = 0; q0 < count; q0 += SMALL_LIST_MAX) {
-    const int cnt = (count - q0) < SMALL_LIST_MAX ? (count - q0) : SMALL_LIST_MAX;
-    L.count = cnt;
-    for (int q = 0; q < cnt; q++) {
-      L.items[q] = items[which[q0 + q]];
-      L.idx[q] = which[q0 + q];
+  for (int cls = 0; cls < 2; cls++) {
+    const int smem = cls == 0 ? cap : (cap > SMALL_QR_THIRD ? SMALL_QR_THIRD : 0);
+    const int64_t most = cls == 0 ? num_sms() : 3 * (int64_t)num_sms();
+    L.count = 0;
+    for (int q = 0; q <= count; q++) {
+      if (q < count) {
+        const mak_batch_item& it = items[which[q]];
+        const bool third = cap > SMALL_QR_THIRD &&
+                           small_qr_bytes(it.dtype, it.m, it.n) <= (size_t)SMALL_QR_THIRD;
+        if (third != (cls == 1)) continue;
+        L.items[L.count] = it;
+        L.idx[L.count++] = which[q];
+      }
+      if (L.count == 0 || (q < count && L.count < SMALL_LIST_MAX)) continue;
+      note_launch();
+      small_qr_list_kernel<<<(int)(L.count < most ? L.count : most), SMALL_QR_THREADS, smem, st>>>(
+          L, positive, infos, smem);
+      MAK_CUDA_TRY(cudaGetLastError());
+      L.count = 0;
     }
-    const int grid = cnt < num_sms() ? cnt : num_sms();
-    note_launch();
-    small_qr_list_kernel<<<grid, SMALL_THREADS, cap, st>>>(L, positive, infos, cap);
-    MAK_CUDA_TRY(cudaGetLastError());
   }
   return 0;
 }
@@ -682,10 +836,21 @@ extern "C" int mak_batched_qr_compact_device(const mak_batch_item* items, int ni
   if (nitems == 0) return 0;
   const int cap = small_qr_cap();
   if (cap <= 0) return MAK_ERR_UNSUPPORTED;
-  const int grid = nitems < num_sms() ? nitems : num_sms();
+  // The host does not see the blocks' sizes: one launch per shared-memory
+  // class, the blocks that fit a third of an SM's first (three CTAs per SM
+  // hide each other's scalar steps), each CTA passing over the other class.
+  cudaStream_t st = (cudaStream_t)stream;
+  const int lo = cap > SMALL_QR_THIRD ? SMALL_QR_THIRD : 0;
+  if (lo > 0) {
+    const int64_t most = 3 * (int64_t)num_sms();
+    note_launch();
+    small_qr_device_kernel<<<(int)(nitems < most ? nitems : most), SMALL_QR_THREADS, lo, st>>>(
+        items, nitems, opts->positive, infos, -1, lo, 0);
+    MAK_CUDA_TRY(cudaGetLastError());
+  }
   note_launch();
-  small_qr_device_kernel<<<grid, SMALL_THREADS, cap, (cudaStream_t)stream>>>(
-      items, nitems, opts->positive, infos, cap);
+  small_qr_device_kernel<<<nitems < num_sms() ? nitems : num_sms(), SMALL_QR_THREADS, cap, st>>>(
+      items, nitems, opts->positive, infos, lo > 0 ? lo : -1, cap, 1);
   return cudaGetLastError() == cudaSuccess ? 0 : MAK_ERR_CUDA;
 }
 
