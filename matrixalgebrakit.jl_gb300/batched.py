@@ -13,6 +13,7 @@ from __future__ import annotations
 import ctypes as ct
 import warnings
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -22,15 +23,88 @@ from .core import (DTYPE_CODE, INFO_BYTES, check_cuda_tensor, check_rc, empty_cm
 from .qr import PRECISION_CODE
 
 
-def _items(As, outs):
-    arr = (_lib.mak_batch_item * len(As))()
-    for i, (A, (Q, R)) in enumerate(zip(As, outs)):
+def _ptr_ld(X, name):
+    m, n = X.shape
+    s0, s1 = X.stride()
+    if s0 == 1 and s1 >= m and m > 1 and n > 1:
+        return X.data_ptr(), s1
+    return X.data_ptr(), ld_or_raise(X, name)
+
+
+def _item_records(As, outs):
+    """The work list as the 64-bit words of its ``mak_batch_item`` records
+    (the element type and the reserved word share the first, little-endian)."""
+    rows = []
+    for A, (Q, R) in zip(As, outs):
         m, n = A.shape
-        arr[i] = _lib.mak_batch_item(DTYPE_CODE[A.dtype], 0, m, n, A.data_ptr(),
-                                     ld_or_raise(A, "A"), Q.data_ptr(), ld_or_raise(Q, "Q"),
-                                     R.data_ptr() if R is not None and R.numel() else None,
-                                     ld_or_raise(R, "R") if R is not None and R.numel() else 1)
-    return arr
+        a, lda = _ptr_ld(A, "A")
+        q, ldq = _ptr_ld(Q, "Q")
+        r, ldr = _ptr_ld(R, "R") if R is not None and R.numel() else (0, 1)
+        rows.append((DTYPE_CODE[A.dtype], m, n, a, lda, q, ldq, r, ldr))
+    return np.array(rows, dtype="<i8").reshape(len(rows), 9)
+
+
+def _items(As, outs):
+    rec = _item_records(As, outs)
+    return (_lib.mak_batch_item * len(As)).from_buffer_copy(rec.tobytes())
+
+
+_ITEM_BYTES = np.array([8, 16, 4, 8])  # by element type code (F64, C64, F32, C32)
+
+
+def _overlaps(rec, with_r_cols):
+    """Whether some input block shares memory with some output block."""
+    es = _ITEM_BYTES[rec[:, 0]]
+    m, n = rec[:, 1], rec[:, 2]
+    k = np.minimum(m, n)
+
+    def spans(col, ld, rows, cols):
+        keep = (rec[:, col] != 0) & (rows > 0) & (cols > 0)
+        lo = rec[keep, col]
+        return lo, lo + (((cols - 1) * rec[:, ld] + rows) * es)[keep]
+
+    ilo, ihi = spans(3, 4, m, n)
+    qlo, qhi = spans(5, 6, m, k)
+    rlo, rhi = spans(7, 8, k, n if with_r_cols else k)
+    olo, ohi = np.concatenate([qlo, rlo]), np.concatenate([qhi, rhi])
+    order = np.argsort(olo)
+    olo, ohi = olo[order], np.maximum.accumulate(ohi[order])
+    at = np.searchsorted(olo, ihi) - 1  # the last output that starts before the input's end
+    return bool(np.any((at >= 0) & (ohi[np.maximum(at, 0)] > ilo)))
+
+
+def _read_in_place(As, outs, fresh_outs, with_r_cols):
+    """The inputs of a device work list whose kernels read each block once and
+    write only the outputs: blocks already in the kernels' layout are read
+    where they are; a block in another layout (or lazily conjugated or
+    negated), or any sharing of memory with the outputs, takes copies."""
+    work = [A if A.stride()[0] == 1 and A.stride()[1] >= A.shape[0] and not A.is_conj()
+            and not A.is_neg() else to_cm(A) for A in As]
+    rec = _item_records(work, outs)
+    if not fresh_outs and _overlaps(rec, with_r_cols):
+        work = [to_cm(A) for A in As]
+        rec = _item_records(work, outs)
+    return work, rec
+
+
+def _check_blocks(As):
+    dev = As[0].device if isinstance(As[0], torch.Tensor) else None
+    for A in As:
+        if not (isinstance(A, torch.Tensor) and A.is_cuda and A.dtype in DTYPE_CODE
+                and A.dim() == 2):
+            check_cuda_tensor(A, "A")
+        if A.device != dev:
+            raise ArgumentError("all blocks must live on one device")
+    return dev
+
+
+def _records_to_device(rec, dev):
+    return torch.from_numpy(rec.view(np.uint8).reshape(-1)).to(dev)
+
+
+def _info_words(infos, n):
+    """The outcome records as 32-bit words, one row per block."""
+    return infos.cpu().numpy().view("<i4").reshape(n, INFO_BYTES // 4)
 
 
 def _read_infos(infos, n):
@@ -94,9 +168,7 @@ def batch_items_device(As, outs):
     """The work list of ``As`` / ``outs`` as a DEVICE array of
     ``mak_batch_item`` records (a uint8 tensor), the layout a caller's own
     kernel may also write."""
-    items = _items(As, outs)
-    raw = torch.frombuffer(bytearray(bytes(items)), dtype=torch.uint8)
-    return raw.to(As[0].device)
+    return _records_to_device(_item_records(As, outs), As[0].device)
 
 
 def batched_qr_compact_device(As, alg=None, copy_inputs=True, outs=None, items=None,
@@ -109,20 +181,20 @@ def batched_qr_compact_device(As, alg=None, copy_inputs=True, outs=None, items=N
     alg = select_algorithm("qr_compact_", None, alg, **kwargs)
     if not As:
         return []
-    dev = As[0].device
-    for A in As:
-        check_cuda_tensor(A, "A")
-        if A.device != dev:
-            raise ArgumentError("all blocks must live on one device")
-    if outs is None:
+    dev = _check_blocks(As)
+    fresh = outs is None
+    if fresh:
         outs = []
         for A in As:
             m, n = A.shape
             k = min(m, n)
             outs.append((empty_cm(m, k, A.dtype, A.device), empty_cm(k, n, A.dtype, A.device)))
-    work_As = [to_cm(A) for A in As] if copy_inputs else list(As)
     if items is None:
-        items = batch_items_device(work_As, outs)
+        if copy_inputs:
+            work_As, rec = _read_in_place(As, outs, fresh, True)
+        else:
+            rec = _item_records(As, outs)
+        items = _records_to_device(rec, dev)
     opts = _lib.mak_qr_opts(int(alg.positive), int(alg.blocksize), PRECISION_CODE[alg.precision], 0)
     L = lib()
     with torch.cuda.device(dev):
@@ -132,11 +204,10 @@ def batched_qr_compact_device(As, alg=None, copy_inputs=True, outs=None, items=N
         check_rc(rc, "mak_batched_qr_compact_device")
         if _capturing:
             return outs
-        res = _read_infos(infos, len(As))
-    for i, inf in enumerate(res):
-        if inf.status != 0:
-            raise RuntimeError(f"mak_batched_qr_compact_device: block {i}: device status "
-                               f"{inf.status}")
+        res = _info_words(infos, len(As))
+    for i in np.flatnonzero(res[:, 0]):
+        raise RuntimeError(f"mak_batched_qr_compact_device: block {i}: device status "
+                           f"{res[i, 0]}")
     return outs
 
 
@@ -156,19 +227,20 @@ def batched_left_polar_device(As, alg=None, copy_inputs=True, outs=None, items=N
     alg = select_algorithm("left_polar_", None, alg, **kwargs)
     if not As:
         return []
-    dev = As[0].device
+    dev = _check_blocks(As)
     for A in As:
-        check_cuda_tensor(A, "A")
-        if A.device != dev:
-            raise ArgumentError("all blocks must live on one device")
         if A.shape[0] < A.shape[1]:
             raise ArgumentError("every block needs at least as many rows as columns")
-    if outs is None:
+    fresh = outs is None
+    if fresh:
         outs = [(empty_cm(A.shape[0], A.shape[1], A.dtype, A.device),
                  empty_cm(A.shape[1], A.shape[1], A.dtype, A.device)) for A in As]
-    work_As = [to_cm(A) for A in As] if copy_inputs else list(As)
     if items is None:
-        items = batch_items_device(work_As, outs)
+        if copy_inputs:
+            work_As, rec = _read_in_place(As, outs, fresh, False)
+        else:
+            rec = _item_records(As, outs)
+        items = _records_to_device(rec, dev)
     opts = _lib.mak_polar_opts(int(alg.maxiter), PRECISION_CODE[alg.precision],
                                float(alg.tol) if alg.tol is not None else 0.0)
     L = lib()
