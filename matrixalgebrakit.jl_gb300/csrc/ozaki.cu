@@ -326,7 +326,7 @@ __device__ __forceinline__ double* oz_out_ptr(double* C, int64_t ldc, int cpx, i
 
 // CHUNK = K-steps per exact accumulator chunk: 32 (512 of K, group sums up
 // to 2^24, converted from their bits) or 8 (128 of K, group sums up to 2^22,
-// converted with one FFMA; products with K <= 128 use this variant).
+// converted with one FFMA; the 32-wide tiles and products with K <= 128).
 // BN = output tile width: 64, or 32 with two accumulator buffers in TMEM
 // (S x 32 columns each) so that the MMAs of the next tile run while the
 // epilogue reads the previous one.
@@ -987,14 +987,8 @@ int oz_gemm(cudaStream_t st, int64_t M, int64_t N, int64_t K, T alpha, Operand<T
   const int64_t Mpad = ceil_div(M > 0 ? M : 1, OZ_BM) * OZ_BM;
   const int64_t Kpad = ceil_div(Kl > 0 ? Kl : 1, OZ_BK) * OZ_BK;
   const int64_t nkt_total = Kpad / OZ_BK;
-  // products with K <= 128 (one short chunk per tile) take 32-wide tiles with
-  // two accumulator sets, so that a tile's MMAs overlap the previous tile's
-  // epilogue; longer products the 64-wide tile (MAK_OZ_NARROW = 0: always 64)
-  const bool small = nkt_total * OZ_BK <= 128;
-  const int BN = (small && tuning(TUNE_OZ_NARROW) != 0) ? 32 : 64;
-  const int64_t Npad = ceil_div(Nl > 0 ? Nl : 1, (int64_t)BN) * BN;
+  const int64_t nchunk = ceil_div(nkt_total, (int64_t)OZ_KSTEPS_PER_CHUNK);
   const int64_t Npad64 = ceil_div(Nl > 0 ? Nl : 1, (int64_t)64) * 64;  // workspace bound
-  const int64_t tiles = (Mpad / OZ_BM) * (Npad / BN);
   // persistent grid cap: the caller's limit, else the thread's budget, else every SM
   if (max_ctas <= 0) max_ctas = split_gemm_cta_budget();
   const int cap = (max_ctas > 0 && max_ctas < num_sms()) ? max_ctas : num_sms();
@@ -1004,9 +998,8 @@ int oz_gemm(cudaStream_t st, int64_t M, int64_t N, int64_t K, T alpha, Operand<T
   // partials stay within the measured bound.  A ragged last wave idles the
   // grid (64 tiles x 3 splits on 152 CTAs: 2 waves at 63 %), so the count is
   // chosen by the waves it takes, not by the CTAs it would fill.
-  int splits = 1;
-  {
-    const int64_t nchunk = ceil_div(nkt_total, OZ_KSTEPS_PER_CHUNK);
+  auto pick = [&](int64_t tiles) -> int {
+    int splits = 1;
     if (tiles < cap && nchunk > 1) {
       double best = 0.0;
       for (int s = 1; s <= 32 && s <= nchunk; s++) {
@@ -1021,10 +1014,26 @@ int oz_gemm(cudaStream_t st, int64_t M, int64_t N, int64_t K, T alpha, Operand<T
         }
       }
     }
-  }
-  const int64_t chunks_per_split =
-      ceil_div(ceil_div(nkt_total, OZ_KSTEPS_PER_CHUNK), splits);
-  splits = (int)ceil_div(ceil_div(nkt_total, OZ_KSTEPS_PER_CHUNK), chunks_per_split);
+    return splits;
+  };
+  // 64-wide tiles have the better rate in a long K (128 x 8192 x 16384: 1065
+  // us against 1435 with 32), but one accumulator set, so that a chunk's MMAs
+  // wait for the epilogue of the chunk before it; 32-wide tiles have two, in
+  // chunks of 128.  The 32-wide tile is taken where an item is one chunk of
+  // 512 or less, so that the wide tile would overlap nothing (16384 x 8192 x
+  // 256: 5.2 -> 2.6 ms, x 512: 9.5 -> 4.9 ms, 128 x 1000 x 2049: 63 -> 62
+  // us), and where the wide tiles would fill less than half the grid
+  // (128 x 128 x 16384: 89 -> 44 us).  MAK_OZ_NARROW = 0: always 64.
+  const bool small = nkt_total * OZ_BK <= 128;
+  const int64_t tiles64 = (Mpad / OZ_BM) * (Npad64 / 64);
+  const int splits64 = pick(tiles64);
+  const bool narrow = tuning(TUNE_OZ_NARROW) != 0 &&
+                      (ceil_div(nchunk, (int64_t)splits64) == 1 || 2 * tiles64 * splits64 < cap);
+  const int BN = narrow ? 32 : 64;
+  const int64_t Npad = ceil_div(Nl > 0 ? Nl : 1, (int64_t)BN) * BN;
+  int splits = narrow ? pick((Mpad / OZ_BM) * (Npad / BN)) : splits64;
+  const int64_t chunks_per_split = ceil_div(nchunk, (int64_t)splits);
+  splits = (int)ceil_div(nchunk, chunks_per_split);
 
   unsigned long long* bitsA = ar.take<unsigned long long>(Mpad + Npad64);
   unsigned long long* bitsB = bitsA + Mpad;
@@ -1079,7 +1088,7 @@ int oz_gemm(cudaStream_t st, int64_t M, int64_t N, int64_t K, T alpha, Operand<T
     const int64_t nwork = (int64_t)tm * tn * splits;
     const int grid = (int)(nwork < cap ? nwork : cap);
     note_launch();
-    if (small && BN == 32)  // one short chunk: the FFMA conversion
+    if (narrow)  // chunks of 128 of K: the FFMA conversion
       oz_gemm_kernel<S, OZ_SMALL_CHUNK, 32>
           <<<grid, OZ_THREADS, oz_smem_bytes<S, 32>(), st>>>(mapA, mapB, args);
     else if (small)
