@@ -37,6 +37,7 @@
 #include "gemm.cuh"
 #include "householder.cuh"
 #include "internal.h"
+#include "util.cuh"
 
 #include <cstdlib>
 #include <mutex>
@@ -1145,7 +1146,8 @@ __global__ void __launch_bounds__(256) reduce_trmm_kernel(int jb, int nt, int sp
   W2[i + (int64_t)c * jb] = (s[0] + s[1]) + (s[2] + s[3]);
 }
 
-constexpr int QR_OUTER_NB = 128;  // outer block of the mixed-precision path
+constexpr int QR_OUTER_NB = 128;  // block of the mixed-precision path
+constexpr double QR_WIDE_MIN_MN = 4.0e6;  // m n from which its block reflectors are merged
 // SMs given to the look-ahead side stream (panels and the block Gram) while
 // the main stream's persistent tensor-core grid takes the rest; 48 by
 // default, MAK_LOOKAHEAD_CTAS overrides it (read once, clamped to 8..120).
@@ -1487,7 +1489,18 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
   // outer block of the mixed path: 128 columns, or 64 for blocks whose
   // columns number at most MAK_QR_OUTER64_MAX_N (default 0: never), where
   // fewer 32-wide panels per block leave fewer within-block native updates
-  const int NBO = mixed ? ((double)n <= tuning(TUNE_QR_OUTER64_MAX_N) ? 64 : QR_OUTER_NB) : nb;
+  const int NBM = mixed ? ((double)n <= tuning(TUNE_QR_OUTER64_MAX_N) ? 64 : QR_OUTER_NB) : nb;
+  // Large problems apply wider block reflectors: two 128-wide blocks merged
+  // for the trailing updates (the second is updated with the first on its
+  // own), four for Q, whose T factors all exist by then.  A product with K =
+  // 256 or 512 reads and writes C, cuts C's digit planes and finds C's maxima
+  // half or a quarter as often, and amortises its epilogue over more of K
+  // (16384 x 8192: K = 128 643, 256 955, 512 1005 bf16 TFLOP/s).  From the
+  // size that takes the look-ahead: below it a block's panels are longer than
+  // the update they would merge.
+  const bool wide = mixed && NBM == QR_OUTER_NB && (double)m * n >= QR_WIDE_MIN_MN;
+  const int NBO = wide ? 2 * NBM : NBM;
+  const int NBQ = wide ? 4 * NBM : NBM;
   const int64_t nblk_o = ceil_div(k, NBO);
 
   T* tau = ar.take<T>(k > 0 ? k : 1);
@@ -1505,44 +1518,49 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
   T* gram_buf = ar.take<T>((size_t)NBMAX * NBMAX);
   unsigned* bar = ar.take<unsigned>(2);
   int* cflag = ar.take<int>(gmax);
-  T *To = nullptr, *Gm = nullptr, *Wm = nullptr, *W2m = nullptr;
+  T *To = nullptr, *Gm = nullptr, *Xm = nullptr, *Tq = nullptr, *Wm = nullptr, *W2m = nullptr;
   char* ozs = nullptr;
   size_t oz_bytes = 0;
+  auto scratch_for = [&](const int64_t (*shapes)[3], int count) -> size_t {
+    size_t bytes = 0;
+    for (int q = 0; q < count; q++) {
+      Arena meas(nullptr, 0);
+      gemm_prec<T>(st, precision, shapes[q][0], shapes[q][1], shapes[q][2], one_<T>(),
+                   opnd<T>(nullptr, 1), opnd<T>(nullptr, 1), zero_<T>(), nullptr, 1, meas,
+                   nullptr);
+      if (meas.off + 1024 > bytes) bytes = meas.off + 1024;
+    }
+    return bytes;
+  };
   if (mixed) {
     To = ar.take<T>((size_t)(nblk_o > 0 ? nblk_o : 1) * NBO * NBO);
     Gm = ar.take<T>((size_t)NBO * NBO);
-    Wm = ar.take<T>((size_t)NBO * (wmax > 0 ? wmax : 1));
-    W2m = ar.take<T>((size_t)NBO * (wmax > 0 ? wmax : 1));
-    // the tensor-core GEMMs run one after another and share one scratch region
-    const int64_t shapes[4][3] = {{NBO, wmax, m}, {m, wmax, NBO}, {NBO, wmax, NBO}, {NBO, NBO, m}};
-    for (auto& sh : shapes) {
-      Arena meas(nullptr, 0);
-      gemm_prec<T>(st, precision, sh[0], sh[1], sh[2], one_<T>(), opnd<T>(nullptr, 1),
-                   opnd<T>(nullptr, 1), zero_<T>(), nullptr, 1, meas, nullptr);
-      if (meas.off + 1024 > oz_bytes) oz_bytes = meas.off + 1024;
+    Wm = ar.take<T>((size_t)NBQ * (wmax > 0 ? wmax : 1));
+    W2m = ar.take<T>((size_t)NBQ * (wmax > 0 ? wmax : 1));
+    if (wide) {
+      Xm = ar.take<T>((size_t)NBO * NBO);
+      Tq = ar.take<T>((size_t)NBQ * NBQ);
     }
+    // the tensor-core GEMMs run one after another and share one scratch region
+    const int64_t shapes[4][3] = {{NBQ, wmax, m}, {m, wmax, NBQ}, {NBQ, wmax, NBQ}, {NBO, NBO, m}};
+    oz_bytes = scratch_for(shapes, 4);
     ozs = ar.take<char>(oz_bytes);
   }
   // the block Gram matrix and the within-block updates of the panels run on
   // the look-ahead stream: their own scratch, and (mixed) W / T^H W of a
-  // panel's update
+  // panel's update or of a 128-wide block's update inside its pair
   size_t gram_bytes = 0;
   char* grams = nullptr;
   T *Wp = nullptr, *W2p = nullptr;
   const bool panel_split = mixed && tuning(TUNE_QR_PANEL_SPLIT) != 0;
   if (mixed) {
-    const int64_t shapes[3][3] = {{NBO, NBO, m}, {NBMAX, NBO, m}, {m, NBO, NBMAX}};
-    for (int q = 0; q < (panel_split ? 3 : 1); q++) {
-      Arena meas(nullptr, 0);
-      gemm_prec<T>(st, precision, shapes[q][0], shapes[q][1], shapes[q][2], one_<T>(),
-                   opnd<T>(nullptr, 1), opnd<T>(nullptr, 1), zero_<T>(), nullptr, 1, meas,
-                   nullptr);
-      if (meas.off + 1024 > gram_bytes) gram_bytes = meas.off + 1024;
-    }
+    const int64_t shapes[5][3] = {{NBM, NBM, m}, {NBMAX, NBM, m}, {m, NBM, NBMAX},
+                                  {m, NBM, NBM}, {NBM, NBM, NBM}};
+    gram_bytes = scratch_for(shapes, wide ? 5 : (panel_split ? 3 : 1));
     grams = ar.take<char>(gram_bytes);
-    if (panel_split) {
-      Wp = ar.take<T>((size_t)NBMAX * NBO);
-      W2p = ar.take<T>((size_t)NBMAX * NBO);
+    if (panel_split || wide) {
+      Wp = ar.take<T>((size_t)NBM * NBM);
+      W2p = ar.take<T>((size_t)NBM * NBM);
     }
   }
   if (ar.base == nullptr) return 0;
@@ -1552,27 +1570,52 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
   MAK_CUDA_TRY(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), st));
 
   // C <- (I - V op(T) V^H) C with the tensor-core GEMMs; op(T) = T^H for the
-  // factorization, T for Q formation (T is JB x JB upper, ld NBO)
+  // factorization, T for Q formation (T is JB x JB upper, leading dimension
+  // ldt), on the scratch W / W2 / sb[0, sbytes) of the stream it runs on
   // max_ctas > 0 leaves the other SMs to the look-ahead side stream
-  auto larfb_mixed = [&](const T* V, int64_t mp, int JB, const T* Tm, int conjtrans, T* Cm,
-                         int64_t ldc, int64_t nc, cudaStream_t s, int max_ctas) -> int {
+  auto larfb_on = [&](const T* V, int64_t mp, int JB, const T* Tm, int ldt, int conjtrans, T* Cm,
+                      int64_t ldc, int64_t nc, cudaStream_t s, int max_ctas, T* W, T* W2,
+                      char* sb, size_t sbytes) -> int {
     if (nc <= 0) return 0;
     {
-      Arena oz(ozs, oz_bytes);
+      Arena oz(sb, sbytes);
       MAK_TRY(gemm_prec<T>(s, precision, JB, nc, mp, one_<T>(),
                            opnd<T>(V, lda, OP_C, MASK_UNIT_LOWER), opnd<T>(Cm, ldc), zero_<T>(),
-                           Wm, JB, oz, status, max_ctas));
+                           W, JB, oz, status, max_ctas));
     }
     {
-      Arena oz(ozs, oz_bytes);
+      Arena oz(sb, sbytes);
       MAK_TRY(gemm_prec<T>(s, precision, JB, nc, JB, one_<T>(),
-                           opnd<T>(Tm, NBO, conjtrans ? OP_C : OP_N, MASK_UPPER),
-                           opnd<T>(Wm, JB), zero_<T>(), W2m, JB, oz, status, max_ctas));
+                           opnd<T>(Tm, ldt, conjtrans ? OP_C : OP_N, MASK_UPPER), opnd<T>(W, JB),
+                           zero_<T>(), W2, JB, oz, status, max_ctas));
     }
-    Arena oz(ozs, oz_bytes);
+    Arena oz(sb, sbytes);
     return gemm_prec<T>(s, precision, mp, nc, JB, -one_<T>(),
-                        opnd<T>(V, lda, OP_N, MASK_UNIT_LOWER), opnd<T>(W2m, JB), one_<T>(), Cm,
+                        opnd<T>(V, lda, OP_N, MASK_UNIT_LOWER), opnd<T>(W2, JB), one_<T>(), Cm,
                         ldc, oz, status, max_ctas);
+  };
+  auto larfb_mixed = [&](const T* V, int64_t mp, int JB, const T* Tm, int ldt, int conjtrans,
+                         T* Cm, int64_t ldc, int64_t nc, cudaStream_t s, int max_ctas) -> int {
+    return larfb_on(V, mp, JB, Tm, ldt, conjtrans, Cm, ldc, nc, s, max_ctas, Wm, W2m, ozs,
+                    oz_bytes);
+  };
+  // T of two block reflectors side by side (ja columns from j0, then jb): its
+  // diagonal blocks Ta, Tb are in place in Tm, its corner is -Ta (Va^H Vb) Tb
+  // (V = [Va Vb], Vb zero above row j0 + ja).  G and X: scratch of ja x jb.
+  auto merge_t = [&](int64_t j0, int ja, int jb, T* Tm, int ldt, T* G, T* X, cudaStream_t s,
+                     char* sb, size_t sbytes, int max_ctas) -> int {
+    const int64_t j1 = j0 + ja;
+    {
+      Arena oz(sb, sbytes);
+      MAK_TRY(gemm_prec<T>(s, precision, ja, jb, m - j1, one_<T>(),
+                           opnd<T>(A + j1 + j0 * lda, lda, OP_C),
+                           opnd<T>(A + j1 + j1 * lda, lda, OP_N, MASK_UNIT_LOWER), zero_<T>(), G,
+                           ja, oz, status, max_ctas));
+    }
+    MAK_TRY(gemm<T>(s, ja, jb, jb, one_<T>(), opnd<T>(G, ja),
+                    opnd<T>(Tm + ja + (int64_t)ja * ldt, ldt, OP_N, MASK_UPPER), zero_<T>(), X, ja));
+    return gemm<T>(s, ja, jb, ja, -one_<T>(), opnd<T>(Tm, ldt, OP_N, MASK_UPPER), opnd<T>(X, ja),
+                   zero_<T>(), Tm + (int64_t)ja * ldt, ldt);
   };
   // C = A[j0:, c0:c1] <- (I - V T^H V^H)... with the native SIMT kernels
   auto larfb_native = [&](int64_t j0, int jb, const T* Tb, int64_t c0, int64_t c1,
@@ -1660,35 +1703,48 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
                                              dim3(PANEL_THREADS), args, ps.smem, s));
     return 0;
   };
-  // factor outer block b: its panels with updates confined to the block,
-  // and (mixed) the 128-wide T factor from the block's Gram matrix
+  // factor outer block b: its panels with updates confined to their 128-wide
+  // block, (mixed) the block's T factor from its Gram matrix, and (wide) the
+  // first block's reflector applied to the second, then their T merged
   auto factor_block = [&](int64_t b, cudaStream_t s) -> int {
     const int64_t J0 = b * NBO;
     const int JB = (int)((k - J0) < NBO ? (k - J0) : NBO);
-    for (int64_t j0 = J0; j0 < J0 + JB; j0 += nb) {
-      const int jb = (int)((J0 + JB - j0) < nb ? (J0 + JB - j0) : nb);
-      MAK_TRY(panel(j0, jb, s));
-      if (panel_split)
-        MAK_TRY(larfb_panel_split(j0, jb, Ts + (j0 / nb) * NBMAX * NBMAX, j0 + jb, J0 + JB, s));
-      else
-        MAK_TRY(larfb_native(j0, jb, Ts + (j0 / nb) * NBMAX * NBMAX, j0 + jb, J0 + JB, s));
+    const int mc = s == st ? 0 : tl_side_ctas;
+    T* const Tb = mixed ? To + b * NBO * NBO : nullptr;
+    for (int64_t M0 = J0; M0 < J0 + JB; M0 += NBM) {
+      const int MB = (int)((J0 + JB - M0) < NBM ? (J0 + JB - M0) : NBM);
+      for (int64_t j0 = M0; j0 < M0 + MB; j0 += nb) {
+        const int jb = (int)((M0 + MB - j0) < nb ? (M0 + MB - j0) : nb);
+        MAK_TRY(panel(j0, jb, s));
+        if (panel_split)
+          MAK_TRY(larfb_panel_split(j0, jb, Ts + (j0 / nb) * NBMAX * NBMAX, j0 + jb, M0 + MB, s));
+        else
+          MAK_TRY(larfb_native(j0, jb, Ts + (j0 / nb) * NBMAX * NBMAX, j0 + jb, M0 + MB, s));
+      }
+      if (!mixed) return 0;
+      const T* V = A + M0 + M0 * lda;
+      {
+        // the Gram matrix fixes the orthogonality of the block reflector; the
+        // split-precision product is FP64-accurate, and 2 m 128^2 flops per
+        // block on the FP64 pipe would sit on the look-ahead's critical path
+        Arena ga(grams, gram_bytes);
+        MAK_TRY(gemm_prec<T>(s, precision, MB, MB, m - M0, one_<T>(),
+                             opnd<T>(V, lda, OP_C, MASK_UNIT_LOWER),
+                             opnd<T>(V, lda, OP_N, MASK_UNIT_LOWER), zero_<T>(), Gm, MB, ga,
+                             status, mc));
+      }
+      T* const Tmid = Tb + (M0 - J0) * (NBO + 1);
+      note_launch();
+      larft_cols_kernel<T><<<(unsigned)ceil_div(MB, 8), 256, 0, s>>>(MB, Gm, MB, tau + M0, Tmid,
+                                                                    NBO);
+      MAK_CUDA_TRY(cudaGetLastError());
+      const int rest = (int)(J0 + JB - M0 - MB);
+      if (rest > 0)
+        MAK_TRY(larfb_on(V, m - M0, MB, Tmid, NBO, 1, A + M0 + (M0 + MB) * lda, lda, rest, s, mc,
+                         Wp, W2p, grams, gram_bytes));
     }
-    if (!mixed) return 0;
-    const T* V = A + J0 + J0 * lda;
-    {
-      // the Gram matrix fixes the orthogonality of the block reflector; the
-      // split-precision product is FP64-accurate, and 2 m 128^2 flops per
-      // block on the FP64 pipe would sit on the look-ahead's critical path
-      Arena ga(grams, gram_bytes);
-      MAK_TRY(gemm_prec<T>(s, precision, JB, JB, m - J0, one_<T>(),
-                           opnd<T>(V, lda, OP_C, MASK_UNIT_LOWER),
-                           opnd<T>(V, lda, OP_N, MASK_UNIT_LOWER), zero_<T>(), Gm, NBO, ga,
-                           status, s == st ? 0 : tl_side_ctas));
-    }
-    note_launch();
-    larft_cols_kernel<T><<<(unsigned)ceil_div(JB, 8), 256, 0, s>>>(JB, Gm, NBO, tau + J0,
-                                                                  To + b * NBO * NBO, NBO);
-    MAK_CUDA_TRY(cudaGetLastError());
+    if (JB > NBM)
+      MAK_TRY(merge_t(J0, NBM, JB - NBM, Tb, NBO, Gm, Xm, s, grams, gram_bytes, mc));
     return 0;
   };
   // block b's reflector applied to the columns [c0, c1)
@@ -1697,7 +1753,7 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
     const int64_t J0 = b * NBO;
     const int JB = (int)((k - J0) < NBO ? (k - J0) : NBO);
     if (mixed)
-      return larfb_mixed(A + J0 + J0 * lda, m - J0, JB, To + b * NBO * NBO, 1,
+      return larfb_mixed(A + J0 + J0 * lda, m - J0, JB, To + b * NBO * NBO, NBO, 1,
                          A + J0 + c0 * lda, lda, c1 - c0, s, max_ctas);
     return larfb_native(J0, JB, Ts + (J0 / nb) * NBMAX * NBMAX, c0, c1, s);
   };
@@ -1753,13 +1809,23 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
 
   // ------------------------------------------- Q = H_1 ... H_k [diag(s); 0]
   if (mixed) {
-    for (int64_t bo = nblk_o - 1; bo >= 0; bo--) {
-      const int64_t J0 = bo * NBO;
-      const int JB = (int)((k - J0) < NBO ? (k - J0) : NBO);
+    for (int64_t bq = ceil_div(k, NBQ) - 1; bq >= 0; bq--) {
+      const int64_t J0 = bq * NBQ;
+      const int JB = (int)((k - J0) < NBQ ? (k - J0) : NBQ);
       const int64_t qt = qcols - J0;
       if (qt <= 0) continue;
-      MAK_TRY(larfb_mixed(A + J0 + J0 * lda, m - J0, JB, To + bo * NBO * NBO, 0,
-                          Q + J0 + J0 * ldq, ldq, qt, st, 0));
+      const T* Tm = To + (J0 / NBO) * NBO * NBO;
+      int ldt = NBO;
+      if (JB > NBO) {  // two outer blocks' T factors merged
+        const int jb = JB - NBO;
+        MAK_TRY(copy_mat<T>(st, NBO, NBO, Tm, NBO, Tq, NBQ));
+        MAK_TRY(copy_mat<T>(st, jb, jb, Tm + NBO * NBO, NBO, Tq + NBO * (NBQ + 1), NBQ));
+        MAK_TRY(merge_t(J0, NBO, jb, Tq, NBQ, Gm, Xm, st, ozs, oz_bytes, 0));
+        Tm = Tq;
+        ldt = NBQ;
+      }
+      MAK_TRY(larfb_mixed(A + J0 + J0 * lda, m - J0, JB, Tm, ldt, 0, Q + J0 + J0 * ldq, ldq, qt,
+                          st, 0));
     }
     return 0;
   }
