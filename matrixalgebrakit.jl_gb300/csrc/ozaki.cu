@@ -800,6 +800,48 @@ struct OzPlaneOut {
   const unsigned long long* bits;  // largest magnitude of each row, IEEE bits
   __nv_bfloat16* planes;
 };
+// The plane values of x, each in the upper half of a word: the fixed-point value f = |x| 2^(FB - Fr) rounded to
+// nearest (f <= 2^(FB - 1)), with x's sign, plus the constant BIAS (64 at every
+// digit position), whose plain base-128 digits t_p are the balanced digits
+// d_p = t_p - 64 in [-64, 63] (the leading one in [-64, 64]): each is one shift
+// and one mask, with no carries.  d_p 2^(-7p) is built in fp32 without a
+// conversion: the float 2^23 + t has t in its low bits, and one FMA with the
+// plane's scale removes 2^23 + 64; the result has at most 7 significant bits,
+// so its upper half is its bf16 form.
+template <int S>
+__device__ __forceinline__ void oz_digits(double x, int Fr, unsigned (&v)[S]) {
+  constexpr int FB = OZ_BITS * S;  // fractional bits of the fixed-point value
+  static_assert(FB <= 56, "the fixed-point value fits 28 + 29 bits");
+  const unsigned long long bts = (unsigned long long)__double_as_longlong(x);
+  int ex = (int)((bts >> 52) & 0x7FF);
+  unsigned long long m = bts & 0x000FFFFFFFFFFFFFull;
+  if (ex == 0) ex = 1; else m |= 0x0010000000000000ull;
+  const int sh = ex - 1075 + FB - Fr;
+  unsigned long long f;
+  // a magnitude beyond the frame (an operand that changed between the two
+  // passes, an infinity) gives 0 rather than digits out of range
+  if (sh >= 0) f = sh >= 11 ? 0 : (m << sh);
+  else if (-sh >= 55) f = 0;
+  else f = (m >> (-sh)) + ((m >> (-sh - 1)) & 1ull);
+  if ((bts & 0x7FFFFFFFFFFFFFFFull) == 0 || f > (1ull << (FB - 1))) f = 0;
+  constexpr unsigned long long BIAS = [] {
+    unsigned long long b = 0;
+    for (int i = 0; i < S; i++) b |= 64ull << (OZ_BITS * i);
+    return b;
+  }();
+  const unsigned long long u = (bts >> 63) ? BIAS - f : BIAS + f;
+  constexpr int H = S / 2 * OZ_BITS;  // bits of the low half
+  const unsigned hi = (unsigned)(u >> H), lo = (unsigned)u & ((1u << H) - 1u);
+#pragma unroll
+  for (int p = 0; p < S; p++) {
+    const int q = S - 1 - p;  // digit position from the bottom
+    const unsigned w = q >= S / 2 ? hi >> (OZ_BITS * (q - S / 2)) : lo >> (OZ_BITS * q);
+    const unsigned t = p == 0 ? w : (w & 127u);
+    const float scale = __uint_as_float((unsigned)(127 - OZ_BITS * p) << 23);
+    v[p] = __float_as_uint(fmaf(__uint_as_float(0x4B000000u | t), scale, -8388672.0f * scale));
+  }
+}
+
 template <class T, int S>
 __global__ void __launch_bounds__(256) oz_split_kernel(OzSrc<T> sa, OzPlaneOut oa, OzSrc<T> sb,
                                                        OzPlaneOut ob, int K, int Kpad,
@@ -808,109 +850,90 @@ __global__ void __launch_bounds__(256) oz_split_kernel(OzSrc<T> sa, OzPlaneOut o
   const OzSrc<T>& s = blockIdx.z == 0 ? sa : sb;
   const OzPlaneOut& o = blockIdx.z == 0 ? oa : ob;
   const int R = o.R, Rpad = o.Rpad;
-  __nv_bfloat16* planes = o.planes;
   const int r0 = blockIdx.y * 64, k0 = blockIdx.x * 64;
   if (r0 >= Rpad) return;  // the shorter side's grid rows (uniform per CTA)
   // row stride 68 doubles: the digit phase's reads (eight rows of eight
   // threads, eight apart in k) fall on distinct banks pairwise
   __shared__ double tile[64][68];
-  // bf16 bits of +-(t - 64) 2^(-7p) for the biased digits t = 0 .. 128 of
-  // plane p ([0]: positive values, [1]: negated)
-  __shared__ unsigned short lut[2][S][130];
   const int tid = threadIdx.x;
   const bool cr = oz_contig_r(s);
-  for (int e = tid; e < 2 * S * 129; e += 256) {
-    const int sg = e / (S * 129), p = (e / 129) % S, t = e % 129;
-    const float v = ldexpf((float)(t - 64), -OZ_BITS * p);
-    lut[sg][p][t] = __bfloat16_as_ushort(__float2bfloat16_rn(sg && t != 64 ? -v : v));
-  }
-  if (oz_plain(s)) {
-    // sixteen independent loads per thread, then the stores to the tile
+  // Each thread cuts two units: one row, eight adjacent k (one 16-byte store
+  // per plane).  A plain operand contiguous along k is read straight into
+  // them; the others go through the tile.
+  double x[2][8];
+  const bool direct = oz_plain(s) && !cr;
+  if (direct) {
     const double* src = reinterpret_cast<const double*>(s.op.p);
     const int64_t ld = s.op.ld;
-    double v[16];
+    const bool wide = ((uintptr_t)src & 15) == 0 && (ld & 1) == 0;  // 16-byte loads
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
-      const int e = tid + 256 * i;
-      int rr, kk;
-      if (cr) { rr = e % 64; kk = e / 64; } else { kk = e % 64; rr = e / 64; }
-      const int r = r0 + rr, k = k0 + kk;
-      v[i] = (r < R && k < K) ? src[cr ? (int64_t)r + (int64_t)k * ld : (int64_t)k + (int64_t)r * ld]
-                              : 0.0;
-    }
+    for (int u = 0; u < 2; u++) {
+      const int e = tid + 256 * u, r = r0 + e / 8, k = k0 + (e % 8) * 8;
+      const double* q = src + (int64_t)r * ld + k;
+      if (wide && r < R && k + 8 <= K) {
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
-      const int e = tid + 256 * i;
-      int rr, kk;
-      if (cr) { rr = e % 64; kk = e / 64; } else { kk = e % 64; rr = e / 64; }
-      tile[rr][kk] = v[i];
+        for (int h = 0; h < 4; h++) {
+          const double2 v = __ldg(reinterpret_cast<const double2*>(q) + h);
+          x[u][2 * h] = v.x;
+          x[u][2 * h + 1] = v.y;
+        }
+      } else {
+#pragma unroll
+        for (int h = 0; h < 8; h++) x[u][h] = (r < R && k + h < K) ? q[h] : 0.0;
+      }
     }
   } else {
-    for (int e = tid; e < 64 * 64; e += 256) {
-      int rr, kk;
-      if (cr) { rr = e % 64; kk = e / 64; } else { kk = e % 64; rr = e / 64; }
-      const int r = r0 + rr, k = k0 + kk;
-      tile[rr][kk] = (r < R && k < K) ? oz_fetch(s, r, k) : 0.0;
+    if (oz_plain(s)) {
+      // contiguous along r: sixteen independent loads per thread, then the tile
+      const double* src = reinterpret_cast<const double*>(s.op.p);
+      const int64_t ld = s.op.ld;
+      double v[16];
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        const int e = tid + 256 * i;
+        const int r = r0 + e % 64, k = k0 + e / 64;
+        v[i] = (r < R && k < K) ? src[(int64_t)r + (int64_t)k * ld] : 0.0;
+      }
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        const int e = tid + 256 * i;
+        tile[e % 64][e / 64] = v[i];
+      }
+    } else {
+      for (int e = tid; e < 64 * 64; e += 256) {
+        int rr, kk;
+        if (cr) { rr = e % 64; kk = e / 64; } else { kk = e % 64; rr = e / 64; }
+        const int r = r0 + rr, k = k0 + kk;
+        tile[rr][kk] = (r < R && k < K) ? oz_fetch(s, r, k) : 0.0;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const int e = tid + 256 * u;
+#pragma unroll
+      for (int h = 0; h < 8; h++) x[u][h] = tile[e / 8][(e % 8) * 8 + h];
     }
   }
-  __syncthreads();
-  constexpr int FB = OZ_BITS * S;  // fractional bits of the fixed-point value
-  static_assert(FB <= 56, "the fixed-point value fits 28 + 28 bits");
   const size_t plane_stride = (size_t)Rpad * Kpad;
-  // each thread: one row, eight adjacent k (one 16-byte store per plane).
-  // Digits are cut with 32-bit integer operations (the value as two 28-bit
-  // halves) and each bf16 plane value d 2^(-7p) is assembled from a table of
-  // the bf16 bit patterns of the digits -64..64 by lowering the exponent
-  // field by 7p: no conversion instructions.
-  for (int e = tid; e < 64 * 8; e += 256) {
-    const int rr = e / 8, kq = (e % 8) * 8;
-    const int r = r0 + rr;
-    const int k = k0 + kq;
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const int e = tid + 256 * u;
+    const int r = r0 + e / 8, k = k0 + (e % 8) * 8;
     if (r >= Rpad || k >= Kpad) continue;
     const int Fr = ((r < R) ? exp_of_absbits(o.bits[r]) : 0) + OZ_HEADROOM;  // frame: |x| < 2^(Fr - 1)
     unsigned packed[S][4];
 #pragma unroll
-    for (int h = 0; h < 8; h++) {
-      const double x = tile[rr][kq + h];
-      const unsigned long long bts = (unsigned long long)__double_as_longlong(x);
-      const bool neg = (bts >> 63) != 0;
-      int ex = (int)((bts >> 52) & 0x7FF);
-      unsigned long long m = bts & 0x000FFFFFFFFFFFFFull;
-      if (ex == 0) ex = 1; else m |= 0x0010000000000000ull;
-      // f = |x| 2^(FB - Fr) rounded to nearest: f <= 2^(FB - 1)
-      const int sh = ex - 1075 + FB - Fr;
-      unsigned long long f;
-      if ((bts & 0x7FFFFFFFFFFFFFFFull) == 0) f = 0;
-      else if (sh >= 0) f = (sh >= 11) ? 0 : (m << sh);
-      else if (-sh >= 55) f = 0;
-      else f = (m >> (-sh)) + ((m >> (-sh - 1)) & 1ull);
-      // balanced base-2^7 digits d_p (plane p weighs 2^(-7p)): d_p in
-      // [-64, 63] below the leading digit, which is in [0, 64].  Adding
-      // 64 to every digit position (the constant BIAS) turns the balanced
-      // digits into the plain base-128 digits t_p = d_p + 64 of f + BIAS, so
-      // each is one shift and one mask, with no carries
-      constexpr unsigned long long BIAS = [] {
-        unsigned long long b = 0;
-        for (int i = 0; i < S; i++) b |= 64ull << (OZ_BITS * i);
-        return b;
-      }();
-      const unsigned long long u = f + BIAS;
-      const unsigned short* tb = &lut[neg ? 1 : 0][0][0];
+    for (int h = 0; h < 4; h++) {
+      unsigned a[S], b[S];
+      oz_digits<S>(x[u][2 * h], Fr, a);
+      oz_digits<S>(x[u][2 * h + 1], Fr, b);
 #pragma unroll
-      for (int p = 0; p < S; p++) {
-        unsigned t = (unsigned)(u >> (OZ_BITS * (S - 1 - p)));
-        // the leading digit is at most 64 when |x| < 2^(Fr - 1); the bound
-        // also keeps the table index in range for an operand that changed
-        // between the two passes
-        t = p == 0 ? (t < 128u ? t : 128u) : (t & 127u);
-        const unsigned b = tb[p * 130 + t];
-        if (h & 1) packed[p][h >> 1] |= b << 16;
-        else packed[p][h >> 1] = b;
-      }
+      for (int p = 0; p < S; p++) packed[p][h] = __byte_perm(a[p], b[p], 0x7632);
     }
 #pragma unroll
     for (int p = 0; p < S; p++)
-      *reinterpret_cast<uint4*>(planes + p * plane_stride + (size_t)r * Kpad + k) =
+      *reinterpret_cast<uint4*>(o.planes + p * plane_stride + (size_t)r * Kpad + k) =
           make_uint4(packed[p][0], packed[p][1], packed[p][2], packed[p][3]);
   }
 }
