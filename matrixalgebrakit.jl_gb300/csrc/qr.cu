@@ -1191,49 +1191,59 @@ LookAhead* lookahead() {
   return state[d] == 1 ? &la[d] : nullptr;
 }
 
-// T factor of a JB-wide block reflector (LAPACK larft, forward, column-wise
-// storage: H_1 ... H_JB = I - V T V^H) from the Gram matrix G = V^H V and
-// tau.  T is the inverse of the upper triangular U with U_ii = 1/tau_i and
-// U_il = G_il (i < l): the larft recurrence T[0:j, j] = -tau_j T[0:j, 0:j]
-// G[0:j, j], T[j, j] = tau_j, satisfies T U = I column by column.  Every
-// column of T is therefore an independent back substitution,
-//   x_k = tau_k,   x_i = -tau_i sum_{l=i+1..k} G_il x_l   (i < k),
-// written with tau_i as a factor so that tau_i = 0 (an identity reflector)
-// zeroes its row and column of T without a division.  One warp per column;
-// lane t owns rows t, t + 32, t + 64, t + 96.
+// T factor of a JB-wide block reflector H_1 ... H_JB = I - V T V^H (forward,
+// column-wise storage) from the Gram matrix G = V^H V and the T factors of its
+// nb-wide panels.  With the panels' columns V_0, V_1, ... and Ta the T factor
+// of panel a, T is block upper triangular with the Ta on its diagonal and
+// satisfies T_ab = -Ta sum_{a < c <= b} G_ac T_cb, so every column is an
+// independent block back substitution.  One warp per column, lane = row of a
+// block; eight columns of G in flight.  A warp-wide FP64 operation holds its
+// sub-partition's pipe for 64 cycles: four warps per CTA, and 288 operations
+// for the last column of 128 against 640 by single rows (Float64 70 us,
+// ComplexF64 197 us per 128 columns before).
+constexpr int LARFT_WARPS = 4;
 template <class T>
-__global__ void __launch_bounds__(256) larft_cols_kernel(int jb, const T* __restrict__ G, int ldg,
-                                                         const T* __restrict__ tau, T* Tout,
-                                                         int ldt) {
-  constexpr int RPL = QR_OUTER_NB / 32;
-  const int lane = threadIdx.x & 31;
-  const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
+__global__ void __launch_bounds__(32 * LARFT_WARPS)
+larft_blocks_kernel(int jb, int nb, const T* __restrict__ G, int ldg, const T* __restrict__ Ts,
+                    T* Tout, int ldt) {
+  __shared__ T xs[LARFT_WARPS][QR_OUTER_NB];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int k = blockIdx.x * LARFT_WARPS + wid;
   if (k >= jb) return;
-  T acc[RPL], x[RPL];
+  T* const x = xs[wid];
+  const int b = k / nb, kc = k - b * nb;
+  for (int i = lane; i < QR_OUTER_NB; i += 32) x[i] = zero_<T>();
+  __syncwarp();
+  if (lane <= kc) x[b * nb + lane] = Ts[(int64_t)b * NBMAX * NBMAX + lane + kc * NBMAX];
+  __syncwarp();
+  for (int a = b - 1; a >= 0; a--) {
+    const bool in = lane < nb;
+    const T* g = G + a * nb + (in ? lane : 0);
+    T y0 = zero_<T>(), y1 = zero_<T>();
+    int l = (a + 1) * nb;
+    for (; l + 7 <= k; l += 8) {
+      T v[8];
 #pragma unroll
-  for (int r = 0; r < RPL; r++) {
-    acc[r] = zero_<T>();
-    x[r] = zero_<T>();
-  }
-  for (int l = k; l >= 0; l--) {
-    const int slot = l >> 5, owner = l & 31;
-    T mine = acc[0];
+      for (int q = 0; q < 8; q++) v[q] = g[(int64_t)(l + q) * ldg];
 #pragma unroll
-    for (int r = 1; r < RPL; r++)
-      if (slot == r) mine = acc[r];
-    const T xl = (l == k) ? tau[k] : shfl_idx_(-(tau[l] * mine), owner);
-#pragma unroll
-    for (int r = 0; r < RPL; r++) {
-      if (slot == r && lane == owner) x[r] = xl;
-      const int i = lane + 32 * r;
-      if (i < l) acc[r] = fma_(G[i + (int64_t)l * ldg], xl, acc[r]);
+      for (int q = 0; q < 8; q += 2) {
+        y0 = fma_(v[q], x[l + q], y0);
+        y1 = fma_(v[q + 1], x[l + q + 1], y1);
+      }
     }
+    for (; l <= k; l++) y0 = fma_(g[(int64_t)l * ldg], x[l], y0);
+    const T y = in ? -(y0 + y1) : zero_<T>();
+    const T* t = Ts + (int64_t)a * NBMAX * NBMAX + lane;
+    T s = zero_<T>();
+#pragma unroll 8
+    for (int c = 0; c < nb; c++) {
+      const T yc = shfl_idx_(y, c);
+      s = fma_(t[c * NBMAX], yc, s);  // Ta is stored with its lower zeros
+    }
+    if (in) x[a * nb + lane] = s;
+    __syncwarp();
   }
-#pragma unroll
-  for (int r = 0; r < RPL; r++) {
-    const int i = lane + 32 * r;
-    if (i < jb) Tout[i + (int64_t)k * ldt] = (i <= k) ? x[r] : zero_<T>();
-  }
+  for (int i = lane; i < jb; i += 32) Tout[i + (int64_t)k * ldt] = i <= k ? x[i] : zero_<T>();
 }
 
 template <class T>
@@ -1735,8 +1745,8 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
       }
       T* const Tmid = Tb + (M0 - J0) * (NBO + 1);
       note_launch();
-      larft_cols_kernel<T><<<(unsigned)ceil_div(MB, 8), 256, 0, s>>>(MB, Gm, MB, tau + M0, Tmid,
-                                                                    NBO);
+      larft_blocks_kernel<T><<<(unsigned)ceil_div(MB, LARFT_WARPS), 32 * LARFT_WARPS, 0, s>>>(
+          MB, nb, Gm, MB, Ts + (M0 / nb) * NBMAX * NBMAX, Tmid, NBO);
       MAK_CUDA_TRY(cudaGetLastError());
       const int rest = (int)(J0 + JB - M0 - MB);
       if (rest > 0)

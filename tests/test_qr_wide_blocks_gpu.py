@@ -40,3 +40,16 @@ def test_merged_block_reflectors(mak, cuda, m, n, dt, full):
     assert float(torch.linalg.norm(Q @ R - Ad) / torch.linalg.norm(Ad)) <= 5e-13
     eye = torch.eye(Q.shape[1], dtype=Q.dtype, device=cuda)
     assert float(torch.linalg.norm(Q.mH @ Q - eye)) <= 5e-13 * np.sqrt(Q.shape[1])
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.complex128], ids=lambda d: np.dtype(d).name)
+@pytest.mark.parametrize("blocksize", [0, 5, 24, 31])
+def test_t_factor_from_panels(mak, cuda, dt, blocksize):
+    """The 128-wide T factor from panels whose width does not divide 128."""
+    rng = np.random.default_rng(blocksize)
+    A = O.gaussian(rng, 700, 300, dt)
+    Ad = to_dev(A, cuda)
+    Q, R = mak.qr_compact(Ad, precision="mixed", blocksize=blocksize)
+    assert O.rel_err(to_host(R), O.qr_compact(A)[1]) <= 5e-13
+    assert O.qr_residual(A, to_host(Q), to_host(R)) <= 5e-13
+    assert O.orth_error(to_host(Q)) <= 5e-13 * np.sqrt(300)
