@@ -62,6 +62,53 @@ constexpr int GEMM_BK = 32;  // K per step (and the granule of a K split)
 template <class T>
 __device__ __forceinline__ bool is_zero_(T v) { return v == zero_<T>(); }
 
+// A thread's share (L elements) of the B x BK tile of an operand at (i0, k0),
+// i along the tile's B side (rows of op(A), columns of op(B)).  `ci`: the
+// stored matrix is contiguous along i, so that i runs fastest over the
+// threads; else k does.  A tile inside the operand that no structure mask
+// touches (decided once, for the whole CTA) is read with one address step per
+// element; the general form costs tens of instructions per element, three
+// quarters of all issued in an FP32 update of K = 32.
+template <class T, int B, int BK, int NT, int L>
+__device__ __forceinline__ void fetch_tile(const Operand<T>& X, bool ci, int64_t i0, int64_t ilim,
+                                           int k0, int kend, T (&v)[L]) {
+  const int tid = threadIdx.x;
+  bool plain = i0 + B <= ilim && k0 + BK <= kend;
+  if (X.mask != MASK_FULL) {
+    const int64_t rlo = ci ? i0 : k0, rhi = rlo + (ci ? B : BK) - 1;
+    const int64_t clo = ci ? k0 : i0, chi = clo + (ci ? BK : B) - 1;
+    plain = plain && (X.mask == MASK_UPPER ? rhi <= clo
+                                           : (X.mask == MASK_LOWER ? rlo >= chi : rlo > chi));
+  }
+  if (plain) {
+    const T* p = X.p + (ci ? (i0 + tid % B) + (int64_t)(k0 + tid / B) * X.ld
+                           : (int64_t)(k0 + tid % BK) + (i0 + tid / BK) * X.ld);
+    const int64_t step = (ci ? NT / B : NT / BK) * X.ld;
+#pragma unroll
+    for (int q = 0; q < L; q++) v[q] = p[q * step];
+    if (traits<T>::cpx && X.op == OP_C) {
+#pragma unroll
+      for (int q = 0; q < L; q++) v[q] = conj_(v[q]);
+    }
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < L; q++) {
+    const int e = tid + q * NT;
+    const int64_t gi = i0 + (ci ? e % B : e / BK);
+    const int gk = k0 + (ci ? e / B : e % BK);
+    T x = zero_<T>();
+    if (gi < ilim && gk < kend) {
+      const int64_t r = ci ? gi : gk, c = ci ? gk : gi;
+      if (X.mask == MASK_UNIT_LOWER && r <= c) x = r == c ? one_<T>() : zero_<T>();
+      else if ((X.mask == MASK_UPPER && r > c) || (X.mask == MASK_LOWER && r < c)) x = zero_<T>();
+      else x = X.p[r + c * X.ld];
+      if (X.op == OP_C) x = conj_(x);
+    }
+    v[q] = x;
+  }
+}
+
 // One BM x BN tile of C per CTA of 256 threads (TM x TN outputs each).  The
 // next K step's elements are fetched into registers while the current one is
 // multiplied.
@@ -91,27 +138,25 @@ gemm_kernel(int M, int N, int K, T alpha, Operand<T> A, Operand<T> B, T beta, T*
     for (int c = 0; c < TN; c++) acc[r][c] = zero_<T>();
 
   T ra[LA], rb[LB];
+  static_assert(NT % BM == 0 && NT % BN == 0 && NT % BK == 0, "whole address steps");
   auto fetch = [&](int k0) {
-#pragma unroll
-    for (int q = 0; q < LA; q++) {
-      const int e = tid + q * NT;
-      int ii, kk;
-      if (A.op == OP_N) { ii = e % BM; kk = e / BM; } else { kk = e % BK; ii = e / BK; }
-      const int64_t gi = m0 + ii;
-      const int gk = k0 + kk;
-      ra[q] = (gi < M && gk < kend) ? load_op(A, gi, gk) : zero_<T>();
-    }
-#pragma unroll
-    for (int q = 0; q < LB; q++) {
-      const int e = tid + q * NT;
-      int kk, jj;
-      if (B.op == OP_N) { kk = e % BK; jj = e / BK; } else { jj = e % BN; kk = e / BN; }
-      const int64_t gj = n0 + jj;
-      const int gk = k0 + kk;
-      rb[q] = (gj < N && gk < kend) ? load_op(B, gk, gj) : zero_<T>();
-    }
+    fetch_tile<T, BM, BK, NT, LA>(A, A.op == OP_N, m0, M, k0, kend, ra);
+    fetch_tile<T, BN, BK, NT, LB>(B, B.op != OP_N, n0, N, k0, kend, rb);
   };
   if (kbeg < kend) fetch(kbeg);
+  // C before the products: its loads are then in flight together (after them,
+  // each would wait for the store before it, which may alias)
+  const bool use_beta = !is_zero_(beta);
+  T cv[TM][TN];
+  if (use_beta) {
+#pragma unroll
+    for (int c = 0; c < TN; c++)
+#pragma unroll
+      for (int r = 0; r < TM; r++) {
+        const int64_t i = m0 + tx + r * RX, j = n0 + ty + c * RY;
+        cv[r][c] = (i < M && j < N) ? C[i + j * ldc] : zero_<T>();
+      }
+  }
   for (int k0 = kbeg; k0 < kend; k0 += BK) {
 #pragma unroll
     for (int q = 0; q < LA; q++) {
@@ -141,7 +186,6 @@ gemm_kernel(int M, int N, int K, T alpha, Operand<T> A, Operand<T> B, T beta, T*
     }
     __syncthreads();
   }
-  const bool use_beta = !is_zero_(beta);
 #pragma unroll
   for (int c = 0; c < TN; c++) {
     int64_t j = n0 + ty + c * RY;
@@ -151,9 +195,130 @@ gemm_kernel(int M, int N, int K, T alpha, Operand<T> A, Operand<T> B, T beta, T*
       int64_t i = m0 + tx + r * RX;
       if (i >= M) continue;
       T v = alpha * acc[r][c];
-      if (use_beta) v = fma_(beta, C[i + j * ldc], v);
+      if (use_beta) v = fma_(beta, cv[r][c], v);
       C[i + j * ldc] = v;
     }
+  }
+}
+
+// The FP32 types' tile: 128 multiply-adds per clock per SM, so the operands'
+// shared-memory reads decide.  A thread's TN columns are adjacent and read as
+// 16-byte vectors; its TM rows are RX apart (lanes along the rows, C accessed
+// in whole lines) or, with ROWC, adjacent and read as vectors too.  Reads per
+// warp and k (in 128-byte wavefronts) against FMA cycles: 128 x 64 (TM 4, TN
+// 8, RX 32) 6 : 8, 64 x 64 (TM 2) 4 : 4, 32 x 128 (TM 4, TN 4, RX 8, ROWC)
+// 2 : 4; the scalar reads of a 4 x 4 tile were 8 : 4.
+template <class T, int BM, int BN, int BK, int TM, int TN, int RX, bool ROWC>
+__global__ void __launch_bounds__(256)
+gemm_f32_kernel(int M, int N, int K, T alpha, Operand<T> A, Operand<T> B, T beta, T* C,
+                int64_t ldc, int kchunk, int64_t split_stride, const int* skip) {
+  if (skipped(skip)) return;
+  constexpr int NT = 256, RY = NT / RX;
+  static_assert(RX * TM == BM && RY * TN == BN, "256 threads cover the tile");
+  constexpr int LA = BM * BK / NT, LB = BN * BK / NT;
+  constexpr int V = 16 / sizeof(T);  // elements per vector read
+  static_assert(TN % V == 0 && (!ROWC || TM % V == 0), "whole vectors");
+  struct alignas(16) Vec { T v[V]; };
+  __shared__ alignas(16) T As[BK][BM + V];
+  __shared__ alignas(16) T Bs[BK][BN + V];
+  const int64_t m0 = (int64_t)blockIdx.x * BM;
+  const int64_t n0 = (int64_t)blockIdx.y * BN;
+  const int kbeg = blockIdx.z * kchunk;
+  const int kend = min(K, kbeg + kchunk);
+  C += blockIdx.z * split_stride;
+  const int tid = threadIdx.x, tx = tid % RX, ty = tid / RX;
+  T acc[TM][TN];
+#pragma unroll
+  for (int r = 0; r < TM; r++)
+#pragma unroll
+    for (int c = 0; c < TN; c++) acc[r][c] = zero_<T>();
+  T ra[LA], rb[LB];
+  static_assert(NT % BM == 0 && NT % BN == 0 && NT % BK == 0, "whole address steps");
+  auto fetch = [&](int k0) {
+    fetch_tile<T, BM, BK, NT, LA>(A, A.op == OP_N, m0, M, k0, kend, ra);
+    fetch_tile<T, BN, BK, NT, LB>(B, B.op != OP_N, n0, N, k0, kend, rb);
+  };
+  if (kbeg < kend) fetch(kbeg);
+  // C before the products: its loads are then in flight together (after them,
+  // each would wait for the store before it, which may alias)
+  const bool use_beta = !is_zero_(beta);
+  T cv[TM][TN];
+  // (a tile inside C takes one address step per element)
+  constexpr int RS = ROWC ? 1 : RX;
+  const bool inner = m0 + BM <= M && n0 + BN <= N;
+  const int64_t i0 = m0 + (ROWC ? tx * TM : tx), j0 = n0 + ty * TN;
+  T* const C0 = C + i0 + j0 * ldc;
+  if (use_beta) {
+#pragma unroll
+    for (int c = 0; c < TN; c++)
+#pragma unroll
+      for (int r = 0; r < TM; r++)
+        cv[r][c] = inner || (i0 + r * RS < M && j0 + c < N) ? C0[r * RS + c * ldc] : zero_<T>();
+  }
+  for (int k0 = kbeg; k0 < kend; k0 += BK) {
+#pragma unroll
+    for (int q = 0; q < LA; q++) {
+      const int e = tid + q * NT;
+      if (A.op == OP_N) As[e / BM][e % BM] = ra[q];
+      else As[e % BK][e / BK] = ra[q];
+    }
+#pragma unroll
+    for (int q = 0; q < LB; q++) {
+      const int e = tid + q * NT;
+      if (B.op == OP_N) Bs[e % BK][e / BK] = rb[q];
+      else Bs[e / BN][e % BN] = rb[q];
+    }
+    __syncthreads();
+    if (k0 + BK < kend) fetch(k0 + BK);
+#pragma unroll 4
+    for (int kk = 0; kk < BK; kk++) {
+      T a[TM], b[TN];
+      if constexpr (ROWC) {
+#pragma unroll
+        for (int r = 0; r < TM; r += V) {
+          const Vec v = *reinterpret_cast<const Vec*>(&As[kk][tx * TM + r]);
+#pragma unroll
+          for (int q = 0; q < V; q++) a[r + q] = v.v[q];
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < TM; r++) a[r] = As[kk][tx + r * RX];
+      }
+#pragma unroll
+      for (int c = 0; c < TN; c += V) {
+        const Vec v = *reinterpret_cast<const Vec*>(&Bs[kk][ty * TN + c]);
+#pragma unroll
+        for (int q = 0; q < V; q++) b[c + q] = v.v[q];
+      }
+#pragma unroll
+      for (int r = 0; r < TM; r++)
+#pragma unroll
+        for (int c = 0; c < TN; c++) acc[r][c] = fma_(a[r], b[c], acc[r][c]);
+    }
+    __syncthreads();
+  }
+  if (use_beta) {
+#pragma unroll
+    for (int c = 0; c < TN; c++)
+#pragma unroll
+      for (int r = 0; r < TM; r++) acc[r][c] = fma_(beta, cv[r][c], alpha * acc[r][c]);
+  } else {
+#pragma unroll
+    for (int c = 0; c < TN; c++)
+#pragma unroll
+      for (int r = 0; r < TM; r++) acc[r][c] = alpha * acc[r][c];
+  }
+  if (inner) {
+#pragma unroll
+    for (int c = 0; c < TN; c++)
+#pragma unroll
+      for (int r = 0; r < TM; r++) C0[r * RS + c * ldc] = acc[r][c];
+  } else {
+#pragma unroll
+    for (int c = 0; c < TN; c++)
+#pragma unroll
+      for (int r = 0; r < TM; r++)
+        if (i0 + r * RS < M && j0 + c < N) C0[r * RS + c * ldc] = acc[r][c];
   }
 }
 
@@ -201,25 +366,36 @@ int gemm(cudaStream_t st, int64_t M, int64_t N, int64_t K, T alpha, Operand<T> A
     if (t32 >= 3 * (int64_t)num_sms()) MAK_GEMM_TILE(32, 32, GEMM_BK, 2, 2);
     else MAK_GEMM_TILE(16, 16, GEMM_BK, 1, 1);
   } else {
-    // FP32 is bound by shared memory bandwidth in a small tile (two loads per
-    // FMA), so it is taken only where the wide ones would leave SMs idle
-    // (1537 x 4093 Float32 LQ 8.6 -> 6.0 ms)
-    if (t32 < 2 * (int64_t)num_sms()) MAK_GEMM_TILE(32, 32, GEMM_BK, 2, 2);
-    else if (M <= 32) MAK_GEMM_TILE(32, 64, 16, 2, 4);
-    else MAK_GEMM_TILE(64, 64, 16, 4, 4);
+    // wide tiles where they fill the GPU (their operand reads are the
+    // cheapest), smaller ones before SMs idle.  The 4093 x 1537 Float32 QR:
+    // W = V^H C 33 -> 20 us, C -= V W2 29 -> 19 us per panel, the LQ 6.0 ->
+    // 5.0 ms (issue slots, 63 % busy; the tiles' sizes hardly matter)
+#define MAK_GEMM32_TILE(BM, BN, BK, TM, TN, RX, ROWC)                                            \
+  gemm_f32_kernel<T, BM, BN, BK, TM, TN, RX, ROWC>                                               \
+      <<<dim3((unsigned)ceil_div(M, BM), (unsigned)ceil_div(N, BN), (unsigned)splits), 256, 0,   \
+         st>>>((int)M, (int)N, (int)K, alpha, A, B, beta, C, ldc, kchunk, split_stride,          \
+               skip_flag())
+    const int64_t sms = num_sms();
+    if (M <= 32 && ceil_div(N, 128) * splits >= sms)
+      MAK_GEMM32_TILE(32, 128, 32 / (sizeof(T) / 4), 4, 4, 8, true);
+    else if (ceil_div(M, 128) * ceil_div(N, 64) * splits >= 2 * sms)
+      MAK_GEMM32_TILE(128, 64, 16, 4, 8, 32, false);
+    else if (t32 >= 4 * sms) MAK_GEMM32_TILE(64, 64, 16, 2, 8, 32, false);
+    else MAK_GEMM_TILE(32, 32, GEMM_BK, 2, 2);
+#undef MAK_GEMM32_TILE
   }
 #undef MAK_GEMM_TILE
   return cudaGetLastError() == cudaSuccess ? 0 : MAK_ERR_CUDA;
 }
 
 // number of K-splits that fills the GPU for an output of M x N: two 32 x 32
-// tiles per SM for the FP64 types (at least 32 of K per split), two 64-wide
-// tiles for the FP32 types (at least 64)
+// tiles per SM for the FP64 types (at least 32 of K per split), two 32 x 128
+// or 64 x 64 tiles for the FP32 types (at least 64)
 template <class T>
 inline int pick_splits(int64_t M, int64_t N, int64_t K, int sms) {
   constexpr bool f64 = sizeof(real_t<T>) == 8;
   const int64_t tiles = f64 ? ceil_div(M, 32) * ceil_div(N, 32)
-                            : ceil_div(M, M <= 32 ? 32 : 64) * ceil_div(N, 64);
+                            : ceil_div(M, M <= 32 ? 32 : 64) * ceil_div(N, M <= 32 ? 128 : 64);
   int64_t want = 2LL * sms;
   if (tiles >= want) return 1;
   int64_t s = ceil_div(want, tiles);

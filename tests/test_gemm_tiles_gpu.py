@@ -44,3 +44,23 @@ def test_native_gemm_tiles(mak, cuda, dt, ops, shape):
     eps = np.finfo(np.float64).eps
     bound = 4 * (k + 4) * eps * (np.abs(a) @ np.abs(b) + np.abs(C0))
     assert np.all(np.abs(to_host(C) - ref) <= 2 * bound)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.complex64], ids=lambda d: np.dtype(d).name)
+@pytest.mark.parametrize("shape", [(4100, 65), (3000, 320), (700, 690), (520, 515), (129, 96)],
+                         ids=lambda s: f"{s[0]}x{s[1]}")
+def test_fp32_tiles_through_qr(mak, cuda, dt, shape):
+    """The FP32 tiles (32 x 128, 128 x 64, 64 x 64, 32 x 32 as the trailing
+    matrix shrinks) with masks, splits and ragged edges, through a QR whose
+    products they are; bound: backward stability, 170 eps sqrt(n)."""
+    m, n = shape
+    rng = np.random.default_rng(m)
+    A = rng.standard_normal((m, n))
+    A = (A + 1j * rng.standard_normal((m, n)) if dt is np.complex64 else A).astype(dt)
+    for X in (A, np.asfortranarray(A.conj().T)):
+        Q, R = mak.qr_compact(to_dev(X, cuda))
+        Qh, Rh = to_host(Q).astype(np.complex128), to_host(R).astype(np.complex128)
+        k = min(X.shape)
+        bound = 2e-5 * np.sqrt(k)
+        assert np.linalg.norm(X - Qh @ Rh) <= bound * np.linalg.norm(X)
+        assert np.linalg.norm(Qh.conj().T @ Qh - np.eye(k)) <= bound * np.sqrt(k)
