@@ -23,6 +23,12 @@ template <class T>
 int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int precision,
                 Arena& ar, mak_info* info);
 
+// inv(R) of the upper triangular n x n matrix R (its upper triangle is read)
+// into X (n x n, leading dimension n, zero below the diagonal).
+template <class T>
+int tri_inverse(cudaStream_t st, int64_t n, const T* R, int64_t ldr, T* X, int precision,
+                Arena& ar, mak_info* info);
+
 int info_reset(cudaStream_t st, mak_info* info);
 
 // qr_pullback! (dA += ...); known_p >= 0 skips the host read of the rank

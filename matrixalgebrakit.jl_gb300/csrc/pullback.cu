@@ -217,13 +217,12 @@ int qr_pullback_run(cudaStream_t st, int64_t m, int64_t n, int full, T* dA, int6
   T* X = ar.take<T>((size_t)(k > 0 ? k : 1) * (k > 0 ? k : 1));
   T* Mm = ar.take<T>((size_t)(k > 0 ? k : 1) * (k > 0 ? k : 1));
   T* Rinv = ar.take<T>((size_t)(k > 0 ? k : 1) * (k > 0 ? k : 1));
-  int* iperm = ar.take<int>(k + 1);
   T* Q1dQ3 = (full && qc > k) ? ar.take<T>((size_t)k * (qc - k)) : nullptr;
   T* dQ3 = (full && qc > k) ? ar.take<T>((size_t)m * (qc - k)) : nullptr;
   size_t gj_ws = 0, oz_ws = 0;
   {
     Arena meas(nullptr, 0);
-    gje_inverse<T>(st, k, nullptr, k, nullptr, precision, meas, nullptr);
+    tri_inverse<T>(st, k, nullptr, k, nullptr, precision, meas, nullptr);
     gj_ws = meas.off + 256;
     const int64_t shapes[4][3] = {{k, k, n}, {m, n, k}, {k, k, m}, {m, k, k}};
     for (auto& sh : shapes) {
@@ -323,15 +322,10 @@ int qr_pullback_run(cudaStream_t st, int64_t m, int64_t n, int full, T* dA, int6
     MAK_CUDA_TRY(cudaGetLastError());
     MAK_TRY(G(m, p, p, one_<T>(), opnd<T>(Q, ldq), opnd<T>(Mm, p), one_<T>(), dQ1, m));
     // dA1 += dQ1 R11^{-H}
-    MAK_TRY(copy_mat<T>(st, p, p, R, ldr, X, p));
     {
-      Arena gj(tail, tail_bytes);
-      MAK_TRY(gje_inverse<T>(st, p, X, p, iperm, precision, gj, info));
+      Arena tri(tail, tail_bytes);
+      MAK_TRY(tri_inverse<T>(st, p, R, ldr, Rinv, precision, tri, info));
     }
-    note_launch();
-    gather_cols_kernel<T><<<dim3((unsigned)ceil_div(p, 128), (unsigned)p), 128, 0, st>>>(
-        (int)p, X, p, iperm, Rinv, p);
-    MAK_CUDA_TRY(cudaGetLastError());
     MAK_TRY(G(m, p, p, one_<T>(), opnd<T>(dQ1, m), opnd<T>(Rinv, p, OP_C, MASK_UPPER), one_<T>(),
               dA, ldda));
   }
@@ -906,7 +900,6 @@ static int qr_null_pullback_run(cudaStream_t st, int64_t m, int64_t n, T* dA, in
   T* G1 = ar.take<T>((size_t)nc * k + 1);
   T* X = ar.take<T>((size_t)nc * k + 1);
   T* Rinv = ar.take<T>((size_t)k * k + 1);
-  int* iperm = ar.take<int>(k + 1);
   size_t tail_bytes = 0;
   {
     Arena mq(nullptr, 0);
@@ -914,7 +907,7 @@ static int qr_null_pullback_run(cudaStream_t st, int64_t m, int64_t n, T* dA, in
               k > 0 ? k : 1, k, 1, 0, precision, mq, nullptr);
     tail_bytes = mq.off + 256;
     Arena mg(nullptr, 0);
-    gje_inverse<T>(st, k, nullptr, k > 0 ? k : 1, nullptr, precision, mg, nullptr);
+    tri_inverse<T>(st, k, nullptr, k > 0 ? k : 1, nullptr, precision, mg, nullptr);
     if (mg.off + 256 > tail_bytes) tail_bytes = mg.off + 256;
     const int64_t shapes[4][3] = {{nc, nc, m}, {nc, k, m}, {nc, k, k}, {m, k, nc}};
     for (auto& sh : shapes) {
@@ -971,13 +964,9 @@ static int qr_null_pullback_run(cudaStream_t st, int64_t m, int64_t n, T* dA, in
       // G1 = dN^H Q;  R^{-1};  X = G1 R^{-H};  dA -= N X
       MAK_TRY(G(nc, k, m, one_<T>(), opnd<T>(dN, lddn, OP_C), opnd<T>(Qc, m), zero_<T>(), G1, nc));
       {
-        Arena gj(tail, tail_bytes);
-        MAK_TRY(gje_inverse<T>(st, k, Rc, k, iperm, precision, gj, info));
+        Arena tri(tail, tail_bytes);
+        MAK_TRY(tri_inverse<T>(st, k, Rc, k, Rinv, precision, tri, info));
       }
-      note_launch();
-      gather_cols_kernel<T><<<dim3((unsigned)ceil_div(k, 128), (unsigned)k), 128, 0, st>>>(
-          (int)k, Rc, k, iperm, Rinv, k);
-      MAK_CUDA_TRY(cudaGetLastError());
       MAK_TRY(G(nc, k, k, one_<T>(), opnd<T>(G1, nc), opnd<T>(Rinv, k, OP_C, MASK_UPPER),
                 zero_<T>(), X, nc));
       MAK_TRY(G(m, k, nc, -one_<T>(), opnd<T>(N, ldn), opnd<T>(X, nc), one_<T>(), dA, ldda));
