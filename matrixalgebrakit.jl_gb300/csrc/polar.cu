@@ -1080,37 +1080,50 @@ __global__ void __launch_bounds__(256) newton_update_kernel(int n, T* X, int64_t
   using R = real_t<T>;
   __shared__ T t[32][33];
   __shared__ R sh[32];
+  __shared__ R gs[2];
   const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {  // two roots and two divisions, once per CTA
+    gs[0] = sqrt(sqrt(nrm2[1] / nrm2[0]));
+    gs[1] = R(1) / gs[0];
+  }
   for (int r = ty; r < 32; r += 8) {
     const int i = i0 + r, j = j0 + tx;
     t[r][tx] = (i < n && j < n) ? Xi[j + (int64_t)iperm[i] * ldi] : zero_<T>();  // t[i'][j'] = Xi[j, iperm[i]]
   }
   __syncthreads();
-  const R g = sqrt(sqrt(nrm2[1] / nrm2[0]));
-  const R ginv = R(1) / g;
-  R dmax = R(0);
+  const R g = gs[0], ginv = gs[1];
+  R dmax = R(0);  // complex: of |D|^2, so that no square root is taken per element
   for (int r = ty; r < 32; r += 8) {
     const int i = i0 + tx, j = j0 + r;
     if (i < n && j < n) {
       const T y = conj_(t[tx][r]) * ginv;
       const T x = g * X[i + (int64_t)j * ldx];
       X[i + (int64_t)j * ldx] = R(0.5) * (x + y);
-      dmax = fmax(dmax, abs_(y - x));
+      dmax = fmax(dmax, traits<T>::cpx ? abs2_(y - x) : abs_(y - x));
     }
   }
   dmax = block_max(dmax, sh);
+  if (traits<T>::cpx) dmax = sqrt(dmax);
   if (threadIdx.x == 0) atomic_max_nonneg(conv, dmax);
 }
 
 // Newton-Schulz finish (mixed precision, Float64 types): once a Newton step
-// measured n * max|D| <= 1/2 (so ||D||_2 <= ||D||_F <= 1/2 and the new
-// iterate's singular values lie in [1, 1.05]), the iteration continues with
+// had ||D||_F <= 1/2 (so ||D||_2 <= 1/2 and the new iterate's singular values
+// lie in [1, 1.05]), the iteration continues with
 // X <- X (3 I - X^H X) / 2, two products on the split tensor-core path
 // instead of a latency-bound Gauss-Jordan inverse; it converges
 // quadratically there (error e -> 1.5 e^2).  Its measure 2 max|dX| is on the
 // Newton step's scale (max|D| = 2 max|dX|) and meets the same tolerance.
-constexpr double NS_SWITCH = 0.5;  // n * max|D| at which Newton-Schulz takes over
+constexpr double NS_SWITCH = 0.5;  // ||D||_F at which Newton-Schulz takes over
+// ||D||_F from the two norms: D = Y/g - g X with Y = X^-H and g^2 = ||Y||/||X||,
+// and <Y, X> = tr(X^-1 X) = n, so ||D||_F^2 = 2 (||X|| ||Y|| - n); n max|D|
+// bounds it from above and decides where rounding hides the difference.
+template <class R>
+__host__ __device__ inline bool ns_takes_over(R conv, R nx2, R ny2, int64_t n) {
+  return (R)n * conv <= (R)NS_SWITCH ||
+         R(2) * (sqrt(nx2) * sqrt(ny2) - (R)n) <= (R)(NS_SWITCH * NS_SWITCH);
+}
 
 // Z <- 1.5 I - 0.5 Z  (n x n, ld n)
 template <class T>
@@ -1150,13 +1163,13 @@ __global__ void __launch_bounds__(256) ns_update_kernel(int64_t nn, T* X, const 
 // w: [0] stopped, [1] steps taken, [2] Newton-Schulz phase, [3] skip flag of
 // the Newton step's kernels, [4] skip flag of the Newton-Schulz step's.
 template <class R>
-__global__ void newton_stop_kernel(const R* conv, R tol, int* w, R* conv_last, int n,
-                                   int ns_ok) {
+__global__ void newton_stop_kernel(const R* conv, const R* nrm2, R tol, int* w, R* conv_last,
+                                   int n, int ns_ok) {
   if (w[0]) return;
   w[1] += 1;
   *conv_last = *conv;
   if (!(*conv > tol)) w[0] = 1;
-  else if (ns_ok && !w[2] && (R)n * *conv <= (R)NS_SWITCH) w[2] = 1;
+  else if (ns_ok && !w[2] && ns_takes_over(*conv, nrm2[0], nrm2[1], (int64_t)n)) w[2] = 1;
   w[3] = w[0] | w[2];
   w[4] = w[0] | !w[2];
 }
@@ -1317,18 +1330,20 @@ int polar_newton_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T
         MAK_TRY(ns_step());
       }
       note_launch();
-      newton_stop_kernel<R><<<1, 1, 0, st>>>(conv, (R)tol, stopw, conv_last, (int)n,
+      newton_stop_kernel<R><<<1, 1, 0, st>>>(conv, nrm2, (R)tol, stopw, conv_last, (int)n,
                                              ns_fixed_ok ? 1 : 0);
       MAK_CUDA_TRY(cudaGetLastError());
     } else {
       MAK_TRY(in_ns ? ns_step() : newton_step(it == 1 && m > n));
-      MAK_CUDA_TRY(cudaMemcpyAsync(&hconv, conv, sizeof(R), cudaMemcpyDeviceToHost, st));
+      R h[3];  // the two squared norms and max|D|
+      MAK_CUDA_TRY(cudaMemcpyAsync(h, nrm2, sizeof(h), cudaMemcpyDeviceToHost, st));
       MAK_CUDA_TRY(cudaStreamSynchronize(st));
+      hconv = h[2];
       if (!(hconv > (R)tol)) {  // also stops on NaN
         converged = hconv <= (R)tol;
         break;
       }
-      if (ns_ok && !in_ns && (R)n * hconv <= (R)NS_SWITCH) in_ns = true;
+      if (ns_ok && !in_ns && ns_takes_over(hconv, h[0], h[1], n)) in_ns = true;
     }
   }
   if (it > maxiter) it = maxiter;

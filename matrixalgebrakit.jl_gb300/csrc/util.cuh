@@ -79,6 +79,12 @@ inline int ctranspose(cudaStream_t st, int64_t m, int64_t n, const T* A, int64_t
 // ---- reductions -------------------------------------------------------------
 // Partial results per CTA, then one CTA folds them in a fixed order.
 constexpr int RED_CTAS = 304;
+constexpr int RED_ROWS = 512;
+__device__ __forceinline__ double sq_sum(double s, double x) { return fma_(x, x, s); }
+__device__ __forceinline__ float sq_sum(float s, float x) { return fma_(x, x, s); }
+template <class R> __device__ __forceinline__ R sq_sum(R s, cplx<R> x) {
+  return fma_(x.re, x.re, fma_(x.im, x.im, s));
+}
 
 // kind 0: sum |a|^2 (Frobenius^2), kind 1: max |a|
 template <class T>
@@ -87,14 +93,31 @@ __global__ void __launch_bounds__(256) reduce_partial_kernel(int64_t m, int64_t 
                                                              real_t<T>* part) {
   using R = real_t<T>;
   __shared__ R sh[32];
-  const int64_t total = m * n;
+  // units of one column by RED_ROWS rows, a warp per unit: lanes along the
+  // rows, four loads in flight, one division per unit
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int64_t chunks = (m + RED_ROWS - 1) / RED_ROWS;
   R acc = R(0);
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    int64_t i = e % m, j = e / m;
-    T v = A[i + j * lda];
-    if (kind == 0) acc += abs2_(v);
-    else acc = fmax(acc, abs_(v));
+  for (int64_t u = (int64_t)blockIdx.x * nw + (threadIdx.x >> 5); u < chunks * n;
+       u += (int64_t)gridDim.x * nw) {
+    const int64_t j = u / chunks, i0 = (u - j * chunks) * RED_ROWS;
+    const int64_t i1 = i0 + RED_ROWS < m ? i0 + RED_ROWS : m;
+    const T* col = A + j * lda;
+    int64_t i = i0 + lane;
+    for (; i + 96 < i1; i += 128) {
+      T v[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) v[q] = col[i + 32 * q];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        if (kind == 0) acc = sq_sum(acc, v[q]);
+        else acc = fmax(acc, abs_(v[q]));
+      }
+    }
+    for (; i < i1; i += 32) {
+      if (kind == 0) acc = sq_sum(acc, col[i]);
+      else acc = fmax(acc, abs_(col[i]));
+    }
   }
   R r = (kind == 0) ? block_sum(acc, sh) : block_max(acc, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = r;
