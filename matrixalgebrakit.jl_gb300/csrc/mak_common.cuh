@@ -432,29 +432,40 @@ __device__ __forceinline__ int dsmem_ld(const int* p, unsigned rank) {
   asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(dsmem_addr(p, rank)) : "memory");
   return v;
 }
-template <class R>
-__device__ __forceinline__ cplx<R> dsmem_ld(const cplx<R>* p, unsigned rank) {
-  return {dsmem_ld(&p->re, rank), dsmem_ld(&p->im, rank)};
+__device__ __forceinline__ zcomplex dsmem_ld(const zcomplex* p, unsigned rank) {
+  zcomplex v;
+  asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];"
+               : "=d"(v.re), "=d"(v.im)
+               : "r"(dsmem_addr(p, rank))
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ ccomplex dsmem_ld(const ccomplex* p, unsigned rank) {
+  ccomplex v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];"
+               : "=f"(v.re), "=f"(v.im)
+               : "r"(dsmem_addr(p, rank))
+               : "memory");
+  return v;
 }
 
-// Stores to the same variable in CTA `rank` of the cluster.
+// Stores to the same variable in CTA `rank` of the cluster (16 bytes: one
+// packet instead of two).
 __device__ __forceinline__ void dsmem_st(double* p, unsigned rank, double v) {
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(dsmem_addr(p, rank)), "d"(v) : "memory");
 }
 __device__ __forceinline__ void dsmem_st(float* p, unsigned rank, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dsmem_addr(p, rank)), "f"(v) : "memory");
 }
-__device__ __forceinline__ void dsmem_st(int* p, unsigned rank, int v) {
-  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(dsmem_addr(p, rank)), "r"(v) : "memory");
+__device__ __forceinline__ void dsmem_st(ccomplex* p, unsigned rank, ccomplex v) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(dsmem_addr(p, rank)), "f"(v.re),
+               "f"(v.im)
+               : "memory");
 }
-__device__ __forceinline__ void dsmem_st(unsigned long long* p, unsigned rank,
-                                         unsigned long long v) {
-  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(dsmem_addr(p, rank)), "l"(v) : "memory");
-}
-template <class R>
-__device__ __forceinline__ void dsmem_st(cplx<R>* p, unsigned rank, cplx<R> v) {
-  dsmem_st(&p->re, rank, v.re);
-  dsmem_st(&p->im, rank, v.im);
+__device__ __forceinline__ void dsmem_st(ulonglong2* p, unsigned rank, ulonglong2 v) {
+  asm volatile("st.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(dsmem_addr(p, rank)), "l"(v.x),
+               "l"(v.y)
+               : "memory");
 }
 
 // --------------------------------------------------------------- host side --

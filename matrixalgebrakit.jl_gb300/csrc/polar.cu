@@ -222,8 +222,11 @@ __global__ void __launch_bounds__(GJ_THREADS) gje_panel_kernel(GjArgs<T> a) {
 // one reciprocal and one round between the CTAs, and the elimination's FP64
 // work (rows x 32 per column at 1.66 per clock per SM) runs beside it.  In a
 // cluster (SYNC_CLUSTER) the candidates are pushed into every CTA's shared
-// memory before the cluster barrier, so that nothing is fetched after it; in
-// a grid they go through L2.  Elementwise arithmetic only: the result does
+// memory before the cluster barrier, so that nothing is fetched after it; the
+// 16-byte type pushes keys only and one warp pulls the winner's row (remote
+// stores run at about 5 bytes per clock: pushing all rows to 16 CTAs took 1650
+// of a ComplexF64 column's 7100 cycles, 5540 with the pull; a Float64 column
+// takes 3220 with the push, 3650 with the pull); in a grid they go through L2.  Elementwise arithmetic only: the result does
 // not depend on the number of CTAs.
 __device__ __forceinline__ unsigned long long pivot_key(double x) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
@@ -305,12 +308,13 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) gje_panel_ahead_kernel(GjArgs<T
   constexpr int GC = kCl ? kGjClusterWide : 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* const Xs = reinterpret_cast<T*>(smem_raw);  // [2][rpc][GJA_LD]
-  // by column parity: the CTAs' candidates (scaled rows) and row jj
-  // (cluster: written by the other CTAs)
-  __shared__ unsigned long long x_key[2][GC];
-  __shared__ int x_idx[2][GC];
-  __shared__ T x_row[2][GC][GJ_NB];
+  // by column parity: the CTAs' candidates, the scaled candidate rows and row
+  // jj (written by the other CTAs; kPull: this CTA's own, read by the others)
+  constexpr bool kPull = kCl && sizeof(T) == 16;
+  __shared__ ulonglong2 x_key[2][GC];  // key, row index
+  __shared__ T x_row[2][kPull ? 1 : GC][GJ_NB];
   __shared__ T x_rowjj[2][GJ_NB];
+  __shared__ T s_row[GJ_NB], s_rjj[GJ_NB];  // what warp 0 pulled, for the others
   const int G = gridDim.x, cb = blockIdx.x, tid = threadIdx.x;
   const int lane = tid & 31, wid = tid >> 5, nw = GJ_THREADS / 32;
   const int b = a.b, k0 = a.k0, rpc = a.rpc;
@@ -338,11 +342,13 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) gje_panel_ahead_kernel(GjArgs<T
   // publish row v (lane = column) of column j's round as this CTA's candidate
   auto put_cand = [&](int par, unsigned long long key, int idx, T v) {
     if constexpr (kCl) {
-      for (int q = 0; q < G; q++) dsmem_st(&x_row[par][cb][lane], (unsigned)q, v);
-      if (lane < G) {
-        dsmem_st(&x_key[par][cb], (unsigned)lane, key);
-        dsmem_st(&x_idx[par][cb], (unsigned)lane, idx);
-      }
+      if constexpr (kPull)
+        x_row[par][0][lane] = v;
+      else
+        for (int q = 0; q < G; q++) dsmem_st(&x_row[par][cb][lane], (unsigned)q, v);
+      if (lane < G)
+        dsmem_st(&x_key[par][cb], (unsigned)lane,
+                 make_ulonglong2(key, (unsigned long long)(unsigned)idx));
     } else {
       if (lane < b) a.cand[((int64_t)par * a.gstride + cb) * GJ_NB + lane] = v;
       if (lane == 0) {
@@ -353,7 +359,10 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) gje_panel_ahead_kernel(GjArgs<T
   };
   auto put_rowjj = [&](int par, T v) {
     if constexpr (kCl) {
-      for (int q = 0; q < G; q++) dsmem_st(&x_rowjj[par][lane], (unsigned)q, v);
+      if constexpr (kPull)
+        x_rowjj[par][lane] = v;
+      else
+        for (int q = 0; q < G; q++) dsmem_st(&x_rowjj[par][lane], (unsigned)q, v);
     } else {
       if (lane < b) a.swapbuf[par * GJ_NB + lane] = v;
     }
@@ -410,8 +419,9 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) gje_panel_ahead_kernel(GjArgs<T
       int idx = INT_MAX;
       if constexpr (kCl) {
         if (lane < G) {
-          key = x_key[par][lane];
-          idx = x_idx[par][lane];
+          const ulonglong2 c = x_key[par][lane];
+          key = c.x;
+          idx = (int)(unsigned)c.y;
           q = lane;
         }
       } else {
@@ -430,19 +440,38 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) gje_panel_ahead_kernel(GjArgs<T
       if (idx == INT_MAX) q = -1;
     }
     T srow, rjj = zero_<T>();
-    if (p != jj || q < 0) {
-      if constexpr (kCl) rjj = x_rowjj[par][lane];
-      else rjj = lane < b ? ld_cg(&a.swapbuf[par * GJ_NB + lane]) : zero_<T>();
-    }
-    if (q >= 0) {
-      if constexpr (kCl) srow = x_row[par][q][lane];
-      else srow = lane < b ? ld_cg(&a.cand[((int64_t)par * a.gstride + q) * GJ_NB + lane])
-                           : zero_<T>();
-    } else {  // no candidate (NaN only): row jj itself
-      T y;
-      R pr;
-      inv_split(shfl_idx_(rjj, j), y, pr);
-      srow = fma_real_(lane == j ? y : rjj * y, pr);
+    if (kPull && wid != 0) {
+      asm volatile("bar.sync 1, %0;" ::"n"(GJ_THREADS) : "memory");
+      srow = s_row[lane];
+      rjj = s_rjj[lane];
+    } else {
+      // row jj is wanted where the pivot's old row is (and by all without a
+      // candidate)
+      if constexpr (kPull) {
+        if (q < 0 || (p != jj && p >= r0 && p < r0 + nr))
+          rjj = dsmem_ld(&x_rowjj[par][lane], (unsigned)(jj / rpc));
+        if (q >= 0) srow = dsmem_ld(&x_row[par][0][lane], (unsigned)q);
+      } else if constexpr (kCl) {
+        if (q < 0 || p != jj) rjj = x_rowjj[par][lane];
+        if (q >= 0) srow = x_row[par][q][lane];
+      } else {
+        if (q < 0 || p != jj)
+          rjj = lane < b ? ld_cg(&a.swapbuf[par * GJ_NB + lane]) : zero_<T>();
+        if (q >= 0)
+          srow = lane < b ? ld_cg(&a.cand[((int64_t)par * a.gstride + q) * GJ_NB + lane])
+                          : zero_<T>();
+      }
+      if (q < 0) {  // no candidate (NaN only): row jj itself
+        T y;
+        R pr;
+        inv_split(shfl_idx_(rjj, j), y, pr);
+        srow = fma_real_(lane == j ? y : rjj * y, pr);
+      }
+      if constexpr (kPull) {
+        s_row[lane] = srow;
+        s_rjj[lane] = rjj;
+        asm volatile("bar.arrive 1, %0;" ::"n"(GJ_THREADS) : "memory");
+      }
     }
     if (cb == 0 && tid == 0) {
       a.piv[jj] = p;
@@ -512,9 +541,10 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) gje_panel_ahead_kernel(GjArgs<T
       }
     }
   }
-  // the last pushes into a CTA's shared memory came before the last column's
-  // barrier, so none is on its way when a CTA leaves
-  __syncthreads();
+  // kPull: no CTA leaves while another may still read its rows; pushes into a
+  // CTA came before the last column's barrier
+  if constexpr (kPull) cluster_sync_all();
+  else __syncthreads();
   const T* const Xl = Xs + ((b - 1) & 1) * slab;
   for (int c = wid; c < b; c += nw)
     for (int r = lane; r < nr; r += 32) Xp[r + (int64_t)c * a.ldx] = Xl[r * GJA_LD + c];
