@@ -64,3 +64,33 @@ def test_fp32_tiles_through_qr(mak, cuda, dt, shape):
         bound = 2e-5 * np.sqrt(k)
         assert np.linalg.norm(X - Qh @ Rh) <= bound * np.linalg.norm(X)
         assert np.linalg.norm(Qh.conj().T @ Qh - np.eye(k)) <= bound * np.sqrt(k)
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.complex128], ids=lambda d: np.dtype(d).name)
+@pytest.mark.parametrize("ops", ["NN", "CN", "NC", "TT"])
+@pytest.mark.parametrize("k", [16, 127, 128, 129, 255, 256, 257, 511, 512, 513])
+def test_split_operands_at_the_edges_of_one_pass(mak, cuda, dt, ops, k):
+    """The split product where its operands' maxima and digits are formed in
+    one pass (K up to 512, complex up to 256) and just beyond, ragged rows,
+    rows of zeros and rows 2^200 apart; bound: 1e-13 of sum |a||b|, the split
+    product's own."""
+    from mak_gb300 import blas
+
+    m, n = 77, 45
+    rng = np.random.default_rng(k)
+
+    def rand(r, c):
+        x = rng.standard_normal((r, c))
+        return (x + 1j * rng.standard_normal((r, c)) if dt is np.complex128 else x).astype(dt)
+
+    a, b = rand(m, k), rand(k, n)
+    a[5] = 0
+    a[7] *= 2.0 ** 100
+    a[8] *= 2.0 ** -100
+    b[:, 3] = 0
+    f = {"N": lambda x: x, "T": lambda x: x.T, "C": lambda x: x.conj().T}
+    C = blas.gemm(to_dev(np.asfortranarray(f[ops[0]](a)), cuda),
+                  to_dev(np.asfortranarray(f[ops[1]](b)), cuda), ops[0], ops[1],
+                  precision="mixed")
+    bound = 1e-13 * (np.abs(a) @ np.abs(b))
+    assert np.all(np.abs(to_host(C) - a @ b) <= bound)
