@@ -112,8 +112,12 @@ constexpr int BLK_MIN_COLS = 8;
 constexpr int BLK_MIN_MP_PER_COL = 3;  // fewer rows per column rarely pass the test
 template <class T>
 constexpr size_t block_extra_bytes() {
-  // partial Gram tiles, G / L / scaled F (one square), top block
-  return sizeof(T) * (size_t)(BLK_TILES * 16 + 2 * NBMAX * BLK_LD) + 16;
+  // partial Gram tiles, G / L / scaled F (one square), top block, a pair's raw
+  // rows by step, 1 / F_jj; four vectors of reals; the steps' failures.  All
+  // behind the slab, not static: static shared memory would take rows from the
+  // slab of every panel, and with them from the tallest matrix there is.
+  return sizeof(T) * (size_t)(BLK_TILES * 16 + 2 * NBMAX * BLK_LD + 9 * NBMAX) +
+         sizeof(real_t<T>) * 4 * NBMAX + sizeof(int) * (NBMAX + 4);
 }
 __device__ __forceinline__ void blk_tile(int t, int& bi, int& bj) {
   bj = 0;
@@ -128,18 +132,19 @@ __device__ __forceinline__ int panel_block_round(const PanelArgs<T>& a, T* Ps, i
                                  unsigned char* extra) {
   using R = real_t<T>;
   constexpr bool kCl = SYNC == SYNC_CLUSTER;
-  __shared__ R dg[NBMAX];     // squared norms of the panel's columns
-  __shared__ R rsv[NBMAX];    // 1 / |beta_j|
-  __shared__ R nrm_s[NBMAX];  // |beta_j|
-  __shared__ T raw[4][2][NBMAX];  // a pair's rows of G before they are scaled, by step
-  __shared__ R sgn_s[NBMAX];  // sign of beta_j
-  __shared__ T scl[NBMAX];    // 1 / F_jj
-  __shared__ int fail_s[NBMAX + 1];  // per step, and [NBMAX]: the norms' range
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
   const int b = blockIdx.x, G = gridDim.x, jb = a.jb;
   T* Gp = reinterpret_cast<T*>(extra);       // [36][4][4] this CTA's partial Gram
   T* Gs = Gp + BLK_TILES * 16;               // upper: G, then D and L; lower: F_jc / F_jj, transposed
   T* T0 = Gs + NBMAX * BLK_LD;               // lower: V_top; upper: F
+  T(*raw)[2][NBMAX] = reinterpret_cast<T(*)[2][NBMAX]>(T0 + NBMAX * BLK_LD);  // [4]: a pair's rows of
+                                                                 // G before they are scaled, by step
+  T* scl = &raw[4][0][0];                    // 1 / F_jj
+  R* dg = reinterpret_cast<R*>(scl + NBMAX); // squared norms of the panel's columns
+  R* rsv = dg + NBMAX;                       // 1 / |beta_j|
+  R* nrm_s = rsv + NBMAX;                    // |beta_j|
+  R* sgn_s = nrm_s + NBMAX;                  // sign of beta_j
+  int* fail_s = reinterpret_cast<int*>(sgn_s + NBMAX);  // per step, and [NBMAX]: the norms' range
   // the top block, straight from the (still unmodified) panel
   T top[NBMAX / 8];
 #pragma unroll
@@ -1569,8 +1574,8 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
     gram_bytes = scratch_for(shapes, wide ? 5 : (panel_split ? 3 : 1));
     grams = ar.take<char>(gram_bytes);
     if (panel_split || wide) {
-      Wp = ar.take<T>((size_t)NBM * NBM);
-      W2p = ar.take<T>((size_t)NBM * NBM);
+      Wp = ar.take<T>((size_t)(wide ? NBM : NBMAX) * NBM);
+      W2p = ar.take<T>((size_t)(wide ? NBM : NBMAX) * NBM);
     }
   }
   if (ar.base == nullptr) return 0;

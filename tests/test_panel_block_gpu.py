@@ -68,3 +68,25 @@ def test_block_round_and_fallback(mak, cuda, dt, kind, shape):
     if kind == "gaussian":
         Ro = O.qr_compact(A)[1]
         assert O.rel_err(Rh, Ro) <= (1e-12 if TOL[dt] < 1e-10 else 2e-5)
+
+
+# The tallest 32-column panels of a 152-SM GPU: rows per CTA that fill the
+# shared memory beside the panel kernel's static arrays.  There the block
+# round's own scratch does not fit and the column rounds take over.
+TALLEST = {"f64": 152 * 838, "c64": 152 * 388, "f32": 152 * 1742, "c32": 152 * 840}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", sorted(TALLEST))
+def test_tallest_panels_are_accepted(mak, dtype):
+    if torch.cuda.get_device_properties(0).multi_processor_count < 152:
+        pytest.skip("needs 152 SMs")
+    td = {"f64": torch.float64, "c64": torch.complex128, "f32": torch.float32,
+          "c32": torch.complex64}[dtype]
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    A = torch.randn(TALLEST[dtype], 32, dtype=td, device="cuda", generator=gen)
+    Q, R = mak.qr_compact(A)
+    eps = torch.finfo(td).eps
+    # backward error of 32 reflectors: a few eps times the column count
+    assert (Q @ R - A).norm() <= 32 * 8 * eps * A.norm()
+    assert (Q.mH @ Q - torch.eye(32, dtype=td, device="cuda")).norm() <= 32 * 8 * eps
