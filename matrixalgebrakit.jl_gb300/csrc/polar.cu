@@ -47,6 +47,7 @@ struct GjArgs {
   int* part_idx;
   T* swapbuf;  // [2][GJ_NB]: row jj by column parity
   T* cand;     // [2][gstride][GJ_NB]: each CTA's pivot candidate row, by column parity
+  T* low;       // [GJ_NB][GJ_NB]: the pivot rows' multipliers, for gje_laswp_save_kernel
   int gstride;  // allocation stride of the per-CTA partials
   unsigned* bar;
   int* status;
@@ -220,7 +221,8 @@ __global__ void __launch_bounds__(GJ_THREADS) gje_panel_kernel(GjArgs<T> a) {
 // row, scales it by its pivot's reciprocal and publishes it, while the other
 // warps eliminate column j from all rows.  So a column's chain is one search,
 // one reciprocal and one round between the CTAs, and the elimination's FP64
-// work (rows x 32 per column at 1.66 per clock per SM) runs beside it.  In a
+// work (rows x 32 per column at 1.66 per clock per SM; kDefer: the half of it to
+// the column's right) runs beside it.  In a
 // cluster (SYNC_CLUSTER) the candidates are pushed into every CTA's shared
 // memory before the cluster barrier, so that nothing is fetched after it; the
 // 16-byte type pushes keys only and one warp pulls the winner's row (remote
@@ -299,8 +301,24 @@ constexpr int GJA_LD = GJ_NB + 1;
 // Warps 1-3 and 5-7 eliminate; warp 4 shares warp 0's SM sub-partition, whose
 // FP64 pipe is left to it, and only passes row jj + 1 on.
 constexpr int GJA_MAIN = 6;
+// kDefer: a column is eliminated from the columns to its right only (lane =
+// row), the columns to its left keep their multipliers, and the row exchange's
+// kernel, which follows every panel, multiplies them by the inverse of the
+// pivot rows' unit triangle (gje_finish_rows) on all SMs that are free.  That
+// halves the FP64 work of the panel's 16 SMs.  Column c of the multipliers
+// stays in buffer c & 1, whose columns up to j nothing else uses any more.
+// From GJA_DEFER_ROWS rows per CTA on: there the halved elimination (per
+// panel, 256 rows of Float64: 137 -> 90 us) is worth more than what the
+// finishing rows add to the row exchange (6 -> 12 us).  left_polar, all in the
+// panel / deferred: Float64 n = 1600 43.8 / 44.7 ms, 1800 59.7 / 59.6, 2040
+// 65.8 / 62.0, 4096 187 / 163; ComplexF64 1100 51.7 / 54.7, 1280 76.4 / 76.0,
+// 1440 83.4 / 80.6; Float32 2100 48.1 / 48.8, 3000 96.2 / 88.5; ComplexF32
+// 1400 35.8 / 36.1, 2100 74.2 / 72.1.
+template <class T>
+constexpr int GJA_DEFER_ROWS = sizeof(real_t<T>) == 8 ? (traits<T>::cpx ? 80 : 112)
+                                                      : (traits<T>::cpx ? 104 : 128);
 // NL: rows per lane of warp 0 (32 NL rows per CTA at most)
-template <class T, int SYNC, int NL>
+template <class T, int SYNC, int NL, bool kDefer>
 __global__ void __launch_bounds__(GJ_THREADS, 1) gje_panel_ahead_kernel(GjArgs<T> a) {
   using R = real_t<T>;
   if (skipped(a.skip)) return;  // the same in every CTA: no barrier is reached
@@ -465,7 +483,7 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) gje_panel_ahead_kernel(GjArgs<T
         T y;
         R pr;
         inv_split(shfl_idx_(rjj, j), y, pr);
-        srow = fma_real_(lane == j ? y : rjj * y, pr);
+        srow = kDefer && lane < j ? rjj : fma_real_(lane == j ? y : rjj * y, pr);
       }
       if constexpr (kPull) {
         s_row[lane] = srow;
@@ -477,11 +495,16 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) gje_panel_ahead_kernel(GjArgs<T
       a.piv[jj] = p;
       if (q >= 0 && key == 0) atomicExch(a.singular, 1);
     }
+    if (kDefer && cb == 0 && wid == 4) a.low[j * GJ_NB + lane] = lane < j ? srow : zero_<T>();
     const int lp = p != jj ? p - r0 : -1;  // the pivot's old row here: row jj moves into it
     const T rjj_j = shfl_idx_(rjj, j);
-    // row r through column j (lane = column)
-    auto through = [&](int r, T x, T f) -> T {
-      return r0 + r == jj ? srow : fma_(-f, srow, lane == j ? zero_<T>() : x);
+    // row r (not row jj) through column j - 1 and through column j (lane = column)
+    auto before = [&](int r) -> T {
+      return r == lp ? rjj
+                     : Xs[(kDefer && lane < j ? lane & 1 : par ^ 1) * slab + r * GJA_LD + lane];
+    };
+    auto through = [&](T x, T f) -> T {
+      return kDefer && lane < j ? x : fma_(-f, srow, lane == j ? zero_<T>() : x);
     };
 
     if (wid == 0) {
@@ -510,18 +533,23 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) gje_panel_ahead_kernel(GjArgs<T
           for (int l = 1; l < NL; l++)
             if (r >> 5 == l) f = fv[l];
           f = shfl_idx_(f, r & 31);
-          v = through(r, r == lp ? rjj : Xo[r * GJA_LD + lane], f);
+          v = through(before(r), f);
         }
-        put_cand(par ^ 1, k2, idx, fma_real_(lane == j + 1 ? y : v * y, pr));
+        put_cand(par ^ 1, k2, idx,
+                 kDefer && lane <= j ? v : fma_real_(lane == j + 1 ? y : v * y, pr));
       }
     } else if (wid == 4) {
       const int r = jj + 1 - r0;
-      if (j + 1 < b && r >= 0 && r < nr) {
-        const bool at = r == lp;
-        put_rowjj(par ^ 1, through(r, at ? rjj : Xo[r * GJA_LD + lane],
-                                   at ? rjj_j : Xo[r * GJA_LD + j]));
+      if (j + 1 < b && r >= 0 && r < nr)
+        put_rowjj(par ^ 1, through(before(r), r == lp ? rjj_j : Xo[r * GJA_LD + j]));
+      // the multipliers of the exchanged rows: the pivot row keeps none
+      if (kDefer && lane < j) {
+        T* const M = Xs + (lane & 1) * slab + lane;
+        if (lp >= 0 && lp < nr) M[lp * GJA_LD] = rjj;
+        if (jj >= r0 && jj < r0 + nr) M[(jj - r0) * GJA_LD] = zero_<T>();
       }
-    } else {
+    } else if constexpr (!kDefer) {
+      // lane = column
       const int mi = wid < 4 ? wid - 1 : wid - 2;
       for (int rb = mi; rb < nr; rb += 4 * GJA_MAIN) {
         T x[4], f[4];
@@ -529,14 +557,39 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) gje_panel_ahead_kernel(GjArgs<T
         for (int k = 0; k < 4; k++) {
           const int r = rb + k * GJA_MAIN;
           if (r < nr) {
-            x[k] = r == lp ? rjj : Xo[r * GJA_LD + lane];
+            x[k] = before(r);
             f[k] = r == lp ? rjj_j : Xo[r * GJA_LD + j];
           }
         }
 #pragma unroll
         for (int k = 0; k < 4; k++) {
           const int r = rb + k * GJA_MAIN;
-          if (r < nr) Xn[r * GJA_LD + lane] = through(r, x[k], f[k]);
+          if (r < nr) Xn[r * GJA_LD + lane] = r0 + r == jj ? srow : through(x[k], f[k]);
+        }
+      }
+    } else {
+      // lane = row: a third of the columns and half of the rows per warp
+      constexpr int H = 2, NH = NL / H;
+      const int mi = wid < 4 ? wid - 1 : wid - 2;
+      const int rb = lane + (mi & 1) * 32 * NH;
+      T f[NH];
+#pragma unroll
+      for (int l = 0; l < NH; l++) {
+        const int r = rb + 32 * l;
+        f[l] = r < nr ? (r == lp ? rjj_j : Xo[r * GJA_LD + j]) : zero_<T>();
+      }
+      for (int c = j + mi / H; c < b; c += GJA_MAIN / H) {
+        const T sc = shfl_idx_(srow, c), rc = shfl_idx_(rjj, c);
+        T x[NH];
+#pragma unroll
+        for (int l = 0; l < NH; l++) {
+          const int r = rb + 32 * l;
+          x[l] = (c == j || r >= nr) ? zero_<T>() : r == lp ? rc : Xo[r * GJA_LD + c];
+        }
+#pragma unroll
+        for (int l = 0; l < NH; l++) {
+          const int r = rb + 32 * l;
+          if (r < nr) Xn[r * GJA_LD + c] = r0 + r == jj ? sc : fma_(-f[l], sc, x[l]);
         }
       }
     }
@@ -545,9 +598,9 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) gje_panel_ahead_kernel(GjArgs<T
   // CTA came before the last column's barrier
   if constexpr (kPull) cluster_sync_all();
   else __syncthreads();
-  const T* const Xl = Xs + ((b - 1) & 1) * slab;
   for (int c = wid; c < b; c += nw)
-    for (int r = lane; r < nr; r += 32) Xp[r + (int64_t)c * a.ldx] = Xl[r * GJA_LD + c];
+    for (int r = lane; r < nr; r += 32)
+      Xp[r + (int64_t)c * a.ldx] = Xs[((kDefer ? c : b - 1) & 1) * slab + r * GJA_LD + c];
 }
 
 // For every column outside the panel [k0, k0 + b): apply the panel's row
@@ -561,13 +614,61 @@ __global__ void __launch_bounds__(GJ_THREADS, 1) gje_panel_ahead_kernel(GjArgs<T
 // exchanges through memory (4096 rows: 140 us per call before).
 // perm, when given, is the composed row permutation of the whole
 // elimination so far, exchanged along by one extra CTA.
+//
+// low, when given: the panel holds multipliers, and the CTAs from fin0 on
+// finish its rows: row w becomes the x with x_q = w_q + sum_{k > q} x_k low[k][q].
+// A row is spread over FIN_LPR lanes (four columns each; two of the 16-byte
+// type): with 32 rows per CTA the work reaches 128 CTAs at 4096 rows.
 constexpr int LASWP_MAX_B = 128;
+template <class T> constexpr int FIN_LPR = sizeof(T) == 16 ? 16 : 8;
+template <class T> constexpr int FIN_ROWS = 256 / FIN_LPR<T>;
+template <class T>
+__device__ __forceinline__ void gje_finish_rows(int n, T* Xp, int64_t ldx, int b, const T* low,
+                                                int blk) {
+  constexpr int LPR = FIN_LPR<T>, NC = GJ_NB / LPR;
+  __shared__ T Ls[GJ_NB * GJ_NB];
+  const int tid = threadIdx.x, q = tid % LPR;
+  const int r = blk * FIN_ROWS<T> + tid / LPR;
+  T x[NC];
+#pragma unroll
+  for (int i = 0; i < NC; i++) {
+    const int c = q + LPR * i;
+    x[i] = r < n && c < b ? Xp[r + (int64_t)c * ldx] : zero_<T>();
+  }
+  for (int e = tid; e < GJ_NB * GJ_NB; e += 256) Ls[e] = e < b * GJ_NB ? low[e] : zero_<T>();
+  __syncthreads();
+#pragma unroll
+  for (int k = GJ_NB - 1; k > 0; k--) {
+    if (k < b) {
+      T u = x[k / LPR];
+      if constexpr (traits<T>::cpx) {
+        u.re = __shfl_sync(0xffffffffu, u.re, k % LPR, LPR);
+        u.im = __shfl_sync(0xffffffffu, u.im, k % LPR, LPR);
+      } else {
+        u = __shfl_sync(0xffffffffu, u, k % LPR, LPR);
+      }
+#pragma unroll
+      for (int i = 0; i < NC; i++)
+        if (LPR * i < k && q + LPR * i < k) x[i] = fma_(u, Ls[k * GJ_NB + q + LPR * i], x[i]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NC; i++) {
+    const int c = q + LPR * i;
+    if (r < n && c < b) Xp[r + (int64_t)c * ldx] = x[i];
+  }
+}
 template <class T>
 __global__ void __launch_bounds__(256) gje_laswp_save_kernel(int n, T* X, int64_t ldx, int k0,
                                                              int b, const int* piv, T* buf,
                                                              int c_lo, int c_hi, int* perm,
+                                                             const T* low, int fin0,
                                                              const int* skip) {
   if (skipped(skip)) return;
+  if (low != nullptr && (int)blockIdx.x >= fin0) {
+    gje_finish_rows<T>(n, X + (int64_t)k0 * ldx, ldx, b, low, (int)blockIdx.x - fin0);
+    return;
+  }
   __shared__ int pv[LASWP_MAX_B];
   __shared__ int pos[2 * LASWP_MAX_B], src[2 * LASWP_MAX_B];
   const int tid = threadIdx.x;
@@ -593,7 +694,7 @@ __global__ void __launch_bounds__(256) gje_laswp_save_kernel(int n, T* X, int64_
     src[e] = s;
   }
   __syncthreads();
-  if (perm != nullptr && blockIdx.x == gridDim.x - 1) {
+  if (perm != nullptr && (int)blockIdx.x == fin0 - 1) {
     // at most 2 x 128 entries: one per thread
     const int s = tid < 2 * b ? src[tid] : -1;
     const int v = s >= 0 ? perm[s] : 0;
@@ -664,9 +765,9 @@ static size_t gj_slab_cap() {
 
 // Launches the panel that runs one column ahead on G CTAs of ga.rpc rows; 1 if
 // it does not fit (shared memory, or the cluster or grid cannot be resident).
-template <class T, int SYNC, int NL>
+template <class T, int SYNC, int NL, bool kDefer>
 static int gje_ahead_launch_nl(cudaStream_t s, GjArgs<T>& ga, int G) {
-  auto kern = gje_panel_ahead_kernel<T, SYNC, NL>;
+  auto kern = gje_panel_ahead_kernel<T, SYNC, NL, kDefer>;
   const size_t smem = 2 * (size_t)ga.rpc * GJA_LD * sizeof(T);
   static PerDevice<int> pd;  // the dynamic shared memory the kernel may take (0: cannot run)
   const int cap = pd.get([&] {
@@ -732,14 +833,20 @@ static int gje_ahead_launch_nl(cudaStream_t s, GjArgs<T>& ga, int G) {
   MAK_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ga));
   return 0;
 }
+// deferred: the panel holds multipliers, whose rows gje_laswp_save_kernel finishes
 template <class T, int SYNC>
-static int gje_ahead_launch(cudaStream_t s, GjArgs<T>& ga, int G) {
+static int gje_ahead_launch(cudaStream_t s, GjArgs<T>& ga, int G, bool& deferred) {
   const int nl = (int)ceil_div(ga.rpc, 32);
-  if (nl <= 1) return gje_ahead_launch_nl<T, SYNC, 1>(s, ga, G);
-  if (nl <= 2) return gje_ahead_launch_nl<T, SYNC, 2>(s, ga, G);
-  if (nl <= 4) return gje_ahead_launch_nl<T, SYNC, 4>(s, ga, G);
-  if (nl <= 8) return gje_ahead_launch_nl<T, SYNC, 8>(s, ga, G);
-  return 1;
+  deferred = ga.rpc > GJA_DEFER_ROWS<T>;
+  if (deferred) {
+    if (nl <= 4) return gje_ahead_launch_nl<T, SYNC, 4, true>(s, ga, G);
+    if (nl <= 8) return gje_ahead_launch_nl<T, SYNC, 8, true>(s, ga, G);
+    return 1;
+  }
+  if (nl <= 1) return gje_ahead_launch_nl<T, SYNC, 1, false>(s, ga, G);
+  if (nl <= 2) return gje_ahead_launch_nl<T, SYNC, 2, false>(s, ga, G);
+  static_assert(GJA_DEFER_ROWS<T> <= 128, "the largest instance below has 4 x 32 rows");
+  return gje_ahead_launch_nl<T, SYNC, 4, false>(s, ga, G);
 }
 
 template <class T>
@@ -769,6 +876,7 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
   int* part_idx = ar.take<int>(2 * sms);
   T* swapbuf = ar.take<T>(2 * GJ_NB);
   T* cand = ar.take<T>((size_t)2 * sms * GJ_NB);
+  T* low = ar.take<T>((size_t)GJ_NB * GJ_NB);
   T* buf = ar.take<T>((size_t)NBO * (n > 0 ? n : 1));
   T* bufo = mixed ? ar.take<T>((size_t)NBO * (n > 0 ? n : 1)) : nullptr;
   unsigned* bar = ar.take<unsigned>(2);
@@ -794,16 +902,16 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
   const size_t cap = gj_slab_cap<T>();
   // one 32-wide panel (cooperative launch, at most max_ctas CTAs: on the
   // look-ahead side stream it leaves the other SMs to the main stream)
-  auto panel = [&](int64_t k0, int b, cudaStream_t s, int max_ctas) -> int {
+  auto panel = [&](int64_t k0, int b, cudaStream_t s, int max_ctas, bool& unfinished) -> int {
     GjArgs<T> ga{X, ldx, (int)n, (int)k0, b, 0, piv, part_val, part_key, part_idx, swapbuf,
-                 cand, sms, bar, &info->status, &info->singular, skip_flag()};
+                 cand, low, sms, bar, &info->status, &info->singular, skip_flag()};
     // The panel that runs one column ahead: one cluster of up to 16 CTAs (at
     // least 32 rows each) up to the size where a column's elimination on 16 SMs
-    // (rows per CTA x 32, complex four times that) takes longer than a grid's
+    // (rows per CTA x 32, complex four times that, half of it deferred) takes longer than a grid's
     // round between its CTAs, about 4.5 us per column; beyond, a cooperative
     // grid while a CTA's rows fit shared memory twice.  Per panel, cluster /
     // grid: Float64 n = 3000 105 / 146 us, 4096 137 / 163 us (both beside the
-    // look-ahead's product); ComplexF64 n = 2048 204 / 184 us.
+    // look-ahead's product); ComplexF64 n = 2048 204 / 184 us (all before the deferral).
     const int64_t cluster_max = traits<T>::cpx && sizeof(real_t<T>) == 8 ? 1536 : 4096;
     if (n <= cluster_max) {
       int64_t G = ceil_div(n, 32);
@@ -811,7 +919,7 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
       const int64_t rpc = ceil_div(n, G);
       G = ceil_div(n, rpc);
       ga.rpc = (int)rpc;
-      const int rc = gje_ahead_launch<T, SYNC_CLUSTER>(s, ga, (int)G);
+      const int rc = gje_ahead_launch<T, SYNC_CLUSTER>(s, ga, (int)G, unfinished);
       if (rc != 1) return rc;
     }
     {
@@ -820,9 +928,10 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
       const int64_t rpc = ceil_div(n, G);
       G = ceil_div(n, rpc);
       ga.rpc = (int)rpc;
-      const int rc = gje_ahead_launch<T, SYNC_GRID>(s, ga, (int)G);
+      const int rc = gje_ahead_launch<T, SYNC_GRID>(s, ga, (int)G, unfinished);
       if (rc != 1) return rc;
     }
+    unfinished = false;
     // grid: rows per CTA >= 64, at most one CTA per SM, slab within shared memory
     int64_t G = ceil_div(n, 64);
     if (G > max_ctas) G = max_ctas;
@@ -854,10 +963,14 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
     const int64_t c_lo = K0, c_hi = K0 + KB;
     for (int64_t k0 = K0; k0 < K0 + KB; k0 += GJ_NB) {
       const int b = (int)((K0 + KB - k0) < GJ_NB ? (K0 + KB - k0) : GJ_NB);
-      MAK_TRY(panel(k0, b, s, max_ctas));
+      bool unfinished = false;  // the panel holds multipliers
+      MAK_TRY(panel(k0, b, s, max_ctas, unfinished));
       note_launch();
-      gje_laswp_save_kernel<T><<<(unsigned)ceil_div(c_hi - c_lo, 8) + 1, 256, 0, s>>>(
-          (int)n, X, ldx, (int)k0, b, piv, buf, (int)c_lo, (int)c_hi, perm, skip_flag());
+      const int fin0 = (int)ceil_div(c_hi - c_lo, 8) + 1;
+      const unsigned fin = unfinished ? (unsigned)ceil_div(n, FIN_ROWS<T>) : 0u;
+      gje_laswp_save_kernel<T><<<(unsigned)fin0 + fin, 256, 0, s>>>(
+          (int)n, X, ldx, (int)k0, b, piv, buf, (int)c_lo, (int)c_hi, perm,
+          unfinished ? low : nullptr, fin0, skip_flag());
       MAK_CUDA_TRY(cudaGetLastError());
       const T* F = X + k0 * ldx;
       if (k0 > c_lo)
@@ -876,7 +989,8 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
     if (c_hi <= c_lo) return 0;
     note_launch();
     gje_laswp_save_kernel<T><<<(unsigned)ceil_div(c_hi - c_lo, 8), 256, 0, s>>>(
-        (int)n, X, ldx, (int)K0, (int)KB, piv, bufo, (int)c_lo, (int)c_hi, nullptr, skip_flag());
+        (int)n, X, ldx, (int)K0, (int)KB, piv, bufo, (int)c_lo, (int)c_hi, nullptr, nullptr,
+        0, skip_flag());
     MAK_CUDA_TRY(cudaGetLastError());
     const T* Fb = X + K0 * ldx;
     const int64_t l1 = c_hi < K0 ? c_hi : K0;  // left part [c_lo, l1)

@@ -61,3 +61,19 @@ def test_tied_candidates(mak, cuda):
     W, P = mak.left_polar(A)
     assert float((W - A / 16).abs().max()) <= 1e-13
     assert float((P - 16 * torch.eye(256, device=cuda, dtype=A.dtype)).abs().max()) <= 1e-11
+
+
+# Rows per CTA (16 CTAs) on both sides of the line from which a panel keeps
+# multipliers that the row exchange's kernel finishes, ragged last panels, and
+# the largest instance; matrices whose pivots move in every column.
+@pytest.mark.parametrize("dt,n", [(torch.float64, 1792), (torch.float64, 1793), (torch.float64, 2049),
+                                  (torch.complex128, 1280), (torch.complex128, 1281),
+                                  (torch.complex128, 2500), (torch.float32, 2048),
+                                  (torch.float32, 2055), (torch.complex64, 1664),
+                                  (torch.complex64, 1665)])
+def test_deferred_multipliers(mak, cuda, dt, n):
+    gen = torch.Generator(device=cuda).manual_seed(n)
+    Q, _ = mak.qr_compact(torch.randn((n, n), generator=gen, device=cuda, dtype=dt))
+    Z, _ = mak.qr_compact(torch.randn((n, n), generator=gen, device=cuda, dtype=dt))
+    d = torch.linspace(1, 100, n, device=cuda, dtype=torch.float64).to(dt)
+    check(mak, Q @ (d[:, None] * Z.mH), BOUND[dt] * (1 if Q.real.dtype == torch.float64 else 5))
