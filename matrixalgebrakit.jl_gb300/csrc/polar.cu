@@ -841,6 +841,8 @@ static int gje_ahead_launch(cudaStream_t s, GjArgs<T>& ga, int G, bool& deferred
   if (deferred) {
     if (nl <= 4) return gje_ahead_launch_nl<T, SYNC, 4, true>(s, ga, G);
     if (nl <= 8) return gje_ahead_launch_nl<T, SYNC, 8, true>(s, ga, G);
+    if constexpr (SYNC == SYNC_CLUSTER && sizeof(real_t<T>) == 4)
+      if (nl <= 16) return gje_ahead_launch_nl<T, SYNC, 16, true>(s, ga, G);
     return 1;
   }
   if (nl <= 1) return gje_ahead_launch_nl<T, SYNC, 1, false>(s, ga, G);
@@ -907,12 +909,14 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
                  cand, low, sms, bar, &info->status, &info->singular, skip_flag()};
     // The panel that runs one column ahead: one cluster of up to 16 CTAs (at
     // least 32 rows each) up to the size where a column's elimination on 16 SMs
-    // (rows per CTA x 32, complex four times that, half of it deferred) takes longer than a grid's
-    // round between its CTAs, about 4.5 us per column; beyond, a cooperative
-    // grid while a CTA's rows fit shared memory twice.  Per panel, cluster /
-    // grid: Float64 n = 3000 105 / 146 us, 4096 137 / 163 us (both beside the
-    // look-ahead's product); ComplexF64 n = 2048 204 / 184 us (all before the deferral).
-    const int64_t cluster_max = traits<T>::cpx && sizeof(real_t<T>) == 8 ? 1536 : 4096;
+    // (half of rows per CTA x 32, complex four times that) takes longer than a
+    // grid's round between its CTAs, about 4.5 us per column; beyond, a
+    // cooperative grid while a CTA's rows fit shared memory twice.  left_polar
+    // (mixed), cluster / grid: Float64 n = 4200 116.8 / 115.4 ms, 6000 229.0 /
+    // 227.7; ComplexF64 2048 60.4 / 64.3, 2500 104.7 / 93.5; Float32 4200 73.9 /
+    // 110.8, 8000 298 / 372; ComplexF32 4200 148 / 177, 6000 333 / 379.
+    const int64_t cluster_max =
+        sizeof(real_t<T>) == 4 ? 8192 : traits<T>::cpx ? 2048 : 4096;
     if (n <= cluster_max) {
       int64_t G = ceil_div(n, 32);
       if (G > kGjClusterWide) G = kGjClusterWide;

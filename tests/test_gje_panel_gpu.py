@@ -77,3 +77,16 @@ def test_deferred_multipliers(mak, cuda, dt, n):
     Z, _ = mak.qr_compact(torch.randn((n, n), generator=gen, device=cuda, dtype=dt))
     d = torch.linspace(1, 100, n, device=cuda, dtype=torch.float64).to(dt)
     check(mak, Q @ (d[:, None] * Z.mH), BOUND[dt] * (1 if Q.real.dtype == torch.float64 else 5))
+
+
+# The largest clusters of the other types and the first grid beyond them
+# (ComplexF32 stops where 16 CTAs' rows no longer fit shared memory twice);
+# W^H W = I and A = W P to n eps.
+@pytest.mark.parametrize("dt,n", [(torch.float32, 4097), (torch.float32, 8192), (torch.float32, 8193),
+                                  (torch.complex64, 4100), (torch.complex64, 7100),
+                                  (torch.complex128, 2048), (torch.complex128, 2049)])
+def test_largest_clusters_by_type(mak, cuda, dt, n):
+    gen = torch.Generator(device=cuda).manual_seed(n)
+    A = torch.randn((n, n), generator=gen, device=cuda, dtype=dt)
+    A = A / np.sqrt(n) + 4 * torch.roll(torch.eye(n, device=cuda, dtype=dt), 1, 0)
+    check(mak, A.t().contiguous().t(), n * torch.finfo(dt).eps, precision="mixed")
