@@ -159,15 +159,17 @@ __global__ void sign_update_kernel(int64_t nn, T* A, const T* Ai, T* Cm, const T
 // Newton-Schulz form of the sign step (mixed precision): B <- 3 I - B, and the
 // update A <- An, C <- Cn with *dpart = partial |An - A|^2
 template <class T>
-__global__ void sign_ns_prepare_kernel(int64_t n, T* B) {
+__global__ void sign_ns_prepare_kernel(int64_t n, T* B, const int* skip) {
+  if (skipped(skip)) return;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n * n;
        e += (int64_t)gridDim.x * blockDim.x)
     B[e] = (e % n == e / n ? make_scalar<T>(real_t<T>(3), 0) : zero_<T>()) - B[e];
 }
 template <class T>
 __global__ void sign_ns_update_kernel(int64_t nn, T* A, const T* An, T* Cm, const T* Cn,
-                                      real_t<T>* dpart) {
+                                      real_t<T>* dpart, const int* skip) {
   using Rr = real_t<T>;
+  if (skipped(skip)) return;
   __shared__ Rr sh[32];
   Rr acc = Rr(0);
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nn;
@@ -183,12 +185,19 @@ __global__ void sign_ns_update_kernel(int64_t nn, T* A, const T* An, T* Cm, cons
 
 // Device stop of the sign iteration without host synchronization: w[0] is
 // the stop flag the later iterations' kernels read on entry, w[1] counts the
-// iterations taken (NaN stops, as the host-checked loop does).
+// iterations taken (NaN stops, as the host-checked loop does).  With ns_ok,
+// w[2] is set once the Newton-Schulz form takes over; w[3] and w[4] are what
+// the kernels of a Newton and of a Newton-Schulz step read.
+constexpr double SIGN_NS_SWITCH = 0.25;
 template <class R>
-__global__ void sign_stop_kernel(const R* dnorm2, R tol, int* w) {
+__global__ void sign_stop_kernel(const R* dnorm2, R tol, bool ns_ok, int* w) {
   if (w[0]) return;
   w[1] += 1;
-  if (!(sqrt(*dnorm2) > tol)) w[0] = 1;
+  const R d = sqrt(*dnorm2);
+  if (!(d > tol)) w[0] = 1;
+  else if (ns_ok && d <= R(SIGN_NS_SWITCH)) w[2] = 1;
+  w[3] = w[0] | w[2];
+  w[4] = w[0] | !w[2];
 }
 __global__ void info_sign_fixed_kernel(mak_info* info, const int* w) {
   info->iterations = w[1];
@@ -401,7 +410,7 @@ struct SylScratch {
   real_t<T>* scal;
   T *Mm, *Ak, *Ck, *Ai, *Tm, *Y, *Pinv;
   int* iperm;
-  int* stopw;  // device stop of the sign iteration: [0] stop flag, [1] iterations
+  int* stopw;  // [5], device stop of the sign iteration (sign_stop_kernel)
   char* tail;
   size_t tail_bytes;
 };
@@ -419,7 +428,7 @@ static SylScratch<T> syl_take(Arena& ar, cudaStream_t st, int64_t m, int64_t n, 
   s.Tm = ar.take<T>(nn + 1);
   s.Y = ar.take<T>((size_t)m * n + 1);
   s.iperm = ar.take<int>(n + 1);
-  s.stopw = ar.take<int>(2);
+  s.stopw = ar.take<int>(5);
   size_t gj_ws = 0, oz_ws = 0;
   {
     Arena meas(nullptr, 0);
@@ -486,20 +495,24 @@ static int syl_solve(cudaStream_t st, int64_t n, const T* P, int64_t ldp, int ma
   MAK_TRY(copy_mat<T>(st, n, n, P, ldp, s.Ak, n));
   const Rr tol = (sizeof(Rr) == 8 ? Rr(1e-13) : Rr(1e-6)) * sqrt((Rr)n);
   int it = 0;
-  // In mixed precision the host-checked loop finishes with Newton-Schulz steps
-  // on the split products once a Newton step moved A by at most 1/4 (A's
-  // eigenvalues are then within about a tenth of 1): X <- X (3 I - X^2) / 2
-  // for X = [[A, C], [0, -A]], i.e. B = 3 I - A^2, A <- A B / 2 and
-  // C <- (C B - A (A C - C A)) / 2, where C A = -(A C)^H since A is Hermitian
-  // and C anti-Hermitian.  Five products instead of a pivoted inverse and two
-  // (n = 512 ComplexF64: 0.6 against 2.6 ms a step), converging quadratically
-  // too.
-  const bool ns_ok = !fixed && precision == MAK_PREC_MIXED && sizeof(Rr) == 8;
+  // In mixed precision the iteration finishes with Newton-Schulz steps on the
+  // split products once a Newton step moved A by at most 1/4 (A's eigenvalues
+  // are then within about a tenth of 1): X <- X (3 I - X^2) / 2 for X = [[A, C],
+  // [0, -A]], i.e. B = 3 I - A^2, A <- A B / 2 and C <- (C B - A (A C - C A)) / 2,
+  // where C A = -(A C)^H since A is Hermitian and C anti-Hermitian.  Five
+  // products instead of a pivoted inverse and two (n = 512 ComplexF64: 0.6
+  // against 2.6 ms a step), converging quadratically too.  The form without
+  // host synchronization launches both kinds of step in every iteration and
+  // skips one by device flags, so that it takes the same steps; its blocks
+  // below SIGN_NS_MIN_N (where a step is bound by its launches) would pay for
+  // the second kind of launches, so neither form switches there.
+  constexpr int64_t SIGN_NS_MIN_N = 384;
+  const bool ns_ok = precision == MAK_PREC_MIXED && sizeof(Rr) == 8 && n >= SIGN_NS_MIN_N;
   const unsigned gr = g1 < RED_CTAS ? g1 : RED_CTAS;
   auto ns_step = [&]() -> int {
     MAK_TRY(G(n, n, n, one_<T>(), opnd<T>(s.Ak, n), opnd<T>(s.Ak, n), zero_<T>(), s.Y, n));
     note_launch();
-    sign_ns_prepare_kernel<T><<<gr, 256, 0, st>>>(n, s.Y);
+    sign_ns_prepare_kernel<T><<<gr, 256, 0, st>>>(n, s.Y, skip_flag());
     MAK_CUDA_TRY(cudaGetLastError());
     MAK_TRY(G(n, n, n, one_<T>(), opnd<T>(s.Ak, n), opnd<T>(s.Ck, n), zero_<T>(), s.Tm, n));
     dim3 g((unsigned)ceil_div(n, 32), (unsigned)ceil_div(n, 32));
@@ -511,16 +524,19 @@ static int syl_solve(cudaStream_t st, int64_t n, const T* P, int64_t ldp, int ma
     MAK_TRY(G(n, n, n, -half, opnd<T>(s.Ak, n), opnd<T>(s.Ai, n), one_<T>(), s.Tm, n));
     MAK_TRY(G(n, n, n, half, opnd<T>(s.Ak, n), opnd<T>(s.Y, n), zero_<T>(), s.Mm, n));
     note_launch();
-    sign_ns_update_kernel<T><<<gr, 256, 0, st>>>((int64_t)nn, s.Ak, s.Mm, s.Ck, s.Tm, red);
+    sign_ns_update_kernel<T><<<gr, 256, 0, st>>>((int64_t)nn, s.Ak, s.Mm, s.Ck, s.Tm, red,
+                                                  skip_flag());
     return cudaGetLastError() == cudaSuccess ? 0 : MAK_ERR_CUDA;
   };
   bool in_ns = false;
-  if (fixed) MAK_CUDA_TRY(cudaMemsetAsync(s.stopw, 0, 2 * sizeof(int), st));
+  if (fixed) {
+    MAK_CUDA_TRY(cudaMemsetAsync(s.stopw, 0, 4 * sizeof(int), st));
+    MAK_CUDA_TRY(cudaMemsetAsync(s.stopw + 4, 1, sizeof(int), st));  // nonzero: not Newton-Schulz yet
+  }
   for (it = 1; it <= maxiter; it++) {
     SkipScope skip(fixed ? s.stopw : skip_flag());
-    if (in_ns) {
-      MAK_TRY(ns_step());
-    } else {
+    if (!in_ns) {
+      SkipScope newton(fixed && ns_ok ? s.stopw + 3 : skip_flag());
       MAK_TRY(inverse(s.Ak, s.Ai));
       if (it == 1) MAK_TRY(copy_mat<T>(st, n, n, s.Ai, n, s.Pinv, n));
       MAK_TRY(reduce_mat<T>(st, n, n, s.Ak, n, 0, red, nrm2));
@@ -533,13 +549,17 @@ static int syl_solve(cudaStream_t st, int64_t n, const T* P, int64_t ldp, int ma
                                                  skip_flag());
       MAK_CUDA_TRY(cudaGetLastError());
     }
+    if (in_ns || (fixed && ns_ok && it > 1)) {
+      SkipScope schulz(fixed ? s.stopw + 4 : skip_flag());
+      MAK_TRY(ns_step());
+    }
     note_launch();
     reduce_final_kernel<Rr><<<1, 256, 0, st>>>((int)gr, red, 0, nrm2 + 2);
     MAK_CUDA_TRY(cudaGetLastError());
     MAK_TRY(herm_project<T>(st, n, s.Ak, n));  // idempotent once A is Hermitian
     if (fixed) {
       note_launch();
-      sign_stop_kernel<Rr><<<1, 1, 0, st>>>(nrm2 + 2, tol, s.stopw);
+      sign_stop_kernel<Rr><<<1, 1, 0, st>>>(nrm2 + 2, tol, ns_ok, s.stopw);
       MAK_CUDA_TRY(cudaGetLastError());
       continue;
     }
@@ -547,7 +567,7 @@ static int syl_solve(cudaStream_t st, int64_t n, const T* P, int64_t ldp, int ma
     MAK_CUDA_TRY(cudaMemcpyAsync(&dnorm2, nrm2 + 2, sizeof(Rr), cudaMemcpyDeviceToHost, st));
     MAK_CUDA_TRY(cudaStreamSynchronize(st));
     if (!(sqrt(dnorm2) > tol)) break;
-    if (ns_ok && sqrt(dnorm2) <= Rr(0.25)) in_ns = true;
+    if (ns_ok && sqrt(dnorm2) <= Rr(SIGN_NS_SWITCH)) in_ns = true;
   }
   if (it > maxiter) it = maxiter;
   *iters = fixed ? -1 : it;
