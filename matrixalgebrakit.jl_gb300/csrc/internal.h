@@ -64,9 +64,11 @@ enum TuneId {
   TUNE_QR_OUTER64_MAX_N,     // mixed QR: 64-wide outer blocks up to this n
   TUNE_LOOKAHEAD_CTAS,       // SMs of the look-ahead side stream
   TUNE_PANEL_HIER_C,         // tall panels: cooperative grid of clusters of this size (0: off)
-  TUNE_PANEL_PAIR,           // QR panels: two columns per barrier round (1) or one (0)
+  TUNE_PANEL_PAIR,           // QR panels: all columns in one round where conditioning allows, else
+                             // two per barrier round (1); one column per round throughout (0)
   TUNE_OZ_MERGED,            // split GEMM: one MMA per A plane over up to 4 B planes (1)
-  TUNE_OZ_NARROW,            // split GEMM, K <= 128: 32-wide tiles, two accumulator sets (1)
+  TUNE_OZ_NARROW,            // split GEMM: 32-wide tiles with two accumulator sets for one chunk of K
+                             // or half-empty grids (1)
   TUNE_LOOKAHEAD_TAIL_COLS,  // far columns from which down the side stream gets more SMs
   TUNE_LOOKAHEAD_TAIL_CTAS,  // the side stream's SMs in that tail
   TUNE_SMALL_QR_BYTES,       // batched QR: blocks up to this many bytes take the one-CTA kernel

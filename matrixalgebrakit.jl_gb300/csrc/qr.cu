@@ -10,7 +10,7 @@
 //
 // Structure on the device, per panel of jb <= 32 columns starting at j0:
 //  1. qr_panel_kernel: ONE launch factors the (m-j0) x jb panel: a
-//     thread-block cluster of up to 8 CTAs for panels of up to 8 x 256 rows
+//     thread-block cluster of up to 16 CTAs for panels of up to 8 x 256 rows
 //     (hardware cluster barrier; clusters of different streams run side by
 //     side, which the batched driver relies on), a cooperative grid of up to
 //     one CTA per SM beyond that (bounded global barrier).
