@@ -90,14 +90,18 @@ struct PanelArgs {
 // V_bot = A_bot F^-1, and the T factor from A = (I - V T V^H) [R; 0]:
 // T = -F R^-1 V_top^-H.
 //
-// The Gram entries carry an error of eps |a_j| |a_c|, so the round is taken
-// only if every column keeps at least half its squared norm after the
-// columns before it are projected out (the pair rounds' test over the whole
-// panel; then cond(R) is small and the factors are as accurate as the column
-// by column ones), and if every squared norm is finite and far from overflow
-// and underflow.  Every CTA repeats the jb x jb work on identical numbers, so
-// all of them take the same branch; nothing has been written when the test
-// fails, and the panel is factored column by column as before.
+// The Gram entries carry an error of eps |a_j| |a_c|, which R's inverse
+// amplifies: with R' the factor of the panel with columns of norm one, Q^H Q
+// - I is of the order of eps ||R'^-1||^2.  Every pivot well above zero does
+// not bound that (32 columns that each keep half their squared norm can reach
+// cond(R') = 10^4), so the round is taken only if every column keeps at least
+// half its squared norm after the columns before it are projected out (the
+// factorization of G is then safe to finish) and ||R'^-1||_F^2, formed from
+// the finished factor, is at most BLK_INV_LIMIT per column; and if every
+// squared norm is finite and far from overflow and underflow.  Every CTA
+// repeats the jb x jb work on identical numbers, so all of them take the same
+// branch; nothing has been written when a test fails, and the panel is
+// factored column by column as before.
 //
 // Bound: FP64 throughput (about 1.6 DFMA per clock per SM): rows x jb^2 / 2
 // multiply-adds for G and as many for V_bot, spread over the CTAs, plus the
@@ -110,19 +114,89 @@ constexpr int BLK_ROWGRP = 7;   // row groups: 36 x 7 = 252 of the 256 threads
 constexpr int BLK_LD = NBMAX + 1;
 constexpr int BLK_MIN_COLS = 8;
 constexpr int BLK_MIN_MP_PER_COL = 3;  // fewer rows per column rarely pass the test
+// ||R'^-1||_F^2 per column: the mean over the columns of their squared norm
+// over their squared distance from the span of the others; about mp / (mp -
+// jb) for Gaussian columns, 1.5 for three rows per column (96 x 32: 1.4 - 1.6).
+// ||Q^H Q - I||_2 of accepted 32-column panels over that of the column rounds,
+// 96 to 9000 rows, Float64 (Float32): 1.0 - 1.1 0.7 - 1.5 (1.7), 1.3 1.2 - 1.8
+// (3.9), 1.6 0.7 - 2.5 (4.1), 2.0 1.0 - 1.5 (2.1), 2.7 2 - 6.5 (8), 4.4 4 - 8
+// (6), 28 30 - 180 (70).  Columns correlated by 0.6 with the next one (2.1 -
+// 2.4) are refused: 1000 x 501 Float64 2.63 ms accepted, 5.55 refused, 7.4 by
+// column rounds on 8 CTAs without the round.
+constexpr float BLK_INV_LIMIT = 2.0f;
 template <class T>
 constexpr size_t block_extra_bytes() {
   // partial Gram tiles, G / L / scaled F (one square), top block, a pair's raw
-  // rows by step, 1 / F_jj; four vectors of reals; the steps' failures.  All
+  // rows by step, 1 / F_jj; four vectors of reals; the steps' failures and the
+  // four warps' parts of ||R'^-1||_F^2.  All
   // behind the slab, not static: static shared memory would take rows from the
   // slab of every panel, and with them from the tallest matrix there is.
   return sizeof(T) * (size_t)(BLK_TILES * 16 + 2 * NBMAX * BLK_LD + 9 * NBMAX) +
-         sizeof(real_t<T>) * 4 * NBMAX + sizeof(int) * (NBMAX + 4);
+         sizeof(real_t<T>) * 4 * NBMAX + sizeof(int) * (NBMAX + 8);
 }
 __device__ __forceinline__ void blk_tile(int t, int& bi, int& bj) {
   bj = 0;
   while ((bj + 1) * (bj + 2) / 2 <= t) bj++;
   bi = t - bj * (bj + 1) / 2;
+}
+
+// x 2^e as a float, for results below 2^127 (e.g. ratios of the panel's column
+// norms taken out of an entry of its factor); integer operations only, so that
+// the FP64 pipe is left to the recurrence that runs beside it
+__device__ __forceinline__ float narrow_exp(double x, int e) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const int ex = (int)((hi >> 20) & 0x7FFu) - 1023 + 127 + e;
+  if (ex <= 0) return 0.0f;
+  return __uint_as_float((hi & 0x80000000u) | (unsigned)(ex < 254 ? ex : 254) << 23 |
+                         (hi & 0xFFFFFu) << 3 | lo >> 29);
+}
+__device__ __forceinline__ float narrow_exp(float x, int e) { return x * pow2_(0.0f, e); }
+template <class R> __device__ __forceinline__ cplx<float> narrow_exp(cplx<R> x, int e) {
+  return {narrow_exp(x.re, e), narrow_exp(x.im, e)};
+}
+__device__ __forceinline__ float sq_(float x) { return x * x; }
+__device__ __forceinline__ float sq_(cplx<float> x) { return fmaf(x.re, x.re, x.im * x.im); }
+
+// Warp w4's part of ||R'^-1||_F^2 (lane = row): R' = D'^1/2 U with U_ik = L_ik
+// |a_i| / |a_k| unit upper triangular and D'_c = D_c / |a_c|^2, so the columns
+// c = w4, w4 + 4, ... of U^-1 by substitution, each divided by D'_c.  In FP32,
+// which is enough: a norm below the limit is that of a matrix within 32
+// 2^-23 |U| of U, and those of the panels refused need no digits.  Beside the
+// elimination's last steps it costs 0.5 us per panel (Float32 1.3); after them
+// 4 us (Float32 2).
+template <class T>
+__device__ __forceinline__ float panel_inverse_norm2(const T* Gs, const real_t<T>* dg, int jb,
+                                                     int w4) {
+  using F = typename std::conditional<traits<T>::cpx, cplx<float>, float>::type;
+  const int lane = threadIdx.x & 31;
+  const int ic = min(lane, jb - 1);
+  const int E = exp2_of(dg[ic]) >> 1;               // |a_i| = 2^E times [1, 2)
+  const float m = narrow_exp(dg[ic], -2 * E);
+  const float rs = rsqrtf(m), s = m * rs;
+  const float w = __fdividef(m, narrow_exp(re_(Gs[ic * BLK_LD + ic]), -2 * E));  // 1 / D'
+  F x[NBMAX / 4];
+#pragma unroll
+  for (int q = 0; q < NBMAX / 4; q++) x[q] = lane == w4 + 4 * q ? one_<F>() : zero_<F>();
+  // a small body, not unrolled: the code runs once per panel, and fetching it
+  // costs more than its arithmetic; the next row is read ahead of the chain
+  T g = lane < jb - 1 ? Gs[lane * BLK_LD + jb - 1] : zero_<T>();
+#pragma unroll 1
+  for (int k = jb - 1; k > 0; k--) {
+    const int Ek = __shfl_sync(0xffffffffu, E, k);
+    const float sk = s * __shfl_sync(0xffffffffu, rs, k);
+    const F u = lane < k ? narrow_exp(g, E - Ek) * sk : zero_<F>();
+    g = lane < k - 1 ? Gs[lane * BLK_LD + k - 1] : zero_<T>();
+#pragma unroll
+    for (int q = 0; q < NBMAX / 4; q++) x[q] = fma_(-u, shfl_idx_(x[q], k), x[q]);
+  }
+  float sum = 0.0f;
+#pragma unroll
+  for (int q = 0; q < NBMAX / 4; q++) {
+    const int c = w4 + 4 * q;
+    const float wc = __shfl_sync(0xffffffffu, w, c);
+    if (c < jb) sum = fmaf(sq_(x[q]), wc, sum);
+  }
+  return warp_sum(sum);
 }
 
 // 1: the panel is factored and stored; 0: not taken (nothing written);
@@ -145,6 +219,7 @@ __device__ __forceinline__ int panel_block_round(const PanelArgs<T>& a, T* Ps, i
   R* nrm_s = rsv + NBMAX;                    // |beta_j|
   R* sgn_s = nrm_s + NBMAX;                  // sign of beta_j
   int* fail_s = reinterpret_cast<int*>(sgn_s + NBMAX);  // per step, and [NBMAX]: the norms' range
+  float* inv2_s = reinterpret_cast<float*>(fail_s + NBMAX + 1);  // [4] parts of ||R'^-1||_F^2
   // the top block, straight from the (still unmodified) panel
   T top[NBMAX / 8];
 #pragma unroll
@@ -363,7 +438,19 @@ __device__ __forceinline__ int panel_block_round(const PanelArgs<T>& a, T* Ps, i
           }
         }
       }
-      __syncthreads();
+      // L and D are complete: while the elimination takes its last two steps,
+      // warps 0-3 look at the whole factor
+      if (it >= np) {
+        if (chol) {
+          asm volatile("bar.arrive 2, %0;" ::"n"(PANEL_THREADS) : "memory");  // the last |beta_j|
+          const float v = panel_inverse_norm2<T>(Gs, dg, jb, w4);
+          if (lane == 0) inv2_s[w4] = v;
+          break;
+        }
+        if (it == np) asm volatile("bar.sync 2, %0;" ::"n"(PANEL_THREADS) : "memory");
+      } else {
+        __syncthreads();
+      }
       // this step's flag (written by its owner before the barrier; one word
       // per step, so that a later step's owner cannot race a slow reader)
       if (it < np && fail_s[it]) {
@@ -409,6 +496,7 @@ __device__ __forceinline__ int panel_block_round(const PanelArgs<T>& a, T* Ps, i
   if constexpr (kCl) cluster_wait();
   if (failed) return 0;
   __syncthreads();
+  if (!((inv2_s[0] + inv2_s[1]) + (inv2_s[2] + inv2_s[3]) <= BLK_INV_LIMIT * jb)) return 0;
   // V_top's entries, scaled
   for (int c = wid; c < jb; c += nw)
     if (lane > c && lane < jb) T0[lane * BLK_LD + c] = T0[lane * BLK_LD + c] * scl[c];
