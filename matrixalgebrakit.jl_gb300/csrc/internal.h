@@ -29,6 +29,10 @@ template <class T>
 int tri_inverse(cudaStream_t st, int64_t n, const T* R, int64_t ldr, T* X, int precision,
                 Arena& ar, mak_info* info);
 
+// whether tri_inverse of this size runs by substitution (else gje_inverse)
+template <class T>
+bool tri_substitution(int64_t n, int precision);
+
 int info_reset(cudaStream_t st, mak_info* info);
 
 // qr_pullback! (dA += ...); known_p >= 0 skips the host read of the rank

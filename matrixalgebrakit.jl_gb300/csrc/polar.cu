@@ -1053,154 +1053,142 @@ int gje_inverse(cudaStream_t st, int64_t n, T* X, int64_t ldx, int* iperm, int p
 }
 
 // ---- inverse of a triangular matrix --------------------------------------------
-// By doubling: the 32 x 32 diagonal blocks first (all at once), then, for s =
-// 32, 64, ..., every pair of neighbouring s-wide inverses gives the corner
-// X_ab = -X_aa R_ab X_bb of the next.  Two launches per level (a split product
-// each from s = 256 in mixed precision), log2(n / 32) levels and n^3 / 3
-// multiply-adds, against n / 32 pivoted panels in sequence (n = 512
-// ComplexF64 2.5 ms).
+// Back substitution on R X = I by row blocks of 32 from the last one up: the
+// block's rows are solved for (tri_solve_kernel) and their product with the
+// columns of R above them subtracted from the rows above, two launches per
+// block and n^3 / 3 multiply-adds, against a pivoted panel, an exchange and
+// updates of all n columns per block in gje_inverse.
+//
+// Substitution because its residual R X - I is bounded by n eps |R| |X| entry
+// by entry whatever R's condition.  Doubling (X_ab = -X_aa R_ab X_bb on ever
+// larger blocks, log2(n / 32) levels) multiplies by the inverses of whole
+// blocks, whose size R X no longer shows: on the factor of 100 smooth columns
+// of condition 3e6 it is wrong by 1e-7 where this is by 5e-12, on 260 of them
+// in every digit.  FP64 products in either precision: rows and columns that
+// meet are graded against each other when R is, and a split product is
+// accurate to the product of their maxima only.
 constexpr int TRI_NB = 32;
 constexpr int TRI_WARPS = 4;
+// FP64 work grows with n^3 and the elimination's split products hardly, so in
+// mixed precision the elimination takes over where it is the faster.  QR
+// pullback by substitution / by elimination: Float64 n = 520 0.69 / 1.83 ms,
+// 2000 6.6 / 10.7, 2800 15.0 / 19.5, 4000 38.3 / 37.7; ComplexF64 520 1.38 /
+// 3.06, 2000 21.9 / 26.4, 2800 53.2 / 51.3.
 template <class T>
-__global__ void __launch_bounds__(32 * TRI_WARPS) tri_diag_kernel(int n, const T* R, int64_t ldr,
-                                                                  T* X, int* singular,
-                                                                  const int* skip) {
+constexpr int64_t TRI_SOLVE_MAX_N = traits<T>::cpx ? 2432 : 3584;
+
+// X <- I
+template <class T>
+__global__ void __launch_bounds__(256) tri_eye_kernel(int n, T* X, const int* skip) {
+  if (skipped(skip)) return;
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  for (int j = blockIdx.y; j < n; j += gridDim.y)
+    if (i < n) X[i + (int64_t)j * n] = i == j ? one_<T>() : zero_<T>();
+}
+// Rows i0 .. i0 + 31 of X from their right-hand sides in place, the columns
+// from i0 on: a warp per column, lane = row, x_l = b_l / R_ll and b_i -= R_il
+// x_l from the last row up.  A chain of 32 steps of about 150 cycles.
+template <class T>
+__global__ void __launch_bounds__(32 * TRI_WARPS) tri_solve_kernel(int n, int i0, const T* R,
+                                                                   int64_t ldr, T* X,
+                                                                   int* singular,
+                                                                   const int* skip) {
   if (skipped(skip)) return;
   __shared__ T U[TRI_NB][TRI_NB + 1];  // U[l][i] = R[i, l]
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int i0 = blockIdx.x * TRI_NB, nb = min(TRI_NB, n - i0);
-  for (int l = wid; l < TRI_NB; l += TRI_WARPS)
-    U[l][lane] = (lane <= l && l < nb) ? R[i0 + lane + (int64_t)(i0 + l) * ldr] : zero_<T>();
+  const int nb = min(TRI_NB, n - i0);
+  for (int l = wid; l < nb; l += TRI_WARPS)
+    U[l][lane] = lane <= l ? R[i0 + lane + (int64_t)(i0 + l) * ldr] : zero_<T>();
   __syncthreads();
   const T d = lane < nb ? U[lane][lane] : one_<T>();
-  if (d == zero_<T>()) atomicExch(singular, 1);
+  if (blockIdx.x == 0 && d == zero_<T>()) atomicExch(singular, 1);
   const T dinv = inv_fast(d);
-  // column k: x_l = dinv_l acc_l from l = k up, acc_i -= R_il x_l (lane = i);
-  // four columns of a warp at a time
-  for (int k0 = wid; k0 < TRI_NB; k0 += 4 * TRI_WARPS) {
-    T acc[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) acc[q] = lane == k0 + q * TRI_WARPS ? one_<T>() : zero_<T>();
-    for (int l = min(TRI_NB - 1, k0 + 3 * TRI_WARPS); l >= 0; l--) {
-      const T u = lane < l ? U[l][lane] : zero_<T>();
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        if (l <= k0 + q * TRI_WARPS) {
-          if (lane == l) acc[q] = acc[q] * dinv;
-          acc[q] = fma_(-u, shfl_idx_(acc[q], l), acc[q]);
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int k = k0 + q * TRI_WARPS;
-      if (k < nb && lane < nb)
-        X[i0 + lane + (int64_t)(i0 + k) * n] = lane <= k ? acc[q] : zero_<T>();
-    }
+  const int c = i0 + (int)blockIdx.x * TRI_WARPS + wid;
+  if (c >= n) return;
+  T* const x = X + i0 + lane + (int64_t)c * n;
+  T b = lane < nb ? *x : zero_<T>();
+  for (int l = nb - 1; l >= 0; l--) {
+    if (lane == l) b = b * dinv;
+    const T u = lane < l ? U[l][lane] : zero_<T>();
+    b = fma_(-u, shfl_idx_(b, l), b);
   }
+  if (lane < nb) *x = b;
 }
 
-// One level, pair blockIdx.z (a = [a0, a0 + s), b behind it): mode 0 Y_ab =
-// R_ab X_bb, mode 1 X_ab = -X_aa Y_ab; 16 x 16 tiles, the zero halves of X_bb
-// and X_aa left out of the K range.
+// Y <- the upper triangle of R, zero below
 template <class T>
-__global__ void __launch_bounds__(256) tri_level_kernel(int n, int s, const T* R, int64_t ldr,
-                                                        T* X, T* Y, int mode, const int* skip) {
+__global__ void __launch_bounds__(256) tri_copy_kernel(int n, const T* R, int64_t ldr, T* Y,
+                                                       const int* skip) {
   if (skipped(skip)) return;
-  constexpr int B = 16, BK = 32, NT = 256, L = B * BK / NT;
-  __shared__ T As[BK][B + 1];
-  __shared__ T Bs[BK][B + 1];
-  const int a0 = 2 * s * blockIdx.z, b0 = a0 + s;
-  const int sb = min(s, n - b0);
-  const int m0 = blockIdx.x * B, n0 = blockIdx.y * B;
-  if (sb <= 0 || n0 >= sb) return;
-  const int64_t ab = a0 + (int64_t)b0 * n;
-  const Operand<T> A = mode == 0 ? Operand<T>{R + a0 + (int64_t)b0 * ldr, ldr, OP_N, MASK_FULL}
-                                 : Operand<T>{X + a0 + (int64_t)a0 * n, n, OP_N, MASK_FULL};
-  const Operand<T> Bo = mode == 0 ? Operand<T>{X + b0 + (int64_t)b0 * n, n, OP_N, MASK_FULL}
-                                  : Operand<T>{Y + ab, n, OP_N, MASK_FULL};
-  const int kend = mode == 0 ? min(sb, n0 + B) : s;  // X_bb[k, j] = 0 for k > j
-  const int kbeg = mode == 0 ? 0 : m0;               // X_aa[i, k] = 0 for k < i
-  const int tid = threadIdx.x, tx = tid % B, ty = tid / B;
-  T acc = zero_<T>(), ra[L], rb[L];
-  auto fetch = [&](int k0) {
-    fetch_tile<T, B, BK, NT, L>(A, true, m0, s, k0, kend, ra);
-    fetch_tile<T, B, BK, NT, L>(Bo, false, n0, sb, k0, kend, rb);
-  };
-  fetch(kbeg);
-  for (int k0 = kbeg; k0 < kend; k0 += BK) {
-#pragma unroll
-    for (int q = 0; q < L; q++) {
-      const int e = tid + q * NT;
-      As[e / B][e % B] = ra[q];
-      Bs[e % BK][e / BK] = rb[q];
-    }
-    __syncthreads();
-    if (k0 + BK < kend) fetch(k0 + BK);
-#pragma unroll 8
-    for (int kk = 0; kk < BK; kk++) acc = fma_(As[kk][tx], Bs[kk][ty], acc);
-    __syncthreads();
-  }
-  if (n0 + ty < sb) {
-    T* const C = mode == 0 ? Y : X;
-    C[ab + m0 + tx + (int64_t)(n0 + ty) * n] = mode == 0 ? acc : -acc;
-  }
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  for (int j = blockIdx.y; j < n; j += gridDim.y)
+    if (i < n) Y[i + (int64_t)j * n] = i <= j ? R[i + (int64_t)j * ldr] : zero_<T>();
+}
+// X[:, j] = Y[:, iperm[j]] above the diagonal, zero below
+template <class T>
+__global__ void __launch_bounds__(256) tri_gather_kernel(int n, const T* Y, const int* iperm,
+                                                         T* X, const int* skip) {
+  if (skipped(skip)) return;
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  for (int j = blockIdx.y; j < n; j += gridDim.y)
+    if (i < n) X[i + (int64_t)j * n] = i <= j ? Y[i + (int64_t)iperm[j] * n] : zero_<T>();
+}
+
+template <class T>
+bool tri_substitution(int64_t n, int precision) {
+  constexpr int64_t most = TRI_SOLVE_MAX_N<T>;
+  return precision != MAK_PREC_MIXED || sizeof(real_t<T>) != 8 || n <= most;
 }
 
 template <class T>
 int tri_inverse(cudaStream_t st, int64_t n, const T* R, int64_t ldr, T* X, int precision,
                 Arena& ar, mak_info* info) {
-  T* Y = ar.take<T>((size_t)n * n + 1);
-  // split products pay from 256-wide blocks (32 to 128: the batched levels)
-  constexpr int64_t wide = 256;
-  const bool mixed = precision == MAK_PREC_MIXED && sizeof(real_t<T>) == 8 && n > wide;
-  char* ozs = nullptr;
-  size_t oz_bytes = 0;
-  if (mixed) {
-    int64_t s = wide;
-    while (2 * s < n) s *= 2;
+  const bool direct = tri_substitution<T>(n, precision);
+  T* Y = nullptr;
+  int* iperm = nullptr;
+  char* gjs = nullptr;
+  size_t gj_bytes = 0;
+  if (!direct) {
     Arena meas(nullptr, 0);
-    gemm_prec<T>(st, precision, s, s, s, one_<T>(), opnd<T>(nullptr, 1), opnd<T>(nullptr, 1),
-                 zero_<T>(), nullptr, 1, meas, nullptr);
-    oz_bytes = meas.off + 1024;
-    ozs = ar.take<char>(oz_bytes);
+    gje_inverse<T>(st, n, nullptr, n, nullptr, precision, meas, nullptr);
+    gj_bytes = meas.off + 256;
+    Y = ar.take<T>((size_t)n * n + 1);
+    iperm = ar.take<int>(n + 1);
+    gjs = ar.take<char>(gj_bytes);
   }
   if (ar.base == nullptr) return 0;
   if (!ar.ok()) return MAK_ERR_WORKSPACE;
   if (n <= 0) return 0;
-  MAK_CUDA_TRY(cudaMemsetAsync(X, 0, (size_t)n * n * sizeof(T), st));
+  if (!direct) {
+    const dim3 g((unsigned)ceil_div(n, 256), (unsigned)(n < 16384 ? n : 16384));
+    note_launch();
+    tri_copy_kernel<T><<<g, 256, 0, st>>>((int)n, R, ldr, Y, skip_flag());
+    MAK_CUDA_TRY(cudaGetLastError());
+    Arena gj(gjs, gj_bytes);
+    MAK_TRY(gje_inverse<T>(st, n, Y, n, iperm, precision, gj, info));
+    note_launch();
+    tri_gather_kernel<T><<<g, 256, 0, st>>>((int)n, Y, iperm, X, skip_flag());
+    MAK_CUDA_TRY(cudaGetLastError());
+    return 0;
+  }
+  const dim3 g((unsigned)ceil_div(n, 256), (unsigned)(n < 16384 ? n : 16384));
   note_launch();
-  tri_diag_kernel<T><<<(unsigned)ceil_div(n, TRI_NB), 32 * TRI_WARPS, 0, st>>>(
-      (int)n, R, ldr, X, &info->singular, skip_flag());
+  tri_eye_kernel<T><<<g, 256, 0, st>>>((int)n, X, skip_flag());
   MAK_CUDA_TRY(cudaGetLastError());
-  for (int64_t s = TRI_NB; s < n; s *= 2) {
-    if (mixed && s >= wide) {
-      for (int64_t a0 = 0; a0 + s < n; a0 += 2 * s) {
-        const int64_t b0 = a0 + s, sb = (n - b0) < s ? (n - b0) : s;
-        {
-          Arena oz(ozs, oz_bytes);
-          MAK_TRY(gemm_prec<T>(st, precision, s, sb, sb, one_<T>(), opnd<T>(R + a0 + b0 * ldr, ldr),
-                               opnd<T>(X + b0 + b0 * n, n), zero_<T>(), Y + a0 + b0 * n, n, oz,
-                               &info->status));
-        }
-        Arena oz(ozs, oz_bytes);
-        MAK_TRY(gemm_prec<T>(st, precision, s, sb, s, -one_<T>(), opnd<T>(X + a0 + a0 * n, n),
-                             opnd<T>(Y + a0 + b0 * n, n), zero_<T>(), X + a0 + b0 * n, n, oz,
-                             &info->status));
-      }
-      continue;
-    }
-    const dim3 g((unsigned)(s / 16), (unsigned)ceil_div(s < n - s ? s : n - s, 16),
-                 (unsigned)ceil_div(n, 2 * s));
-    for (int mode = 0; mode < 2; mode++) {
-      note_launch();
-      tri_level_kernel<T><<<g, 256, 0, st>>>((int)n, (int)s, R, ldr, X, Y, mode, skip_flag());
-      MAK_CUDA_TRY(cudaGetLastError());
-    }
+  for (int64_t i0 = (n - 1) / TRI_NB * TRI_NB; i0 >= 0; i0 -= TRI_NB) {
+    const int64_t nb = (n - i0) < TRI_NB ? (n - i0) : TRI_NB;
+    note_launch();
+    tri_solve_kernel<T><<<(unsigned)ceil_div(n - i0, TRI_WARPS), 32 * TRI_WARPS, 0, st>>>(
+        (int)n, (int)i0, R, ldr, X, &info->singular, skip_flag());
+    MAK_CUDA_TRY(cudaGetLastError());
+    if (i0 > 0)
+      MAK_TRY(gemm<T>(st, i0, n - i0, nb, -one_<T>(), opnd<T>(R + i0 * ldr, ldr),
+                      opnd<T>(X + i0 + i0 * n, n), one_<T>(), X + i0 * n, n));
   }
   return 0;
 }
-#define MAK_INST_TRI(T) \
+#define MAK_INST_TRI(T)                               \
+  template bool tri_substitution<T>(int64_t, int);        \
   template int tri_inverse<T>(cudaStream_t, int64_t, const T*, int64_t, T*, int, Arena&, mak_info*);
 MAK_INST_TRI(double)
 MAK_INST_TRI(float)
@@ -1377,7 +1365,7 @@ int polar_newton_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T
     Arena meas(nullptr, 0);
     gje_inverse<T>(st, n, nullptr, n, nullptr, precision, meas, nullptr);
     gj_ws = meas.off + 256;
-    if (m > n) {  // the first iterate is triangular
+    if (m > n && tri_substitution<T>(n, precision)) {  // the first iterate is triangular
       Arena mt(nullptr, 0);
       tri_inverse<T>(st, n, nullptr, n, nullptr, precision, mt, nullptr);
       if (mt.off + 256 > gj_ws) gj_ws = mt.off + 256;
@@ -1423,6 +1411,7 @@ int polar_newton_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T
                                       : RED_CTAS);
   // one Newton step: X <- (g X + X^{-H}/g) / 2, measure max|D| into conv.  The
   // first iterate of a tall A is the triangular R.
+  const bool tri_first = m > n && tri_substitution<T>(n, precision);
   auto newton_step = [&](bool triangular) -> int {
     if (triangular) {
       Arena sub(tail, tail_bytes);
@@ -1471,7 +1460,7 @@ int polar_newton_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T
       // neither once the loop has stopped)
       {
         SkipScope skip_newton(stopw + 3);
-        MAK_TRY(newton_step(it == 1 && m > n));
+        MAK_TRY(newton_step(it == 1 && tri_first));
       }
       if (ns_fixed_ok) {
         SkipScope skip_ns(stopw + 4);
@@ -1482,7 +1471,7 @@ int polar_newton_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T
                                              ns_fixed_ok ? 1 : 0);
       MAK_CUDA_TRY(cudaGetLastError());
     } else {
-      MAK_TRY(in_ns ? ns_step() : newton_step(it == 1 && m > n));
+      MAK_TRY(in_ns ? ns_step() : newton_step(it == 1 && tri_first));
       R h[3];  // the two squared norms and max|D|
       MAK_CUDA_TRY(cudaMemcpyAsync(h, nrm2, sizeof(h), cudaMemcpyDeviceToHost, st));
       MAK_CUDA_TRY(cudaStreamSynchronize(st));
