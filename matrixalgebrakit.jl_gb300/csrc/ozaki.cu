@@ -77,8 +77,12 @@ constexpr long long OZ_SPIN = 1ll << 26;
 
 // Row (column) exponents of the operands are kept as the IEEE bit patterns
 // of the largest magnitudes and decoded where they are used.
+// by halves: a mask over the whole word may become a floating-point absolute
+// value, whose NaN carries a sign again (a NaN with its sign bit set then
+// raised its row's frame by 2^2048 and the whole row came out zero)
 __device__ __forceinline__ unsigned long long absbits(double x) {
-  return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+  return (unsigned long long)((unsigned)__double2hiint(x) & 0x7FFFFFFFu) << 32 |
+         (unsigned)__double2loint(x);
 }
 __device__ __forceinline__ int exp_of_absbits(unsigned long long b) {
   // smallest e with |x| < 2^e (frexp exponent); 0 for x == 0
