@@ -58,6 +58,7 @@ __device__ __forceinline__ T load_op(const Operand<T>& X, int64_t i, int64_t k) 
 
 int num_sms();
 constexpr int GEMM_BK = 32;  // K per step (and the granule of a K split)
+constexpr int GEMM_GRID_Y = 65535;  // column tiles per launch
 
 template <class T>
 __device__ __forceinline__ bool is_zero_(T v) { return v == zero_<T>(); }
@@ -115,7 +116,7 @@ __device__ __forceinline__ void fetch_tile(const Operand<T>& X, bool ci, int64_t
 template <class T, int BM, int BN, int BK, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_kernel(int M, int N, int K, T alpha, Operand<T> A, Operand<T> B, T beta, T* C,
-            int64_t ldc, int kchunk, int64_t split_stride, const int* skip) {
+            int64_t ldc, int kchunk, int64_t split_stride, int64_t col0, const int* skip) {
   if (skipped(skip)) return;
   constexpr int RX = BM / TM;  // threads along rows
   constexpr int RY = BN / TN;  // threads along columns
@@ -125,7 +126,7 @@ gemm_kernel(int M, int N, int K, T alpha, Operand<T> A, Operand<T> B, T beta, T*
   __shared__ T As[BK][BM + 1];
   __shared__ T Bs[BK][BN + 1];
   const int64_t m0 = (int64_t)blockIdx.x * BM;
-  const int64_t n0 = (int64_t)blockIdx.y * BN;
+  const int64_t n0 = col0 + (int64_t)blockIdx.y * BN;
   const int kbeg = blockIdx.z * kchunk;
   const int kend = min(K, kbeg + kchunk);
   C += blockIdx.z * split_stride;
@@ -211,7 +212,7 @@ gemm_kernel(int M, int N, int K, T alpha, Operand<T> A, Operand<T> B, T beta, T*
 template <class T, int BM, int BN, int BK, int TM, int TN, int RX, bool ROWC>
 __global__ void __launch_bounds__(256)
 gemm_f32_kernel(int M, int N, int K, T alpha, Operand<T> A, Operand<T> B, T beta, T* C,
-                int64_t ldc, int kchunk, int64_t split_stride, const int* skip) {
+                int64_t ldc, int kchunk, int64_t split_stride, int64_t col0, const int* skip) {
   if (skipped(skip)) return;
   constexpr int NT = 256, RY = NT / RX;
   static_assert(RX * TM == BM && RY * TN == BN, "256 threads cover the tile");
@@ -222,7 +223,7 @@ gemm_f32_kernel(int M, int N, int K, T alpha, Operand<T> A, Operand<T> B, T beta
   __shared__ alignas(16) T As[BK][BM + V];
   __shared__ alignas(16) T Bs[BK][BN + V];
   const int64_t m0 = (int64_t)blockIdx.x * BM;
-  const int64_t n0 = (int64_t)blockIdx.y * BN;
+  const int64_t n0 = col0 + (int64_t)blockIdx.y * BN;
   const int kbeg = blockIdx.z * kchunk;
   const int kend = min(K, kbeg + kchunk);
   C += blockIdx.z * split_stride;
@@ -349,12 +350,20 @@ int gemm(cudaStream_t st, int64_t M, int64_t N, int64_t K, T alpha, Operand<T> A
   if (used_splits) *used_splits = splits;
   if (splits > 1) beta = zero_<T>();
   ProfScope prof(st, PROF_GEMM_NATIVE, (traits<T>::cpx ? 8.0 : 2.0) * M * N * K);
-  note_launch();
+  // Column tiles are blockIdx.y, of which a grid has 65535: wider outputs (more
+  // than 2,097,120 columns of 32) take one launch per that many tiles.
+#define MAK_GEMM_COLS(BM, BN, ...)                                                               \
+  for (int64_t col0 = 0; col0 < N; col0 += (int64_t)GEMM_GRID_Y * BN) {                          \
+    const int64_t cols = N - col0 < (int64_t)GEMM_GRID_Y * BN ? N - col0                         \
+                                                              : (int64_t)GEMM_GRID_Y * BN;       \
+    note_launch();                                                                               \
+    __VA_ARGS__                                                                                  \
+        <<<dim3((unsigned)ceil_div(M, BM), (unsigned)ceil_div(cols, BN), (unsigned)splits), 256, \
+           0, st>>>((int)M, (int)N, (int)K, alpha, A, B, beta, C, ldc, kchunk, split_stride,     \
+                    col0, skip_flag());                                                          \
+  }
 #define MAK_GEMM_TILE(BM, BN, BK, TM, TN)                                                        \
-  gemm_kernel<T, BM, BN, BK, TM, TN>                                                             \
-      <<<dim3((unsigned)ceil_div(M, BM), (unsigned)ceil_div(N, BN), (unsigned)splits), 256, 0,   \
-         st>>>((int)M, (int)N, (int)K, alpha, A, B, beta, C, ldc, kchunk, split_stride,          \
-               skip_flag())
+  MAK_GEMM_COLS(BM, BN, gemm_kernel<T, BM, BN, BK, TM, TN>)
   const int64_t t32 = ceil_div(M, 32) * ceil_div(N, 32) * splits;
   if constexpr (sizeof(real_t<T>) == 8) {
     // The FP64 pipe is so slow that the operand traffic of a small tile costs
@@ -363,28 +372,32 @@ int gemm(cudaStream_t st, int64_t M, int64_t N, int64_t K, T alpha, Operand<T> A
     // Against 64 x 64 (and 32 x 64) tiles: a 512 x 64 x 32 complex update 140
     // -> 14.5 us, 1000 x 501 Float64 QR 4.5 -> 2.6 ms, 300 uneven blocks 188
     // -> 139 ms; 3000^3 45.3 -> 44.4 ms (1.22 TFLOP/s), 700^3 0.85 -> 0.83 ms.
-    if (t32 >= 3 * (int64_t)num_sms()) MAK_GEMM_TILE(32, 32, GEMM_BK, 2, 2);
-    else MAK_GEMM_TILE(16, 16, GEMM_BK, 1, 1);
+    if (t32 >= 3 * (int64_t)num_sms()) {
+      MAK_GEMM_TILE(32, 32, GEMM_BK, 2, 2)
+    } else {
+      MAK_GEMM_TILE(16, 16, GEMM_BK, 1, 1)
+    }
   } else {
     // wide tiles where they fill the GPU (their operand reads are the
     // cheapest), smaller ones before SMs idle.  The 4093 x 1537 Float32 QR:
     // W = V^H C 33 -> 20 us, C -= V W2 29 -> 19 us per panel, the LQ 6.0 ->
     // 5.0 ms (issue slots, 63 % busy; the tiles' sizes hardly matter)
 #define MAK_GEMM32_TILE(BM, BN, BK, TM, TN, RX, ROWC)                                            \
-  gemm_f32_kernel<T, BM, BN, BK, TM, TN, RX, ROWC>                                               \
-      <<<dim3((unsigned)ceil_div(M, BM), (unsigned)ceil_div(N, BN), (unsigned)splits), 256, 0,   \
-         st>>>((int)M, (int)N, (int)K, alpha, A, B, beta, C, ldc, kchunk, split_stride,          \
-               skip_flag())
+  MAK_GEMM_COLS(BM, BN, gemm_f32_kernel<T, BM, BN, BK, TM, TN, RX, ROWC>)
     const int64_t sms = num_sms();
-    if (M <= 32 && ceil_div(N, 128) * splits >= sms)
-      MAK_GEMM32_TILE(32, 128, 32 / (sizeof(T) / 4), 4, 4, 8, true);
-    else if (ceil_div(M, 128) * ceil_div(N, 64) * splits >= 2 * sms)
-      MAK_GEMM32_TILE(128, 64, 16, 4, 8, 32, false);
-    else if (t32 >= 4 * sms) MAK_GEMM32_TILE(64, 64, 16, 2, 8, 32, false);
-    else MAK_GEMM_TILE(32, 32, GEMM_BK, 2, 2);
+    if (M <= 32 && ceil_div(N, 128) * splits >= sms) {
+      MAK_GEMM32_TILE(32, 128, 32 / (sizeof(T) / 4), 4, 4, 8, true)
+    } else if (ceil_div(M, 128) * ceil_div(N, 64) * splits >= 2 * sms) {
+      MAK_GEMM32_TILE(128, 64, 16, 4, 8, 32, false)
+    } else if (t32 >= 4 * sms) {
+      MAK_GEMM32_TILE(64, 64, 16, 2, 8, 32, false)
+    } else {
+      MAK_GEMM_TILE(32, 32, GEMM_BK, 2, 2)
+    }
 #undef MAK_GEMM32_TILE
   }
 #undef MAK_GEMM_TILE
+#undef MAK_GEMM_COLS
   return cudaGetLastError() == cudaSuccess ? 0 : MAK_ERR_CUDA;
 }
 
