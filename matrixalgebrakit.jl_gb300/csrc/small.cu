@@ -73,10 +73,22 @@ struct SmallQrScratch {
 constexpr int SMALL_STATIC_CHUNK = 32;
 constexpr int SMALL_QR_THIRD = 72 * 1024;  // three CTAs per SM
 
-// magnitudes for which neither a product x a (|a| up to the type's range over
-// this window) nor a sum of squares leaves the range
+// The reflector's column x is multiplied unscaled with the columns to its
+// right.  Window of |x| in which its sum of squares stays in range, and range
+// of the block's columns (each by its largest magnitude; a reflection keeps
+// their norms) in which the products with an x of the window do, their last
+// digits included: 2^+-(100 + 800) of 2^+-1022, 2^+-(20 + 80) of 2^+-126.
 __device__ __forceinline__ bool small_in_window(double v) { return v > 0x1p-100 && v < 0x1p100; }
 __device__ __forceinline__ bool small_in_window(float v) { return v > 0x1p-20f && v < 0x1p20f; }
+template <class R> struct SmallRange;
+template <> struct SmallRange<double> {  // by the upper word of the bits
+  static constexpr unsigned lo = (1023u - 800u) << 20, hi = (1023u + 800u) << 20;
+  __device__ static unsigned top(unsigned long long key) { return (unsigned)(key >> 32); }
+};
+template <> struct SmallRange<float> {
+  static constexpr unsigned lo = (127u - 80u) << 23, hi = (127u + 80u) << 23;
+  __device__ static unsigned top(unsigned key) { return key; }
+};
 
 // this warp's partial dot products d_c = sum_r conj(x_r) S[r, c] over its
 // slice of the rows j+1 .. m-1, for the columns c0 .. c0 + nc - 1: lane =
@@ -191,7 +203,11 @@ __device__ void small_qr_item(const mak_batch_item& it, int positive, mak_info* 
       }
   }
   sh.fs = sh.part + SMALL_QR_WARPS * sh.chunk;
-  for (int c = wid; c < n; c += 4 * nw)
+  // the smallest and largest of the columns' maxima (columns of zeros aside)
+  using Rg = SmallRange<R>;
+  unsigned cmin = 0xFFFFFFFFu, cmax = 0u;
+  for (int c = wid; c < n; c += 4 * nw) {
+    unsigned top[4] = {0u, 0u, 0u, 0u};
     for (int r = lane; r < m; r += 32) {
       T v[4];
 #pragma unroll
@@ -199,9 +215,27 @@ __device__ void small_qr_item(const mak_batch_item& it, int positive, mak_info* 
         if (c + q * nw < n) v[q] = A[r + (int64_t)(c + q * nw) * it.lda];
 #pragma unroll
       for (int q = 0; q < 4; q++)
-        if (c + q * nw < n) S[r + (c + q * nw) * ld] = v[q];
+        if (c + q * nw < n) {
+          S[r + (c + q * nw) * ld] = v[q];
+          top[q] = max(top[q], Rg::top(mag_key(v[q])));
+        }
     }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const unsigned t = __reduce_max_sync(0xffffffffu, top[q]);
+      cmax = max(cmax, t);
+      if (t != 0u) cmin = min(cmin, t);
+    }
+  }
+  if (lane == 0) sh.key[wid] = (unsigned long long)cmax << 32 | cmin;
   __syncthreads();
+#pragma unroll
+  for (int w = 0; w < nw; w++) {
+    cmax = max(cmax, (unsigned)(sh.key[w] >> 32));
+    cmin = min(cmin, (unsigned)sh.key[w]);
+  }
+  const bool ranged = cmin >= Rg::lo && cmax < Rg::hi;
+  __syncthreads();  // the keys are rewritten
 
   // ---- factorization: one reflector per column.  The dot products of the
   // unscaled column x with itself and the columns to its right come first;
@@ -236,7 +270,8 @@ __device__ void small_qr_item(const mak_batch_item& it, int positive, mak_info* 
         for (int w = 1; w < nw; w++) mk = sh.key[w] > mk ? sh.key[w] : mk;
         const R amax = NK::val((typename NK::K)mk);
         const T alpha = x[j];
-        if (small_in_window(amax) && (!(abs2_(alpha) > R(0)) || small_in_window(abs_max_(alpha)))) {
+        if (ranged && small_in_window(amax) &&
+            (!(abs2_(alpha) > R(0)) || small_in_window(abs_max_(alpha)))) {
           const R ssq = re_(small_sum(sh, 0));
           const R n2 = sq_add(ssq, alpha);
           const R rs = rsqrt_b3(n2);
@@ -250,9 +285,9 @@ __device__ void small_qr_item(const mak_batch_item& it, int positive, mak_info* 
           scal = inv_b3(alpha - beta);
           fast = true;
         } else if (amax < R(INFINITY) && amax > R(0)) {
-          // rare: outside the window, the norm of x scaled by 2^-e, e the
-          // exponent of the largest magnitude (clamped); v first, then its
-          // dot products
+          // rare: outside the window or the range, the norm of x scaled by
+          // 2^-e, e the exponent of the largest magnitude (clamped); v first,
+          // then its dot products
           int e = 0;
           frexp(amax, &e);
           e = e > 1000 ? 1000 : (e < -1000 ? -1000 : e);
