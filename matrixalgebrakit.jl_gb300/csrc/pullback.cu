@@ -106,7 +106,8 @@ __global__ void copyltu_kernel(int p, T* M, int64_t ldm) {
 // B = s (M - M^H), or s (M + M^H) with sum set   (n x n, out of place)
 template <class T>
 __global__ void antiherm_kernel(int n, const T* M, int64_t ldm, real_t<T> s, T* B, int64_t ldb,
-                                bool sum = false) {
+                                bool sum = false, const int* skip = nullptr) {
+  if (skipped(skip)) return;
   __shared__ T t[32][33];
   const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -517,7 +518,7 @@ static int syl_solve(cudaStream_t st, int64_t n, const T* P, int64_t ldp, int ma
     MAK_TRY(G(n, n, n, one_<T>(), opnd<T>(s.Ak, n), opnd<T>(s.Ck, n), zero_<T>(), s.Tm, n));
     dim3 g((unsigned)ceil_div(n, 32), (unsigned)ceil_div(n, 32));
     note_launch();
-    antiherm_kernel<T><<<g, 256, 0, st>>>((int)n, s.Tm, n, Rr(1), s.Ai, n, true);
+    antiherm_kernel<T><<<g, 256, 0, st>>>((int)n, s.Tm, n, Rr(1), s.Ai, n, true, skip_flag());
     MAK_CUDA_TRY(cudaGetLastError());
     const T half = make_scalar<T>(Rr(0.5), 0);
     MAK_TRY(G(n, n, n, half, opnd<T>(s.Ck, n), opnd<T>(s.Y, n), zero_<T>(), s.Tm, n));
