@@ -71,6 +71,9 @@ struct SmallQrScratch {
   int chunk;
 };
 constexpr int SMALL_STATIC_CHUNK = 32;
+// keys and the smallest dot-product scratch, sized for the widest type
+constexpr size_t SMALL_QR_STAT =
+    8 * SMALL_QR_WARPS + sizeof(zcomplex) * (SMALL_QR_WARPS + 1) * SMALL_STATIC_CHUNK;
 constexpr int SMALL_QR_THIRD = 72 * 1024;  // three CTAs per SM
 
 // The reflector's column x is multiplied unscaled with the columns to its
@@ -157,6 +160,10 @@ __device__ __forceinline__ void small_update(T* S, int ld, int m, int j, const T
   }
 }
 
+// barrier of the ordinary form's four warps (its CTA may have more)
+__device__ __forceinline__ void small_sync() {
+  asm volatile("bar.sync 1, %0;" ::"n"(SMALL_QR_THREADS) : "memory");
+}
 template <class T>
 __device__ void small_qr_item(const mak_batch_item& it, int positive, mak_info* info,
                               unsigned char* dyn, int cap_bytes, unsigned char* stat) {
@@ -228,14 +235,14 @@ __device__ void small_qr_item(const mak_batch_item& it, int positive, mak_info* 
     }
   }
   if (lane == 0) sh.key[wid] = (unsigned long long)cmax << 32 | cmin;
-  __syncthreads();
+  small_sync();
 #pragma unroll
   for (int w = 0; w < nw; w++) {
     cmax = max(cmax, (unsigned)(sh.key[w] >> 32));
     cmin = min(cmin, (unsigned)sh.key[w]);
   }
   const bool ranged = cmin >= Rg::lo && cmax < Rg::hi;
-  __syncthreads();  // the keys are rewritten
+  small_sync();  // the keys are rewritten
 
   // ---- factorization: one reflector per column.  The dot products of the
   // unscaled column x with itself and the columns to its right come first;
@@ -262,7 +269,7 @@ __device__ void small_qr_item(const mak_batch_item& it, int positive, mak_info* 
         if (lane == 0) sh.key[wid] = (unsigned long long)mk;
       }
       small_dots(S, ld, m, j, x, c0, nc, sh);
-      __syncthreads();
+      small_sync();
       if (c0 == j) {
         // every warp repeats the scalars (each on its own FP64 pipe)
         unsigned long long mk = sh.key[0];
@@ -301,11 +308,11 @@ __device__ void small_qr_item(const mak_batch_item& it, int positive, mak_info* 
           larfg_scalars_ssq(alpha, re_(small_sum(sh, 0)), amax, beta, tau, scal);
         }
         if (scaled) {
-          __syncthreads();
+          small_sync();
           for (int r = j + 1 + tid; r < m; r += bd) x[r] = x[r] * scal;
-          __syncthreads();
+          small_sync();
           small_dots(S, ld, m, j, x, c0, nc, sh);
-          __syncthreads();
+          small_sync();
         }
       }
       for (int e = wid * 32 + lane; e < nc; e += bd) {
@@ -317,9 +324,9 @@ __device__ void small_qr_item(const mak_batch_item& it, int positive, mak_info* 
         sh.fs[e] = scaled ? f : f * scal;
         S[j + (c0 + e) * ld] = a - f;
       }
-      __syncthreads();
+      small_sync();
       small_update(S, ld, m, j, x, c0, c0 == j ? 1 : 0, nc, sh);
-      __syncthreads();
+      small_sync();
     }
     if (!scaled)
       for (int r = j + 1 + tid; r < m; r += bd) x[r] = x[r] * scal;
@@ -328,18 +335,18 @@ __device__ void small_qr_item(const mak_batch_item& it, int positive, mak_info* 
       taus[j] = tau;
     }
   }
-  __syncthreads();
+  small_sync();
 
   // ---- R with the gauge: R[i, c] = conj(s_i) A[i, c] (i <= c), 0 below
   for (int i = tid; i < k; i += bd) sgn[i] = positive ? sign_safe_(S[i + i * ld]) : one_<T>();
-  __syncthreads();
+  small_sync();
   if (it.R != nullptr) {
     T* Rout = (T*)it.R;
     for (int c = wid; c < n; c += nw)
       for (int i = lane; i < k; i += 32)
         Rout[i + (int64_t)c * it.ldr] = (i <= c) ? conj_(sgn[i]) * S[i + c * ld] : zero_<T>();
   }
-  __syncthreads();
+  small_sync();
 
   // ---- Q = H_0 ... H_{k-1} [I_k; 0], formed in place over the reflectors
   for (int j = k - 1; j >= 0; j--) {
@@ -349,16 +356,16 @@ __device__ void small_qr_item(const mak_batch_item& it, int positive, mak_info* 
     for (int c0 = j + 1; c0 < k; c0 += sh.chunk) {
       const int nc = min(sh.chunk, k - c0);
       small_dots(S, ld, m, j, v, c0, nc, sh);
-      __syncthreads();
+      small_sync();
       for (int e = tid; e < nc; e += bd) {
         const T a = S[j + (c0 + e) * ld];
         const T f = tau * (a + small_sum(sh, e));
         sh.fs[e] = f;
         S[j + (c0 + e) * ld] = a - f;
       }
-      __syncthreads();
+      small_sync();
       small_update(S, ld, m, j, v, c0, 0, nc, sh);
-      __syncthreads();
+      small_sync();
     }
     // column j of Q: e_j - tau v
     for (int r = tid; r < m; r += bd) {
@@ -368,11 +375,172 @@ __device__ void small_qr_item(const mak_batch_item& it, int positive, mak_info* 
       else q = -(tau * v[r]);
       v[r] = q;
     }
-    __syncthreads();
+    small_sync();
   }
   T* Qout = (T*)it.Q;
   for (int c = wid; c < k; c += nw)
     for (int r = lane; r < m; r += 32) Qout[r + (int64_t)c * it.ldq] = S[r + c * ld] * sgn[c];
+}
+
+// ---- tall, narrow blocks -------------------------------------------------------
+// Eight warps, lanes along the rows, a warp and its butterfly sums per column.
+// With many rows to a column the sums cost little, and the few columns would
+// leave most lanes of the form above idle.  One block, this form / that one:
+// Float64 150 x 20 156 / 182 us, 400 x 16 161 / 281, 1000 x 4 52 / 130, 3000 x
+// 8 217 / 746, 12000 x 1 35 / 266; Float32 1000 x 20 140 / 291.
+template <class T>
+__device__ void small_qr_tall_item(const mak_batch_item& it, int positive, mak_info* info,
+                              unsigned char* dyn, int cap_bytes, SmallScratch& sh) {
+  using R = real_t<T>;
+  using NK = NormKey<R>;
+  using Key = typename NK::K;
+  const int64_t m64 = it.m, n64 = it.n;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+  const int bd = blockDim.x;
+  if (tid == 0) {
+    info->status = 0;
+    info->iterations = 0;
+    info->rank = 0;
+    info->converged = 0;
+    info->residual = 0.0;
+    info->gauge = 0.0;
+    info->gauge_atol = 0.0;
+    info->singular = 0;
+    info->pad = 0;
+  }
+  if (m64 < 0 || n64 < 0 || small_qr_bytes(it.dtype, m64, n64) > (size_t)cap_bytes) {
+    if (tid == 0) info->status = MAK_ERR_UNSUPPORTED;
+    return;
+  }
+  const int m = (int)m64, n = (int)n64, k = m < n ? m : n;
+  if (k == 0) return;
+  const T* A = (const T*)it.A;
+  T* S = reinterpret_cast<T*>(dyn);  // m x n, ld m
+  T* taus = S + (int64_t)m * n;      // k
+  T* sgn = taus + k;                 // k
+  for (int c = 0; c < n; c++)
+    for (int r = tid; r < m; r += bd) S[r + c * m] = A[r + (int64_t)c * it.lda];
+  __syncthreads();
+
+  // ---- factorization: one reflector per column
+  R* red_r = reinterpret_cast<R*>(sh.red_r);
+  Key* red_k = reinterpret_cast<Key*>(sh.red_k);
+  T* sc = reinterpret_cast<T*>(sh.sc);
+  for (int j = 0; j < k; j++) {
+    T* col = S + j * m;
+    // sum of squares and largest magnitude of x = column j below the diagonal
+    R ss = R(0);
+    Key mk = 0;
+    for (int r = j + 1 + tid; r < m; r += bd) {
+      const T x = col[r];
+      ss = sq_add(ss, x);
+      const Key q = mag_key(x);
+      mk = q > mk ? q : mk;
+    }
+    ss = warp_sum(ss);
+    mk = warp_max_key(mk);
+    if (lane == 0) {
+      red_r[wid] = ss;
+      red_k[wid] = mk;
+    }
+    __syncthreads();
+    if (tid == 0) {
+      R s2 = R(0);
+      Key m2 = 0;
+      for (int w = 0; w < nw; w++) {
+        s2 += red_r[w];
+        m2 = red_k[w] > m2 ? red_k[w] : m2;
+      }
+      sh.sc_r[0] = (double)s2;
+      sh.sc_r[1] = (double)NK::val(m2);
+      sh.sc_flag = norm_needs_rescale<R>(m2);
+    }
+    __syncthreads();
+    R xnorm = R(0);
+    const bool rescale = sh.sc_flag != 0;
+    if (rescale) {
+      // rare: the squares would overflow or underflow; sum them scaled by
+      // 2^-e, e the exponent of the largest magnitude (clamped)
+      int e = 0;
+      frexp((R)sh.sc_r[1], &e);
+      e = e > 1000 ? 1000 : (e < -1000 ? -1000 : e);
+      const R scale = ldexp(R(1), -e);
+      R s3 = R(0);
+      for (int r = j + 1 + tid; r < m; r += bd) ssq_scaled_add(s3, col[r], scale);
+      s3 = block_sum(s3, red_r);
+      xnorm = sqrt(s3) * ldexp(R(1), e);
+    }
+    if (tid == 0) {
+      T beta, tau, scal;
+      if (rescale) larfg_scalars(col[j], xnorm, beta, tau, scal);
+      else larfg_scalars_ssq(col[j], (R)sh.sc_r[0], (R)sh.sc_r[1], beta, tau, scal);
+      sc[0] = beta;
+      sc[1] = tau;
+      sc[2] = scal;
+      taus[j] = tau;
+    }
+    __syncthreads();
+    const T beta = sc[0], tau = sc[1], scal = sc[2];
+    for (int r = j + 1 + tid; r < m; r += bd) col[r] = col[r] * scal;
+    __syncthreads();
+    // H_j^H on the columns to the right: w_c = A[j,c] + sum_{r>j} conj(v_r)
+    // A[r,c], A[:,c] -= v conj(tau) w_c (v_j = 1); a warp per column
+    for (int c = j + 1 + wid; c < n; c += nw) {
+      T* pc = S + c * m;
+      const T ajc = pc[j];
+      T acc = zero_<T>();
+      for (int r = j + 1 + lane; r < m; r += 32) acc = fma_(conj_(col[r]), pc[r], acc);
+      acc = warp_sum(acc);
+      const T f = conj_(tau) * (ajc + acc);
+      __syncwarp();
+      if (lane == 0) pc[j] = ajc - f;
+      for (int r = j + 1 + lane; r < m; r += 32) pc[r] = fma_(-col[r], f, pc[r]);
+    }
+    if (tid == 0) col[j] = beta;
+    __syncthreads();
+  }
+
+  // ---- R with the gauge: R[i, c] = conj(s_i) A[i, c] (i <= c), 0 below
+  for (int i = tid; i < k; i += bd) sgn[i] = positive ? sign_safe_(S[i + i * m]) : one_<T>();
+  __syncthreads();
+  if (it.R != nullptr) {
+    T* Rout = (T*)it.R;
+    for (int c = 0; c < n; c++)
+      for (int i = tid; i < k; i += bd)
+        Rout[i + (int64_t)c * it.ldr] = (i <= c) ? conj_(sgn[i]) * S[i + c * m] : zero_<T>();
+  }
+  __syncthreads();
+
+  // ---- Q = H_0 ... H_{k-1} [I_k; 0], formed in place over the reflectors
+  for (int j = k - 1; j >= 0; j--) {
+    T* col = S + j * m;
+    const T tau = taus[j];
+    // H_j on the columns c in (j, k): rows >= j (rows < j are zero there)
+    for (int c = j + 1 + wid; c < k; c += nw) {
+      T* pc = S + c * m;
+      const T qj = pc[j];
+      T acc = zero_<T>();
+      for (int r = j + 1 + lane; r < m; r += 32) acc = fma_(conj_(col[r]), pc[r], acc);
+      acc = warp_sum(acc);
+      const T f = tau * (qj + acc);
+      __syncwarp();
+      if (lane == 0) pc[j] = qj - f;
+      for (int r = j + 1 + lane; r < m; r += 32) pc[r] = fma_(-col[r], f, pc[r]);
+    }
+    __syncthreads();
+    // column j of Q: e_j - tau v
+    for (int r = tid; r < m; r += bd) {
+      T q;
+      if (r < j) q = zero_<T>();
+      else if (r == j) q = one_<T>() - tau;
+      else q = -(tau * col[r]);
+      col[r] = q;
+    }
+    __syncthreads();
+  }
+  T* Qout = (T*)it.Q;
+  for (int c = 0; c < k; c++)
+    for (int r = tid; r < m; r += bd) Qout[r + (int64_t)c * it.ldq] = S[r + c * m] * sgn[c];
 }
 
 // ---------------------------------------------------------------- polar --
@@ -726,9 +894,7 @@ small_polar_device_kernel(const mak_batch_item* items, int count, int maxiter, d
 
 __device__ void small_qr_dispatch(const mak_batch_item& it, int positive, mak_info* info,
                                   unsigned char* dyn, int cap_bytes) {
-  // keys and the smallest dot-product scratch, sized for the widest type
-  __shared__ __align__(16) unsigned char
-      stat[8 * SMALL_QR_WARPS + sizeof(zcomplex) * (SMALL_QR_WARPS + 1) * SMALL_STATIC_CHUNK];
+  __shared__ __align__(16) unsigned char stat[SMALL_QR_STAT];
   switch (it.dtype) {
     case MAK_F64: small_qr_item<double>(it, positive, info, dyn, cap_bytes, stat); break;
     case MAK_C64: small_qr_item<zcomplex>(it, positive, info, dyn, cap_bytes, stat); break;
@@ -740,29 +906,85 @@ __device__ void small_qr_dispatch(const mak_batch_item& it, int positive, mak_in
   __syncthreads();  // the shared block is reused by the next item
 }
 
-// Items of more than lo_bytes up to the launch's cap_bytes (and, with all set,
-// those beyond it, which report MAK_ERR_UNSUPPORTED)
-__device__ __forceinline__ bool small_qr_mine(const mak_batch_item& it, int lo_bytes,
-                                              int cap_bytes, int all) {
-  if (it.m < 0 || it.n < 0) return all != 0;
-  const int64_t need = (int64_t)small_qr_bytes(it.dtype, it.m, it.n);
-  return need > lo_bytes && (all || need <= cap_bytes);
+// Whether a block that fits takes the tall form.  Alone on its SM (no more
+// blocks than SMs, or one of more than a third of an SM's shared memory): from 6
+// rows per column on, 4 in the FP32 types (tall / ordinary form, us: Float64 64
+// x 16 101 / 88, 150 x 20 156 / 182; Float32 64 x 16 41 / 45, 128 x 32 110 /
+// 112).  Where three ordinary CTAs share the SM and hide each other's chains:
+// from 16 rows per column on, if the columns are long (700 blocks: Float64 150 x
+// 20 760 / 522, 256 x 4 128 / 137, 1000 x 4 237 / 401; ComplexF64 128 x 8 387 /
+// 460; ComplexF32 400 x 16 336 / 299, 1000 x 4 104 / 127).
+__host__ __device__ inline bool small_qr_tall(int dtype, int64_t m, int64_t n, bool few) {
+  if (m < 4 || n < 1) return false;
+  const bool f64 = dtype == MAK_F64 || dtype == MAK_C64;
+  if (few || small_qr_bytes(dtype, m, n) > (size_t)SMALL_QR_THIRD) return m >= (f64 ? 6 : 4) * n;
+  return m >= 16 * n && m >= (dtype == MAK_C64 ? 128 : (f64 ? 256 : 512));
 }
-__global__ void __launch_bounds__(SMALL_QR_THREADS)
+// One kernel of four warps for the ordinary blocks of which three share an SM,
+// one of eight for the rest: the tall blocks with all eight, the others with the
+// first four.
+__device__ void small_qr_wide_dispatch(const mak_batch_item& it, int positive, mak_info* info,
+                                       unsigned char* dyn, int cap_bytes, bool few) {
+  __shared__ __align__(16) unsigned char stat[SMALL_QR_STAT];
+  static_assert(sizeof(SmallScratch) <= SMALL_QR_STAT, "the tall form's scratch");
+  SmallScratch& sh = *reinterpret_cast<SmallScratch*>(stat);
+  const bool fits = it.m >= 0 && it.n >= 0 &&
+                    small_qr_bytes(it.dtype, it.m, it.n) <= (size_t)cap_bytes;
+  const bool tall = fits && small_qr_tall(it.dtype, it.m, it.n, few);
+  const bool mine = tall || threadIdx.x < SMALL_QR_THREADS;
+  const auto run = [&](auto zero) {
+    using T = decltype(zero);
+    if (tall) small_qr_tall_item<T>(it, positive, info, dyn, cap_bytes, sh);
+    else if (mine) small_qr_item<T>(it, positive, info, dyn, cap_bytes, stat);
+  };
+  switch (it.dtype) {
+    case MAK_F64: run(double()); break;
+    case MAK_C64: run(zcomplex()); break;
+    case MAK_F32: run(float()); break;
+    case MAK_C32: run(ccomplex()); break;
+    default:
+      if (threadIdx.x == 0) info->status = MAK_ERR_UNSUPPORTED;
+  }
+  __syncthreads();  // the shared block is reused by the next item
+}
+// ordinary blocks of up to lo_bytes
+__device__ __forceinline__ bool small_qr_third(const mak_batch_item& it, int lo_bytes) {
+  return it.m >= 0 && it.n >= 0 &&
+         (int64_t)small_qr_bytes(it.dtype, it.m, it.n) <= lo_bytes &&
+         !small_qr_tall(it.dtype, it.m, it.n, false);
+}
+__global__ void __launch_bounds__(SMALL_QR_THREADS, 3)
 small_qr_list_kernel(const __grid_constant__ SmallList L, int positive, mak_info* infos,
                      int cap_bytes) {
   extern __shared__ __align__(16) unsigned char small_dyn[];
   for (int q = blockIdx.x; q < L.count; q += gridDim.x)
     small_qr_dispatch(L.items[q], positive, infos + L.idx[q], small_dyn, cap_bytes);
 }
+__global__ void __launch_bounds__(SMALL_THREADS, 1)
+small_qr_wide_list_kernel(const __grid_constant__ SmallList L, int positive, mak_info* infos,
+                          int cap_bytes, bool few) {
+  extern __shared__ __align__(16) unsigned char small_dyn[];
+  for (int q = blockIdx.x; q < L.count; q += gridDim.x)
+    small_qr_wide_dispatch(L.items[q], positive, infos + L.idx[q], small_dyn, cap_bytes, few);
+}
 
-__global__ void __launch_bounds__(SMALL_QR_THREADS)
+__global__ void __launch_bounds__(SMALL_QR_THREADS, 3)
 small_qr_device_kernel(const mak_batch_item* items, int count, int positive, mak_info* infos,
-                       int lo_bytes, int cap_bytes, int all) {
+                       int cap_bytes) {
   extern __shared__ __align__(16) unsigned char small_dyn[];
   for (int q = blockIdx.x; q < count; q += gridDim.x)
-    if (small_qr_mine(items[q], lo_bytes, cap_bytes, all))
+    if (small_qr_third(items[q], cap_bytes))
       small_qr_dispatch(items[q], positive, infos + q, small_dyn, cap_bytes);
+}
+// all items (few), or those the kernel above has passed over; blocks beyond
+// cap_bytes report MAK_ERR_UNSUPPORTED
+__global__ void __launch_bounds__(SMALL_THREADS, 1)
+small_qr_wide_device_kernel(const mak_batch_item* items, int count, int positive,
+                            mak_info* infos, int cap_bytes, int lo_bytes, bool few) {
+  extern __shared__ __align__(16) unsigned char small_dyn[];
+  for (int q = blockIdx.x; q < count; q += gridDim.x)
+    if (few || !small_qr_third(items[q], lo_bytes))
+      small_qr_wide_dispatch(items[q], positive, infos + q, small_dyn, cap_bytes, few);
 }
 
 // the largest dynamic shared memory of the small-block kernels on this
@@ -777,6 +999,10 @@ static int small_smem_limit() {
     cudaFuncSetAttribute(small_qr_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
     cudaFuncSetAttribute(small_qr_device_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          cap);
+    cudaFuncSetAttribute(small_qr_wide_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         cap);
+    cudaFuncSetAttribute(small_qr_wide_device_kernel,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
     cudaFuncSetAttribute(small_polar_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          cap);
     cudaFuncSetAttribute(small_polar_device_kernel,
@@ -827,29 +1053,34 @@ int small_polar_launch(cudaStream_t st, const mak_batch_item* items, const int* 
   return 0;
 }
 
-// one persistent launch (per SMALL_LIST_MAX items and shared-memory class)
-// over the listed items: the blocks that fit a third of an SM's shared memory
-// run three CTAs per SM
+// one persistent launch (per SMALL_LIST_MAX items and class) over the listed
+// items: with more blocks than SMs, the ordinary blocks that fit a third of an
+// SM's shared memory (three CTAs per SM); the others
 int small_qr_launch(cudaStream_t st, const mak_batch_item* items, const int* which, int count,
                     int positive, mak_info* infos, int cap) {
   static thread_local SmallList L;
+  const int64_t sms = num_sms();
+  const bool few = count <= sms;
+  const int lo = cap > SMALL_QR_THIRD && !few ? SMALL_QR_THIRD : -1;
   for (int cls = 0; cls < 2; cls++) {
-    const int smem = cls == 0 ? cap : (cap > SMALL_QR_THIRD ? SMALL_QR_THIRD : 0);
-    const int64_t most = cls == 0 ? num_sms() : 3 * (int64_t)num_sms();
     L.count = 0;
     for (int q = 0; q <= count; q++) {
       if (q < count) {
         const mak_batch_item& it = items[which[q]];
-        const bool third = cap > SMALL_QR_THIRD &&
-                           small_qr_bytes(it.dtype, it.m, it.n) <= (size_t)SMALL_QR_THIRD;
+        const bool third = (int64_t)small_qr_bytes(it.dtype, it.m, it.n) <= lo &&
+                           !small_qr_tall(it.dtype, it.m, it.n, false);
         if (third != (cls == 1)) continue;
         L.items[L.count] = it;
         L.idx[L.count++] = which[q];
       }
       if (L.count == 0 || (q < count && L.count < SMALL_LIST_MAX)) continue;
+      const int64_t most = cls == 1 ? 3 * sms : sms;
+      const int grid = (int)(L.count < most ? L.count : most);
       note_launch();
-      small_qr_list_kernel<<<(int)(L.count < most ? L.count : most), SMALL_QR_THREADS, smem, st>>>(
-          L, positive, infos, smem);
+      if (cls == 1)
+        small_qr_list_kernel<<<grid, SMALL_QR_THREADS, lo, st>>>(L, positive, infos, lo);
+      else
+        small_qr_wide_list_kernel<<<grid, SMALL_THREADS, cap, st>>>(L, positive, infos, cap, few);
       MAK_CUDA_TRY(cudaGetLastError());
       L.count = 0;
     }
@@ -871,21 +1102,22 @@ extern "C" int mak_batched_qr_compact_device(const mak_batch_item* items, int ni
   if (nitems == 0) return 0;
   const int cap = small_qr_cap();
   if (cap <= 0) return MAK_ERR_UNSUPPORTED;
-  // The host does not see the blocks' sizes: one launch per shared-memory
-  // class, the blocks that fit a third of an SM's first (three CTAs per SM
-  // hide each other's scalar steps), each CTA passing over the other class.
+  // The host does not see the blocks' sizes: with more blocks than SMs one
+  // launch per class, each CTA passing over the other class's blocks, those of
+  // which three share an SM first (they hide each other's scalar steps).
   cudaStream_t st = (cudaStream_t)stream;
-  const int lo = cap > SMALL_QR_THIRD ? SMALL_QR_THIRD : 0;
+  const bool few = nitems <= num_sms();
+  const int lo = cap > SMALL_QR_THIRD && !few ? SMALL_QR_THIRD : -1;
   if (lo > 0) {
     const int64_t most = 3 * (int64_t)num_sms();
     note_launch();
     small_qr_device_kernel<<<(int)(nitems < most ? nitems : most), SMALL_QR_THREADS, lo, st>>>(
-        items, nitems, opts->positive, infos, -1, lo, 0);
+        items, nitems, opts->positive, infos, lo);
     MAK_CUDA_TRY(cudaGetLastError());
   }
   note_launch();
-  small_qr_device_kernel<<<nitems < num_sms() ? nitems : num_sms(), SMALL_QR_THREADS, cap, st>>>(
-      items, nitems, opts->positive, infos, lo > 0 ? lo : -1, cap, 1);
+  small_qr_wide_device_kernel<<<few ? nitems : num_sms(), SMALL_THREADS, cap, st>>>(
+      items, nitems, opts->positive, infos, cap, lo, few);
   return cudaGetLastError() == cudaSuccess ? 0 : MAK_ERR_CUDA;
 }
 
