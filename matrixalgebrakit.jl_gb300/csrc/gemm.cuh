@@ -173,8 +173,9 @@ gemm_kernel(int M, int N, int K, T alpha, Operand<T> A, Operand<T> B, T beta, T*
     }
     __syncthreads();
     if (k0 + BK < kend) fetch(k0 + BK);
+    const int kn = min(BK, kend - k0);  // the last step may be short: no padding multiplied
 #pragma unroll 4
-    for (int kk = 0; kk < BK; kk++) {
+    for (int kk = 0; kk < kn; kk++) {
       T a[TM], b[TN];
 #pragma unroll
       for (int r = 0; r < TM; r++) a[r] = As[kk][tx + r * RX];
@@ -271,8 +272,9 @@ gemm_f32_kernel(int M, int N, int K, T alpha, Operand<T> A, Operand<T> B, T beta
     }
     __syncthreads();
     if (k0 + BK < kend) fetch(k0 + BK);
+    const int kn = min(BK, kend - k0);  // the last step may be short: no padding multiplied
 #pragma unroll 4
-    for (int kk = 0; kk < BK; kk++) {
+    for (int kk = 0; kk < kn; kk++) {
       T a[TM], b[TN];
       if constexpr (ROWC) {
 #pragma unroll
@@ -372,7 +374,10 @@ int gemm(cudaStream_t st, int64_t M, int64_t N, int64_t K, T alpha, Operand<T> A
     // Against 64 x 64 (and 32 x 64) tiles: a 512 x 64 x 32 complex update 140
     // -> 14.5 us, 1000 x 501 Float64 QR 4.5 -> 2.6 ms, 300 uneven blocks 188
     // -> 139 ms; 3000^3 45.3 -> 44.4 ms (1.22 TFLOP/s), 700^3 0.85 -> 0.83 ms.
-    if (t32 >= 3 * (int64_t)num_sms()) {
+    // Outputs of at most 16 rows take 16 x 16 tiles at any width: half of a 32-row
+    // tile would be padding (gemm call of 8 x 100000 x 8: 286 us with 32-row tiles
+    // and K padded to 32, 139 now; ComplexF64 814 and 239).
+    if (t32 >= 3 * (int64_t)num_sms() && M > 16) {
       MAK_GEMM_TILE(32, 32, GEMM_BK, 2, 2)
     } else {
       MAK_GEMM_TILE(16, 16, GEMM_BK, 1, 1)
@@ -385,8 +390,15 @@ int gemm(cudaStream_t st, int64_t M, int64_t N, int64_t K, T alpha, Operand<T> A
 #define MAK_GEMM32_TILE(BM, BN, BK, TM, TN, RX, ROWC)                                            \
   MAK_GEMM_COLS(BM, BN, gemm_f32_kernel<T, BM, BN, BK, TM, TN, RX, ROWC>)
     const int64_t sms = num_sms();
+    constexpr int BK32 = 32 / (sizeof(T) / 4);
     if (M <= 32 && ceil_div(N, 128) * splits >= sms) {
-      MAK_GEMM32_TILE(32, 128, 32 / (sizeof(T) / 4), 4, 4, 8, true)
+      // (a short K: half the step, whose padding costs fetches; QR of 8 x
+      // 1000000 Float32 579 -> 505 us, 8 x 1000000 ComplexF32 780 -> 555)
+      if (2 * K <= BK32) {
+        MAK_GEMM32_TILE(32, 128, BK32 / 2, 4, 4, 8, true)
+      } else {
+        MAK_GEMM32_TILE(32, 128, BK32, 4, 4, 8, true)
+      }
     } else if (ceil_div(M, 128) * ceil_div(N, 64) * splits >= 2 * sms) {
       MAK_GEMM32_TILE(128, 64, 16, 4, 8, 32, false)
     } else if (t32 >= 4 * sms) {

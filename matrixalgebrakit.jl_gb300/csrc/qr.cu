@@ -1196,21 +1196,25 @@ qr_panel_kernel(PanelArgs<T> a) {
 }
 
 // W2[:, c] = op(Tm) * sum_s Wpart[s][:, c]   (op = ^H for the factorization,
-// identity for Q formation).  Fixed summation order -> deterministic.  Eight
-// columns per CTA, one output per thread: the FP64 work of the product is
-// spread over as many SMs as there are column groups (32 columns per CTA left
-// most of them idle: 500 columns 17.5 us).
-constexpr int TRMM_COLS = 8;
+// identity for Q formation).  Fixed summation order -> deterministic.  One
+// output per thread, eight columns per CTA of 32 rows: the FP64 work of the
+// product is spread over as many SMs as there are column groups (32 columns per
+// CTA left most of them idle: 500 columns 17.5 us).  16 or 32 columns where 16
+// or 8 rows are all there are (8 x 100000: 68 us with 32 rows of threads).
+constexpr int TRMM_THREADS = 256;
+__host__ __device__ constexpr int trmm_rows(int jb) { return jb <= 8 ? 8 : (jb <= 16 ? 16 : 32); }
+__host__ __device__ constexpr int trmm_cols(int jb) { return TRMM_THREADS / trmm_rows(jb); }
 template <class T>
-__global__ void __launch_bounds__(256) reduce_trmm_kernel(int jb, int nt, int splits,
+__global__ void __launch_bounds__(TRMM_THREADS) reduce_trmm_kernel(int jb, int nt, int splits,
                                                           const T* __restrict__ Wpart,
                                                           int64_t sstride,
                                                           const T* __restrict__ Tm, int conjtrans,
                                                           T* __restrict__ W2) {
   __shared__ T Ts[NBMAX][NBMAX + 1];
-  __shared__ T Ws[TRMM_COLS][NBMAX];
-  const int i = threadIdx.x & 31, cc = threadIdx.x >> 5;
-  const int c = blockIdx.x * TRMM_COLS + cc;
+  __shared__ T Ws[TRMM_THREADS];
+  const int rows = trmm_rows(jb);
+  const int i = threadIdx.x & (rows - 1);
+  const int c = blockIdx.x * trmm_cols(jb) + threadIdx.x / rows;
   for (int e = threadIdx.x; e < jb * jb; e += blockDim.x) {
     const int r = e % jb, l = e / jb;
     if (conjtrans) Ts[l][r] = conj_(Tm[r + l * NBMAX]);
@@ -1227,15 +1231,16 @@ __global__ void __launch_bounds__(256) reduce_trmm_kernel(int jb, int nt, int sp
     }
     for (; q < splits; q++) w += src[q * sstride];
   }
-  Ws[cc][i] = w;
+  Ws[threadIdx.x] = w;
   __syncthreads();
   if (i >= jb || c >= nt) return;
+  const T* const wc = Ws + threadIdx.x - i;  // the column's entries
   T s[4] = {zero_<T>(), zero_<T>(), zero_<T>(), zero_<T>()};
   int l = 0;
   for (; l + 3 < jb; l += 4)
 #pragma unroll
-    for (int q = 0; q < 4; q++) s[q] = fma_(Ts[i][l + q], Ws[cc][l + q], s[q]);
-  for (; l < jb; l++) s[0] = fma_(Ts[i][l], Ws[cc][l], s[0]);
+    for (int q = 0; q < 4; q++) s[q] = fma_(Ts[i][l + q], wc[l + q], s[q]);
+  for (; l < jb; l++) s[0] = fma_(Ts[i][l], wc[l], s[0]);
   W2[i + (int64_t)c * jb] = (s[0] + s[1]) + (s[2] + s[3]);
 }
 
@@ -1734,7 +1739,7 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
     MAK_TRY(gemm<T>(s, jb, nt, mp, one_<T>(), opnd<T>(Ap, lda, OP_C, MASK_UNIT_LOWER),
                     opnd<T>(C, lda), zero_<T>(), Wpart, jb, splits, (int64_t)jb * nt, &used));
     note_launch();
-    reduce_trmm_kernel<T><<<(unsigned)ceil_div(nt, TRMM_COLS), 256, 0, s>>>(jb, (int)nt, used, Wpart,
+    reduce_trmm_kernel<T><<<(unsigned)ceil_div(nt, trmm_cols(jb)), 256, 0, s>>>(jb, (int)nt, used, Wpart,
                                                                       (int64_t)jb * nt, Tb, 1, W2);
     MAK_CUDA_TRY(cudaGetLastError());
     return gemm<T>(s, mp, nt, jb, -one_<T>(), opnd<T>(Ap, lda, OP_N, MASK_UNIT_LOWER),
@@ -1759,7 +1764,7 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
                            Wp, jb, ga, status, mc));
     }
     note_launch();
-    reduce_trmm_kernel<T><<<(unsigned)ceil_div(nt, TRMM_COLS), 256, 0, s>>>(jb, (int)nt, 1, Wp,
+    reduce_trmm_kernel<T><<<(unsigned)ceil_div(nt, trmm_cols(jb)), 256, 0, s>>>(jb, (int)nt, 1, Wp,
                                                                       (int64_t)jb * nt, Tb, 1, W2p);
     MAK_CUDA_TRY(cudaGetLastError());
     Arena ga(grams, gram_bytes);
@@ -1947,7 +1952,7 @@ int qr_run(cudaStream_t st, int64_t m, int64_t n, T* A, int64_t lda, T* Q, int64
     MAK_TRY(gemm<T>(st, jb, qt, mp, one_<T>(), opnd<T>(Ap, lda, OP_C, MASK_UNIT_LOWER),
                     opnd<T>(Qs, ldq), zero_<T>(), Wpart, jb, splits, (int64_t)jb * qt, &used));
     note_launch();
-    reduce_trmm_kernel<T><<<(unsigned)ceil_div(qt, TRMM_COLS), 256, 0, st>>>(
+    reduce_trmm_kernel<T><<<(unsigned)ceil_div(qt, trmm_cols(jb)), 256, 0, st>>>(
         jb, (int)qt, used, Wpart, (int64_t)jb * qt, Tb, 0, W2);
     MAK_CUDA_TRY(cudaGetLastError());
     MAK_TRY(gemm<T>(st, mp, qt, jb, -one_<T>(), opnd<T>(Ap, lda, OP_N, MASK_UNIT_LOWER),
