@@ -14,10 +14,12 @@
 // The inverse is an in-place blocked Gauss-Jordan elimination with partial
 // pivoting (gje_inverse): per block column of 32 a panel kernel (pivot
 // search + row exchange + elimination, one barrier per column, panel rows
-// resident in shared memory; a thread-block cluster of up to 16 CTAs for
-// n <= 4096, a cooperative grid with a bounded global barrier beyond), a
-// row-exchange/save kernel for the other columns and one rank-32 GEMM update -- 2n^3 flops in total,
-// the same count as the reference's LU + inverse.  The Newton update reads
+// resident in shared memory; a thread-block cluster of up to 16 CTAs for n up
+// to 4096 in Float64, 2048 in ComplexF64 and 8192 in the FP32 types as far as
+// its rows fit, a cooperative grid with a bounded global barrier beyond), a
+// row-exchange/save kernel for the other columns and one rank-32 GEMM update
+// -- 2n^3 flops in total, the same count as the reference's LU + inverse.  The
+// triangular first iterate of a tall A is inverted by substitution.  The Newton update reads
 // X^{-H} straight out of the eliminated matrix through the inverse column
 // permutation (no separate transpose or permutation pass) and fuses the
 // avgdiff step, the scaling and the max-abs convergence measure.  For

@@ -336,7 +336,7 @@ __device__ __forceinline__ int panel_block_round(const PanelArgs<T>& a, T* Ps, i
   // behind.  A step takes the column pair 2P, 2P + 1, whose two rows one warp
   // owns (pair P: warp P mod 4 of each group; lane = column): the owner forms
   // both in registers and publishes them, a barrier follows, then the other
-  // rows.  On GB300 a dependent FP64 operation takes about 100 cycles and a
+  // rows.  On GB300 a dependent FP64 operation takes 61 cycles (measured) and a
   // warp-wide one holds its sub-partition's FP64 pipe for 64, so the chains
   // are kept short (four operations from D_j to D_{j+1} with no square root
   // between them, five from alpha_j to alpha_{j+1}), and the next owner

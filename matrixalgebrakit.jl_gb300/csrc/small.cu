@@ -3,13 +3,13 @@
 // For a block whose m x n elements fit one CTA's shared memory, the batched
 // driver's per-block chain of launches (panels, block updates, Q formation:
 // qr_householder!, src/implementations/qr.jl:132-188, once per block) is
-// replaced by a single persistent launch that walks a list of block
-// descriptors (mak_batch_item): CTA b takes items b, b + gridDim.x, ...
+// replaced by a persistent launch (two for more blocks than SMs, by the shared
+// memory they take) that walks a list of block descriptors (mak_batch_item): CTA b takes items b, b + gridDim.x, ...
 // and for each
 //   1. loads the block into shared memory,
-//   2. factors it column by column (LAPACK geqr2 order; the reflector
-//      scalars come from the same larfg helpers as the multi-CTA panel, so
-//      beta is real and R's diagonal carries its sign),
+//   2. factors it column by column (LAPACK geqr2 order and larfg conventions,
+//      so beta is real and R's diagonal carries its sign; lane = column, or
+//      lane = row for tall, narrow blocks),
 //   3. writes R with the positive gauge (rows scaled by conj(s_i), s =
 //      sign_safe(diag R), src/common/gauge.jl:16-25),
 //   4. forms Q in place over the reflectors (org2r order: H_{k-1} first on
